@@ -966,6 +966,7 @@ void Engine::flux_vjp(const double* obs, int64_t n_obs, const std::vector<double
       const int tev = fp64_entries_per_cta(v);  // entries per CTA of that variant
       part_.reserve(sizeof(double) * 2 * kFdPartials * N);
       w.lev = lev_.as<double>(); w.cap = lev_cap_; w.tile_entries = tev; w.part = part_.as<double>();
+      set_phase_reach(w);
       check(launch_fd_wave_fp64(w, (int)std::min<int64_t>((N + tev - 1) / tev, wave_grid(0, v)), v, st),
             "adjoint forward");
     }

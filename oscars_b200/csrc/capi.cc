@@ -893,13 +893,10 @@ OSC_API int osc_variant_name(int kind, int variant, char* name, long long capaci
     if (kind != 0 && kind != 2 && kind != 3)
       throw osc::Error{OSC_ERR_INVALID, "kind must be 0 (fp64), 2 (mixed) or 3 (batched mixed)"};
     if (variant < 0 || variant >= n_variants_of(kind)) throw osc::Error{OSC_ERR_RANGE, "variant out of range"};
-    static const char* const kFp64[] = {"k_fd_wave_fp64<1,7>", "k_fd_wave_fp64<2,7>", "k_fd_wave_fp64<4,7>",
-                                        "k_fd_wave_fp64<4,5>"};
     static const char* const kBatch[] = {"k_batch_wave<4,4>", "k_batch_wave<4,1>", "k_batch_wave<2,4>",
                                          "k_batch_wave<1,4>"};
-    static_assert(sizeof(kFp64) / sizeof(kFp64[0]) == osc::kFp64Variants, "FP64 variant names");
     static_assert(sizeof(kBatch) / sizeof(kBatch[0]) == osc::kBatchVariants, "batch variant names");
-    const char* n = kind == 0 ? kFp64[variant] : kind == 2 ? osc::mixed_variant_name(variant) : kBatch[variant];
+    const char* n = kind == 0 ? osc::fp64_variant_name(variant) : kind == 2 ? osc::mixed_variant_name(variant) : kBatch[variant];
     if (!name || capacity <= (long long)std::strlen(n)) throw osc::Error{OSC_ERR_LENGTH, "name buffer too small"};
     std::strcpy(name, n);
     return OSC_OK;

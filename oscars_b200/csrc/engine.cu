@@ -146,6 +146,9 @@ void Engine::upload_trajectory(const double* pinned) {
   nknots_ = n;
   tstart_ = k.tstart;
   tstop_ = k.tstop;
+  x_start_[0] = k.y[0];
+  x_start_[1] = k.y[n];
+  x_start_[2] = k.y[2 * n];
   knots_version_ = model.knots_version;
   lev_filled_ = -1;
   mrec_filled_ = -1;
@@ -221,6 +224,13 @@ int request_levels(const osc_rad_opts& o, int max_supported, int* ext_from) {
   if (lstop < 0) throw Error{OSC_ERR_RANGE, "max_level -1 selects only extended levels, which this GPU build does not support"};
   *ext_from = lstop > lstop_mem ? lstop_mem : kMaxLevelMemory;
   return lstop;
+}
+
+// The trajectory's extent for the FP64 waves' phase bound.
+void Engine::set_phase_reach(FdWaveArgs& w) const {
+  for (int i = 0; i < 3; ++i) w.x_start[i] = x_start_[i];
+  w.t_abs = std::max(std::fabs(tstart_), std::fabs(tstop_));
+  w.t_len = tstop_ - tstart_;
 }
 
 // Make levels 0..L resident.
@@ -380,10 +390,14 @@ void polarization_vector(const osc_rad_opts& o, double P[6], bool& project) {
 // host round trip; entries still unconverged after it make the host extend the cache.
 constexpr int kPrefillLevel = 14;
 constexpr int kMinSpan = 32;
-// Sample-split flux / spectrum waves (FP64 and mixed): spans of at least one staged chunk, so that a
+// Sample-split mixed flux / spectrum waves: spans of at least one staged chunk, so that a
 // unit's fixed costs (its first copy, the partial store, the tile counter) stay small beside its
 // arithmetic.
 constexpr int kMinSpanSplit = 128;
+// FP64 waves: 64-sample spans (16 samples a thread) halve the serial part of waves too small to fill
+// the chip; 32 cost more in partial sums than they saved (51 x 51 map: 151 / 144 / 159 us of kernels at
+// 128 / 64 / 32).
+constexpr int kMinSpanFp64 = 64;
 
 int Engine::wave_grid(int kind, int variant) {
   if (wave_grid_[kind][variant] == 0) {
@@ -495,7 +509,7 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
   const int resident = wave_grid(kind, variant);  // CTAs resident at once on the device
   const int tile = rq.power_density ? (mixed ? pd_mixed_entries_per_cta() : 128)
                                     : (mixed ? mixed_entries_per_cta(variant) : fp64_entries_per_cta(variant));
-  const int min_span = rq.power_density ? kMinSpan : kMinSpanSplit;
+  const int min_span = rq.power_density ? kMinSpan : mixed ? kMinSpanSplit : kMinSpanFp64;
   const int64_t target = 4 * (int64_t)resident;   // >= 4 waves of equal units per launch
   const int64_t N = n_items;
   // Partial-sum buffer: a wave has tiles x spans units with spans the smallest power of two reaching
@@ -510,7 +524,7 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
   auto grid_for = [&](int L) -> int {
     if (L == Lfirst) {
       const WavePlan pl = wave_plan(1, L, N, tile, target, min_span);
-      return (int)std::min<int64_t>(pl.tiles * pl.spans, resident);
+      return (int)std::min<int64_t>(pl.tiles * pl.spans * pl.nseg, resident);
     }
     const int64_t span_max = wave_spans(L, 1, INT64_MAX, min_span);
     return (int)std::min<int64_t>(ntiles * span_max, resident);
@@ -630,6 +644,7 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
       w.n_e = (int64_t)rq.omega.size(); w.n_items = N; w.act = act_in; w.n_act = nact_in;
       w.first = first; w.level = L; w.tile_entries = tile; w.min_span = min_span; w.target_units = target;
       w.part = part_.as<double>(); w.err = cnt + kCntErr; w.work = fw + wv % 2;
+      set_phase_reach(w);
       w.fused = 1;
       w.tile_done = fz3 + 16;
       w.zero_u32 = fz3 + (wv + 2) % 3;

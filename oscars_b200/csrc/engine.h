@@ -136,6 +136,7 @@ class Engine {
   uint64_t knots_version_ = ~0ull;
   int64_t nknots_ = 0;
   double tstart_ = 0, tstop_ = 0;
+  double x_start_[3] = {0, 0, 0};  // first trajectory point
   // level cache
   DevBuf lev_;
   int64_t lev_cap_ = 0;
@@ -246,6 +247,7 @@ class Engine {
   void use_stream(cudaStream_t s);
   // model.knots to the device (pinned: the same knots laid out t | y | ypp | diag in pinned memory)
   void upload_trajectory(const double* pinned = nullptr);
+  void set_phase_reach(FdWaveArgs& w) const;
   void ensure_levels(int L);
   void reserve_levels(int L);
   void fill_levels(int64_t s_begin, int64_t s_end, cudaStream_t s);

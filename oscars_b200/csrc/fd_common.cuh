@@ -552,12 +552,31 @@ __device__ void fd_tile_finalize_grouped(const FdFinalArgs& A, const WavePlan& P
     double t[6] = {0, 0, 0, 0, 0, 0};
     double dm = 0;
     if (live) {
-      for (int sp = grp; sp < P.spans; sp += G) {
+      // kFinBatch spans' partials are in flight at a time: read one after another they cost an L2
+      // round trip each, which was most of a small wave's time at its 64 to 256 spans
+      constexpr int kFinBatch = 4;
+      int sp = grp;
+      for (; sp + (kFinBatch - 1) * G < P.spans; sp += kFinBatch * G) {
+        double v[kFinBatch][7];
+#pragma unroll
+        for (int b = 0; b < kFinBatch; ++b) {
+          const double* p = A.part + fused_part_index(P, tile, g, sp + b * G, 0, q, TE);
+#pragma unroll
+          for (int k = 0; k < 6; ++k) v[b][k] = __ldcg(p + k * TE);
+          v[b][6] = __ldcg(p + 8 * TE);
+        }
+#pragma unroll
+        for (int b = 0; b < kFinBatch; ++b) {
+#pragma unroll
+          for (int k = 0; k < 6; ++k) t[k] += v[b][k];
+          dm = fmax(dm, v[b][6]);  // -1: an empty span (they only trail the segment)
+        }
+      }
+      for (; sp < P.spans; sp += G) {
         const double* p = A.part + fused_part_index(P, tile, g, sp, 0, q, TE);
 #pragma unroll
         for (int k = 0; k < 6; ++k) t[k] += __ldcg(p + k * TE);
-        const double d = __ldcg(p + 8 * TE);
-        if (d >= 0) dm = fmax(dm, d);  // -1: an empty span (they only trail the segment)
+        dm = fmax(dm, __ldcg(p + 8 * TE));
       }
     }
     if (G > 1) {
@@ -605,15 +624,15 @@ __device__ void fd_tile_finalize_grouped(const FdFinalArgs& A, const WavePlan& P
                        A.samples, A.level_max);
 }
 
-// End of a unit of a fused wave with the grouped finalize (the mixed kernels): as fused_unit_done.
+// End of a unit of a fused wave with the grouped finalize: as fused_unit_done, for tiles of `units` units.
 template <int THREADS>
 __device__ __forceinline__ void fused_unit_done_grouped(const FdWaveArgs& A, const WavePlan& P, int64_t tile,
-                                                        int64_t n_act, int* s_last, int TE, double* red) {
+                                                        int64_t n_act, int* s_last, int TE, double* red, int units) {
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
     const unsigned done = atomicAdd(&A.tile_done[tile], 1u);
-    *s_last = done == (unsigned)(P.spans - 1);
+    *s_last = done == (unsigned)(units - 1);
     if (*s_last) __threadfence();
   }
   __syncthreads();

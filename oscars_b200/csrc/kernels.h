@@ -15,12 +15,14 @@ constexpr int kFdPartials = 9;  // 6 complex-sum components, first phase, last p
 // kernels skip sample 0); `spans` splits every segment so that tiles x spans reaches target_units.
 struct WavePlan {
   int nseg;
-  int spans;
+  int spans, log2_spans;
   int64_t tiles;
   int64_t seg_b[2], seg_e[2], span_len[2];
 };
 
-// Segments of a wave with a given span count (tiles left to the caller).
+// Segments of a wave with a given span count, a power of two (tiles left to the caller).  Shifts only:
+// the wave kernels form their plan in one thread before anything else can start, and 64-bit divisions
+// made that ~1 us of every launch.
 __host__ __device__ inline WavePlan wave_plan_spans(int first, int L, int spans) {
   WavePlan p;
   const int64_t lo = (int64_t)1 << L, hi = (int64_t)2 << L;
@@ -28,15 +30,18 @@ __host__ __device__ inline WavePlan wave_plan_spans(int first, int L, int spans)
   // segment 0: levels 0..L-1 on the first wave (level 0 alone when L == 0), else level L
   const int64_t b0 = first ? 1 : lo, e0 = first ? (L >= 1 ? lo : 2) : hi;
   const int64_t b1 = lo, e1 = hi;  // segment 1 (first wave with L >= 1): level L
+  int k = 0;
+  while ((1 << k) < spans) ++k;
   p.tiles = 0;
   p.spans = spans;
+  p.log2_spans = k;
   const int64_t a0 = b0 & ~(int64_t)1, a1 = b1 & ~(int64_t)1;
   p.seg_b[0] = a0;
   p.seg_e[0] = e0;
-  p.span_len[0] = ((e0 - a0 + spans - 1) / spans + 1) & ~(int64_t)1;
+  p.span_len[0] = (((e0 - a0 + spans - 1) >> k) + 1) & ~(int64_t)1;
   p.seg_b[1] = p.nseg == 2 ? a1 : 0;
   p.seg_e[1] = p.nseg == 2 ? e1 : 0;
-  p.span_len[1] = p.nseg == 2 ? (((e1 - a1 + spans - 1) / spans + 1) & ~(int64_t)1) : 0;
+  p.span_len[1] = p.nseg == 2 ? ((((e1 - a1 + spans - 1) >> k) + 1) & ~(int64_t)1) : 0;
   return p;
 }
 
@@ -44,14 +49,19 @@ __host__ __device__ inline WavePlan wave_plan_spans(int first, int L, int spans)
 // min_span samples of level L.
 __host__ __device__ inline int wave_spans(int L, int64_t tiles, int64_t target_units, int min_span) {
   const int64_t lo = (int64_t)1 << L;
-  int spans = 1;
-  while (tiles * spans < target_units && lo / (spans * 2) >= min_span) spans *= 2;
-  return spans;
+  int k = 0;
+  while ((tiles << k) < target_units && (lo >> (k + 1)) >= min_span) ++k;
+  return 1 << k;
+}
+
+// Tiles of tile_entries (entry counts stay below 2^31).
+__host__ __device__ inline int64_t wave_tiles(int64_t n_act, int tile_entries) {
+  return (int64_t)(((unsigned)n_act + (unsigned)tile_entries - 1u) / (unsigned)tile_entries);
 }
 
 __host__ __device__ inline WavePlan wave_plan(int first, int L, int64_t n_act, int tile_entries, int64_t target_units,
                                               int min_span) {
-  const int64_t tiles = (n_act + tile_entries - 1) / tile_entries;
+  const int64_t tiles = wave_tiles(n_act, tile_entries);
   WavePlan p = wave_plan_spans(first, L, wave_spans(L, tiles, target_units, min_span));
   p.tiles = tiles;
   return p;
@@ -96,6 +106,7 @@ struct FdWaveArgs {
   const unsigned* n_act;    // device count of `act`
   int first, level, tile_entries, min_span;
   int64_t target_units;
+  double x_start[3], t_abs, t_len;  // FP64 waves: first trajectory point, max |t|, duration (phase_reach)
   double* part;             // partials, entry-major: [slot][seg][span][kFdPartials]; fused: see below
   unsigned* err;
   unsigned long long* work;  // next unit to take (zero at launch; the finalize resets it)
@@ -214,6 +225,7 @@ const char* mixed_variant_name(int variant);  // kernel and template arguments o
 int mixed_blocks_per_sm(int variant);
 int fp64_blocks_per_sm(bool power_density, int variant);
 int fp64_entries_per_cta(int variant);
+const char* fp64_variant_name(int variant);
 
 // FP64 level samples [s_begin, s_end) (10 SoA arrays of stride cap) and their per-level beta-difference
 // maxima; levels above ext_from are the reference's extended levels.

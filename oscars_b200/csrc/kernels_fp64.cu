@@ -100,18 +100,68 @@ constexpr int kFdChunk = 128;
 __device__ __forceinline__ double fd_phase(double T, double X, double Y, double Z, double Ox, double Oy, double Oz,
                                            double mw) {
   const double Rx = __dsub_rn(Ox, X), Ry = __dsub_rn(Oy, Y), Rz = __dsub_rn(Oz, Z);
-  const double D = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(Rx, Rx), __dmul_rn(Ry, Ry)), __dmul_rn(Rz, Rz)));
-  return __dmul_rn(mw, __dadd_rn(T, __ddiv_rn(D, kCLight)));
+  const double s = __dadd_rn(__dadd_rn(__dmul_rn(Rx, Rx), __dmul_rn(Ry, Ry)), __dmul_rn(Rz, Rz));
+  return __dmul_rn(mw, __dadd_rn(T, over_c(sqrt_by(s, rsqrt_near(s)))));
+}
+
+// Retarded time t + D/c and amplitude of one sample for an observer.  D, n and 1 - n.b round as the
+// reference's operations do (their last bits move the phase and the ill-conditioned 1 - n.b); the rest
+// is well conditioned and is formed with FMA from n x (u x a) = u (n.a) - a (n.u), u = n - b:
+//   e = u k1 - a k2,  k1 = ((1 - b^2) / D + n.a) / (D om^2),  k2 = (n.u) / (D om^2),  om = 1 - n.b.
+// 59 FP64 operations (with the library's square root and six divisions: ~115).
+struct FdTerm {
+  double tau, ex, ey, ez;
+};
+__device__ __forceinline__ FdTerm fd_term(double T, double X, double Y, double Z, double bx, double by, double bz,
+                                          double ax, double ay, double az, double ob2, double Ox, double Oy, double Oz) {
+  const double Rx = __dsub_rn(Ox, X), Ry = __dsub_rn(Oy, Y), Rz = __dsub_rn(Oz, Z);
+  const double s = __dadd_rn(__dadd_rn(__dmul_rn(Rx, Rx), __dmul_rn(Ry, Ry)), __dmul_rn(Rz, Rz));
+  const double y = rsqrt_near(s), D = sqrt_by(s, y);
+  FdTerm f;
+  f.tau = __dadd_rn(T, over_c(D));
+  const double nx = quot_by(Rx, D, y), ny = quot_by(Ry, D, y), nz = quot_by(Rz, D, y);
+  const double om =
+      __dsub_rn(1.0, __dadd_rn(__dadd_rn(__dmul_rn(nx, bx), __dmul_rn(ny, by)), __dmul_rn(nz, bz)));
+  const double ux = __dsub_rn(nx, bx), uy = __dsub_rn(ny, by), uz = __dsub_rn(nz, bz);
+  const double na = fma(nx, ax, fma(ny, ay, nz * az));
+  const double nu = fma(nx, ux, fma(ny, uy, nz * uz));
+  const double io = rcp_near(om);
+  const double f2 = y * io * io;
+  const double k1 = f2 * fma(ob2, y, na), k2 = -(f2 * nu);
+  f.ex = fma(ux, k1, ax * k2);
+  f.ey = fma(uy, k1, ay * k2);
+  f.ez = fma(uz, k1, az * k2);
+  return f;
+}
+
+// 1 - b^2 of a sample, in the reference's operations.
+__device__ __forceinline__ double one_minus_b2(double bx, double by, double bz) {
+  return __dsub_rn(1.0, __dadd_rn(__dadd_rn(__dmul_rn(bx, bx), __dmul_rn(by, by)), __dmul_rn(bz, bz)));
+}
+
+// Bound of |w (t + D/c)| over a trajectory: it starts at A.x_start, lasts A.t_len and its times lie
+// within A.t_abs of zero, and the particle is slower than light.
+__device__ __forceinline__ double phase_reach(const FdWaveArgs& A, double Ox, double Oy, double Oz, double mw) {
+  const double dx = Ox - A.x_start[0], dy = Oy - A.x_start[1], dz = Oz - A.x_start[2];
+  return fabs(mw) * (A.t_abs + A.t_len + sqrt(dx * dx + dy * dy + dz * dz) * kInvC1);
 }
 
 // Sample-split FP64 sum: the CTA's 128 threads form SUB groups of TE = 128 / SUB threads, one entry
 // per thread; group g takes the g-th of SUB equal parts of every staged chunk of the 10 level arrays.
 // Each part starts from the phase of the sample before it (the chunk's previous sample, the previous
-// chunk's last one, or the span's predecessor read from the level cache), so the largest phase step
-// of a span covers exactly the consecutive pairs of the serial order and spans need no joining
-// (dmax_spans_joined); the groups' sums are combined in shared memory in group order.  Fused waves
-// finalize their tiles with all threads (fused_unit_done_grouped); unfused waves store entry-major
-// partials for k_fd_finalize.
+// chunk's last one, or the span's predecessor read from the level cache), so the phase steps of a
+// span cover exactly the consecutive pairs of the serial order and spans need no joining
+// (dmax_spans_joined); the stop rule only asks whether a step reaches pi, so a span stores pi or 0 in the
+// place of its largest step.  The groups' sums are combined in shared memory in group order.  Fused
+// waves finalize their tiles with all threads (fused_unit_done_grouped); unfused waves store
+// entry-major partials for k_fd_finalize.
+//
+// Bound by the FP64 pipe: 95 instructions per (entry, sample) at one per two cycles and
+// sub-partition, 71 % of its cycles busy in the first wave of a 201 x 201 map (with the library's
+// divisions, square root and sincos: ~165 instructions at 64 %).  1 - b^2 depends on the sample
+// alone and is formed once per staged chunk.  What a unit waits for before its first sample is
+// requested early: the next unit's number at the start of this one, its first chunk during this one's
+// last, the span's predecessor before the observer.
 template <int SUB, int MINB>
 __global__ void __launch_bounds__(kFdThreads, MINB) k_fd_wave_fp64(FdWaveArgs A) {
   constexpr int TE = kFdThreads / SUB;
@@ -120,8 +170,13 @@ __global__ void __launch_bounds__(kFdThreads, MINB) k_fd_wave_fp64(FdWaveArgs A)
     return;
   }
   __shared__ __align__(16) Stage<10, kFdChunk> st;
+  __shared__ double ob2[kFdChunk + 2];
   __shared__ double red[SUB > 1 ? SUB - 1 : 1][7][TE];
   __shared__ int s_last;
+  __shared__ int64_t next_unit;
+  // the plan is uniform over the CTA; keeping it in shared memory frees the registers its
+  // fields would otherwise hold across the sample loop
+  __shared__ WavePlan P;
   const int tid = threadIdx.x;
   const int grp = tid / TE, q = tid % TE;
   if (A.fused && blockIdx.x == 0 && tid == 0) {  // counters of the following wave
@@ -129,171 +184,163 @@ __global__ void __launch_bounds__(kFdThreads, MINB) k_fd_wave_fp64(FdWaveArgs A)
     if (A.zero_u64) *A.zero_u64 = 0;
   }
   const int64_t n_act = A.act ? (int64_t)*A.n_act : A.n_items;
-  // the plan is uniform over the CTA; keeping it in shared memory frees the registers its
-  // fields would otherwise hold across the sample loop
-  __shared__ WavePlan P;
-  if (threadIdx.x == 0) P = wave_plan(A.first, A.level, n_act, TE, A.target_units, A.min_span);
-  __syncthreads();
-  const int64_t units = P.tiles * P.spans;
   if (tid == 0) {
+    P = wave_plan(A.first, A.level, n_act, TE, A.target_units, A.min_span);
     mbar_init(&st.bar[0], 1);
     mbar_init(&st.bar[1], 1);
     fence_barrier_init();
   }
   __syncthreads();
-  uint32_t phase_bits = 0;  // parity of the next completion expected on each buffer
-  __shared__ int64_t next_unit;
-  for (;;) {  // CTAs take (tile, span) units from a shared counter until the wave's units run out
-    if (tid == 0) next_unit = (int64_t)atomicAdd(A.work, 1ull);
-    __syncthreads();
-    const int64_t u = next_unit;
-    __syncthreads();
-    if (u >= units) break;
-    const int64_t tile = u / P.spans;
-    const int span = (int)(u % P.spans);
+  // units (tile, segment, span), spans fastest: the first is the CTA's own, the others come from a
+  // shared counter until the wave's units run out
+  const int64_t units = (P.tiles * P.nseg) << P.log2_spans;
+  auto unit_range = [&](int64_t u, int64_t& b0, int64_t& b1) {
+    const int64_t r = u >> P.log2_spans;
+    const int g = P.nseg == 2 ? (int)(r & 1) : 0;
+    b0 = seg_begin(P, g) + (u & (P.spans - 1)) * seg_span(P, g);
+    b1 = min(seg_end(P, g), b0 + seg_span(P, g));
+  };
+  auto issue = [&](int64_t lo, int64_t end, int b) {  // chunk [lo, lo + kFdChunk) of a range ending at end
+    const int64_t hi = min(end, lo + kFdChunk);
+    stage_issue<10, kFdChunk>(st, b, A.lev, A.cap, lo & ~(int64_t)1, (hi + 1) & ~(int64_t)1);
+  };
+  uint32_t staged = 0;  // chunks taken so far: buffer staged & 1, its completion parity (staged >> 1) & 1
+  int64_t u = blockIdx.x;
+  if (tid == 0 && u < units) {
+    int64_t b0, b1;
+    unit_range(u, b0, b1);
+    if (b0 < b1) issue(b0, b1, 0);
+  }
+  while (u < units) {
+    int64_t after = 0;
+    if (tid == 0) after = (int64_t)gridDim.x + (int64_t)atomicAdd(A.work, 1ull);
+    int64_t b0, b1;
+    unit_range(u, b0, b1);
+    const int64_t nchunks = b1 > b0 ? (b1 - b0 + kFdChunk - 1) / kFdChunk : 0;
+    const int span = (int)u & (P.spans - 1);
+    const int g = P.nseg == 2 ? (int)(u >> P.log2_spans) & 1 : 0;
+    const int64_t tile = u >> (P.log2_spans + P.nseg - 1);
+    // the sample before the span (sample 0, the unused slot, never is one)
+    const bool joins = span > 0 && nchunks > 0 && b0 - 1 >= 1;
+    double cT = 0, cX = 0, cY = 0, cZ = 0;
+    if (joins) {
+      const double* c = A.lev + (b0 - 1);
+      cT = c[0]; cX = c[A.cap]; cY = c[2 * A.cap]; cZ = c[3 * A.cap];
+    }
     const int64_t slot = tile * TE + q;
     const bool live = slot < n_act;
-    const int64_t item = live ? (A.act ? (int64_t)A.act[slot] : slot) : 0;
-    const int64_t io = item / A.n_e, ie = item % A.n_e;
-    const double Ox = A.obs[3 * io], Oy = A.obs[3 * io + 1], Oz = A.obs[3 * io + 2];
+    const unsigned item = live ? (A.act ? (unsigned)A.act[slot] : (unsigned)slot) : 0u;
+    const unsigned io = item / (unsigned)A.n_e, ie = item - io * (unsigned)A.n_e;
+    const double* ob = A.obs + 3 * (int64_t)io;
+    const double Ox = ob[0], Oy = ob[1], Oz = ob[2];
     const double mw = -A.omega[ie];
-    for (int g = 0; g < P.nseg; ++g) {
-      const int64_t b0 = seg_begin(P, g) + (int64_t)span * seg_span(P, g);
-      const int64_t b1 = min(seg_end(P, g), b0 + seg_span(P, g));
-      double sxr = 0, sxi = 0, syr = 0, syi = 0, szr = 0, szi = 0;
-      double dmax = 0;
-      bool any = false;
-      const int64_t nchunks = b1 > b0 ? (b1 - b0 + kFdChunk - 1) / kFdChunk : 0;
-      // phase of the sample before a part that starts a chunk: the span's predecessor (span > 0;
-      // sample 0, the unused slot, never is one), then the previous chunk's last sample
-      double carry = 0;
-      bool have_carry = false;
-      if (live && span > 0 && nchunks > 0 && b0 - 1 >= 1) {
-        const int64_t s = b0 - 1;
-        const double* L = A.lev;
-        carry = fd_phase(L[s], L[A.cap + s], L[2 * A.cap + s], L[3 * A.cap + s], Ox, Oy, Oz, mw);
-        have_carry = true;
-      }
-      if (tid == 0 && nchunks > 0) {
-        const int64_t lo = b0, hi = min(b1, b0 + kFdChunk);
-        stage_issue<10, kFdChunk>(st, 0, A.lev, A.cap, lo & ~(int64_t)1, (hi + 1) & ~(int64_t)1);
-      }
-      for (int64_t c = 0; c < nchunks; ++c) {
-        const int buf = (int)(c & 1);
-        const int64_t lo = b0 + c * kFdChunk, hi = min(b1, lo + kFdChunk);
-        if (tid == 0 && c + 1 < nchunks) {  // prefetch the next chunk into the other buffer
-          const int64_t lo2 = lo + kFdChunk, hi2 = min(b1, lo2 + kFdChunk);
-          stage_issue<10, kFdChunk>(st, buf ^ 1, A.lev, A.cap, lo2 & ~(int64_t)1, (hi2 + 1) & ~(int64_t)1);
+    const bool near = phase_reach(A, Ox, Oy, Oz, mw) < kPhaseFast;  // (false for NaN)
+    // phase of the sample before a part that starts a chunk: the span's predecessor, then the previous
+    // chunk's last sample (NaN: no step into the segment's first sample)
+    double carry = __longlong_as_double(0x7ff8000000000000ll);
+    if (joins) carry = fd_phase(cT, cX, cY, cZ, Ox, Oy, Oz, mw);
+    double sxr = 0, sxi = 0, syr = 0, syi = 0, szr = 0, szi = 0;
+    bool wide = false;  // a phase step of pi or more
+    bool any = false;
+    for (int64_t c = 0; c < nchunks; ++c, ++staged) {
+      const int buf = (int)(staged & 1u);
+      const int64_t lo = b0 + c * kFdChunk, hi = min(b1, lo + kFdChunk);
+      if (tid == 0) {  // the chunk after this one, of this unit or the next, into the other buffer
+        if (c + 1 < nchunks) {
+          issue(lo + kFdChunk, b1, buf ^ 1);
+        } else if (after < units) {
+          int64_t n0, n1;
+          unit_range(after, n0, n1);
+          if (n0 < n1) issue(n0, n1, buf ^ 1);
         }
-        if (!mbar_wait(&st.bar[buf], (phase_bits >> buf) & 1u)) {
-          if (tid == 0) atomicOr(A.err, kErrTmaTimeout);
-          return;
-        }
-        phase_bits ^= 1u << buf;
-        const int64_t lo_al = lo & ~(int64_t)1;
-        const double* sT = st.v[buf][0];
-        const double* sX = st.v[buf][1];
-        const double* sY = st.v[buf][2];
-        const double* sZ = st.v[buf][3];
-        const double* sBx = st.v[buf][4];
-        const double* sBy = st.v[buf][5];
-        const double* sBz = st.v[buf][6];
-        const double* sAx = st.v[buf][7];
-        const double* sAy = st.v[buf][8];
-        const double* sAz = st.v[buf][9];
-        const int ja = (int)(max(lo, (int64_t)1) - lo_al);  // sample 0 is the unused slot
-        const int jb = (int)(hi - lo_al);
-        const int j0 = ja + ((jb - ja) * grp) / SUB, j1 = ja + ((jb - ja) * (grp + 1)) / SUB;  // this group's part
-        if (live && j0 < j1) {
-          double last;
-          bool have;
-          if (j0 > ja) {
-            last = fd_phase(sT[j0 - 1], sX[j0 - 1], sY[j0 - 1], sZ[j0 - 1], Ox, Oy, Oz, mw);
-            have = true;
-          } else {
-            last = carry;
-            have = have_carry;
-          }
+      }
+      if (!mbar_wait(&st.bar[buf], (staged >> 1) & 1u)) {
+        if (tid == 0) atomicOr(A.err, kErrTmaTimeout);
+        return;
+      }
+      const int64_t lo_al = lo & ~(int64_t)1;
+      const double* sT = st.v[buf][0];
+      const double* sX = st.v[buf][1];
+      const double* sY = st.v[buf][2];
+      const double* sZ = st.v[buf][3];
+      const double* sBx = st.v[buf][4];
+      const double* sBy = st.v[buf][5];
+      const double* sBz = st.v[buf][6];
+      const double* sAx = st.v[buf][7];
+      const double* sAy = st.v[buf][8];
+      const double* sAz = st.v[buf][9];
+      const int ja = (int)(max(lo, (int64_t)1) - lo_al);  // sample 0 is the unused slot
+      const int jb = (int)(hi - lo_al);
+      const int j0 = ja + ((jb - ja) * grp) / SUB, j1 = ja + ((jb - ja) * (grp + 1)) / SUB;  // this group's part
+      for (int j = tid; j < jb; j += kFdThreads) ob2[j] = one_minus_b2(sBx[j], sBy[j], sBz[j]);
+      __syncthreads();
+      if (live && j0 < j1) {
+        double last = carry;
+        if (j0 > ja) last = fd_phase(sT[j0 - 1], sX[j0 - 1], sY[j0 - 1], sZ[j0 - 1], Ox, Oy, Oz, mw);
+        auto sum = [&](auto trig) {
+#pragma unroll 2
           for (int j = j0; j < j1; ++j) {
-            const double T = sT[j];
-            const double Rx = __dsub_rn(Ox, sX[j]), Ry = __dsub_rn(Oy, sY[j]), Rz = __dsub_rn(Oz, sZ[j]);
-            const double D = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(Rx, Rx), __dmul_rn(Ry, Ry)), __dmul_rn(Rz, Rz)));
-            const double ph = __dmul_rn(mw, __dadd_rn(T, __ddiv_rn(D, kCLight)));
-            if (have) {
-              const double dp = fabs(__dsub_rn(ph, last));
-              dmax = dp > dmax ? dp : dmax;
-            }
-            have = true;
+            const FdTerm f = fd_term(sT[j], sX[j], sY[j], sZ[j], sBx[j], sBy[j], sBz[j], sAx[j], sAy[j], sAz[j], ob2[j],
+                                     Ox, Oy, Oz);
+            const double ph = __dmul_rn(mw, f.tau);
+            wide |= fabs(__dsub_rn(ph, last)) >= kPiD;
             last = ph;
-            const double bx = sBx[j], by = sBy[j], bz = sBz[j];
-            const double nx = __ddiv_rn(Rx, D), ny = __ddiv_rn(Ry, D), nz = __ddiv_rn(Rz, D);
-            const double b2 = __dadd_rn(__dadd_rn(__dmul_rn(bx, bx), __dmul_rn(by, by)), __dmul_rn(bz, bz));
-            const double ndb = __dadd_rn(__dadd_rn(__dmul_rn(nx, bx), __dmul_rn(ny, by)), __dmul_rn(nz, bz));
-            const double om = __dsub_rn(1.0, ndb);
-            const double p2 = __dmul_rn(om, om);
-            const double den1 = __dmul_rn(__dmul_rn(D, D), p2);
-            const double den2 = __dmul_rn(D, p2);
-            const double ob2 = __dsub_rn(1.0, b2);
-            const double ux = __dsub_rn(nx, bx), uy = __dsub_rn(ny, by), uz = __dsub_rn(nz, bz);
-            const double ax = sAx[j], ay = sAy[j], az = sAz[j];
-            const double wx = __dsub_rn(__dmul_rn(uy, az), __dmul_rn(ay, uz));
-            const double wy = __dsub_rn(__dmul_rn(uz, ax), __dmul_rn(az, ux));
-            const double wz = __dsub_rn(__dmul_rn(ux, ay), __dmul_rn(ax, uy));
-            const double vx = __dsub_rn(__dmul_rn(ny, wz), __dmul_rn(wy, nz));
-            const double vy = __dsub_rn(__dmul_rn(nz, wx), __dmul_rn(wz, nx));
-            const double vz = __dsub_rn(__dmul_rn(nx, wy), __dmul_rn(wx, ny));
-            // The two amplitude terms need only relative accuracy: one quotient per term, then
-            // multiplications (the reference divides each component; the difference is ~1 ulp).
-            const double f1 = ob2 / den1, f2 = 1.0 / den2;
-            const double ex = fma(ux, f1, vx * f2);
-            const double ey = fma(uy, f1, vy * f2);
-            const double ez = fma(uz, f1, vz * f2);
             double sn, cs;
-            sincos(reduce_2pi(ph), &sn, &cs);
-            sxr = fma(ex, cs, sxr); sxi = fma(ex, sn, sxi);
-            syr = fma(ey, cs, syr); syi = fma(ey, sn, syi);
-            szr = fma(ez, cs, szr); szi = fma(ez, sn, szi);
+            trig(ph, &sn, &cs);
+            sxr = fma(f.ex, cs, sxr); sxi = fma(f.ex, sn, sxi);
+            syr = fma(f.ey, cs, syr); syi = fma(f.ey, sn, syi);
+            szr = fma(f.ez, cs, szr); szi = fma(f.ez, sn, szi);
           }
-          any = true;
-        }
-        if (live && c + 1 < nchunks) {  // a full chunk: its last sample precedes the next chunk
-          const int jl = jb - 1;
-          carry = fd_phase(sT[jl], sX[jl], sY[jl], sZ[jl], Ox, Oy, Oz, mw);
-          have_carry = true;
-        }
-        __syncthreads();  // everyone is done with `buf` before it is refilled
+        };
+        if (near) sum([](double ph, double* sn, double* cs) { sincos_fast(ph, sn, cs); });
+        else sum([](double ph, double* sn, double* cs) { sincos_far(ph, sn, cs); });
+        any = true;
       }
-      // combine the groups' sums in group order; group 0 stores the span's partial
-      double S[6] = {sxr, sxi, syr, syi, szr, szi};
-      double dm = any ? dmax : -1.0;
-      if (SUB > 1) {
-        if (grp > 0) {
-#pragma unroll
-          for (int k = 0; k < 6; ++k) red[grp - 1][k][q] = S[k];
-          red[grp - 1][6][q] = dm;
-        }
-        __syncthreads();
-        if (grp == 0)
-          for (int o = 0; o < SUB - 1; ++o) {
-#pragma unroll
-            for (int k = 0; k < 6; ++k) S[k] += red[o][k][q];
-            dm = fmax(dm, red[o][6][q]);
-          }
-        __syncthreads();
+      if (live && c + 1 < nchunks) {  // a full chunk: its last sample precedes the next chunk
+        const int jl = jb - 1;
+        carry = fd_phase(sT[jl], sX[jl], sY[jl], sZ[jl], Ox, Oy, Oz, mw);
       }
-      if (live && grp == 0) {
-        // entry-major for the finalize kernel (an entry's spans contiguous); tile-major when fused
-        double* p = A.fused ? A.part + fused_part_index(P, tile, g, span, 0, q, TE)
-                            : A.part + (slot * P.nseg * P.spans + g * P.spans + span) * kFdPartials;
-        const int64_t cs = A.fused ? TE : 1;  // stride between components
-#pragma unroll
-        for (int k = 0; k < 6; ++k) p[k * cs] = S[k];
-        p[6 * cs] = 0.0;
-        p[7 * cs] = 0.0;
-        p[8 * cs] = dm;  // -1 marks an empty span
-      }
+      __syncthreads();  // everyone is done with `buf` before it is refilled
     }
-    if (A.fused) fused_unit_done_grouped<kFdThreads>(A, P, tile, n_act, &s_last, TE, &red[0][0][0]);
+    if (nchunks == 0) {  // (no unit of a planned wave is empty)
+      if (tid == 0 && after < units) {
+        int64_t n0, n1;
+        unit_range(after, n0, n1);
+        if (n0 < n1) issue(n0, n1, (int)(staged & 1u));
+      }
+      __syncthreads();
+    }
+    // combine the groups' sums in group order; group 0 stores the span's partial
+    double S[6] = {sxr, sxi, syr, syi, szr, szi};
+    double dm = any ? (wide ? kPiD : 0.0) : -1.0;
+    if (SUB > 1) {
+      if (grp > 0) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) red[grp - 1][k][q] = S[k];
+        red[grp - 1][6][q] = dm;
+      }
+      __syncthreads();
+      if (grp == 0)
+        for (int o = 0; o < SUB - 1; ++o) {
+#pragma unroll
+          for (int k = 0; k < 6; ++k) S[k] += red[o][k][q];
+          dm = fmax(dm, red[o][6][q]);
+        }
+    }
+    if (live && grp == 0) {
+      // entry-major for the finalize kernel (an entry's spans contiguous); tile-major when fused
+      double* p = A.fused ? A.part + fused_part_index(P, tile, g, span, 0, q, TE)
+                          : A.part + (slot * P.nseg * P.spans + g * P.spans + span) * kFdPartials;
+      const int64_t cs = A.fused ? TE : 1;  // stride between components
+#pragma unroll
+      for (int k = 0; k < 6; ++k) p[k * cs] = S[k];
+      if (!A.fused) p[6] = p[7] = 0.0;  // no step left to join between spans
+      p[8 * cs] = dm;  // -1 marks an empty span
+    }
+    if (tid == 0) next_unit = after;
+    if (A.fused) fused_unit_done_grouped<kFdThreads>(A, P, tile, n_act, &s_last, TE, &red[0][0][0], P.nseg * P.spans);
+    else __syncthreads();
+    u = next_unit;
   }
 }
 
@@ -513,18 +560,31 @@ cudaError_t launch_level_fill(const double* knots, int64_t n, double tstart, dou
   return cudaGetLastError();
 }
 
-// Compiled variants of the FP64 wave kernel: (groups SUB of 128 / SUB entries, minimum CTAs per SM).
-// Variant 0 keeps 128 entries per CTA (the allocation-free entry point sizes its partials for it).
-static const int kFp64Sub[kFp64Variants] = {1, 2, 4, 4};
+// Compiled variants of the FP64 wave kernel: groups SUB of 128 / SUB entries, minimum CTAs per SM.
+// Variant 0 keeps 128 entries per CTA (the allocation-free entry point sizes its partials for it); the
+// others trade registers for resident warps (132, 122 and 80 a thread): 3 to 6 CTAs measured within 3 %
+// of each other on a 201 x 201 map, fewer the better on small grids, so the autotuner chooses.
+#define OSC_FP64_VARIANTS(X) \
+  X(0, 1, 7)                 \
+  X(1, 4, 3)                 \
+  X(2, 4, 4)                 \
+  X(3, 4, 6)
+
+#define OSC_SUB(i, sub, minb) sub,
+static const int kFp64Sub[kFp64Variants] = {OSC_FP64_VARIANTS(OSC_SUB)};
 
 int fp64_entries_per_cta(int variant) { return dev::kFdThreads / kFp64Sub[variant]; }
+const char* fp64_variant_name(int variant) {
+#define OSC_NAME(i, sub, minb) "k_fd_wave_fp64<" #sub "," #minb ">",
+  static const char* const kNames[kFp64Variants] = {OSC_FP64_VARIANTS(OSC_NAME)};
+  return variant >= 0 && variant < kFp64Variants ? kNames[variant] : "";
+}
 
 cudaError_t launch_fd_wave_fp64(const FdWaveArgs& a, int grid, int variant, cudaStream_t st) {
   switch (variant) {
-    case 1: dev::k_fd_wave_fp64<2, 7><<<grid, dev::kFdThreads, 0, st>>>(a); break;
-    case 2: dev::k_fd_wave_fp64<4, 7><<<grid, dev::kFdThreads, 0, st>>>(a); break;
-    case 3: dev::k_fd_wave_fp64<4, 5><<<grid, dev::kFdThreads, 0, st>>>(a); break;
-    default: dev::k_fd_wave_fp64<1, 7><<<grid, dev::kFdThreads, 0, st>>>(a); break;
+#define OSC_LAUNCH(i, sub, minb) \
+    case i: dev::k_fd_wave_fp64<sub, minb><<<grid, dev::kFdThreads, 0, st>>>(a); break;
+    OSC_FP64_VARIANTS(OSC_LAUNCH)
   }
   return cudaGetLastError();
 }
@@ -556,10 +616,9 @@ int fp64_blocks_per_sm(bool power_density, int variant) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dev::k_pd_wave_fp64, dev::kPdThreads, 0);
   } else {
     switch (variant) {
-      case 1: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dev::k_fd_wave_fp64<2, 7>, dev::kFdThreads, 0); break;
-      case 2: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dev::k_fd_wave_fp64<4, 7>, dev::kFdThreads, 0); break;
-      case 3: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dev::k_fd_wave_fp64<4, 5>, dev::kFdThreads, 0); break;
-      default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dev::k_fd_wave_fp64<1, 7>, dev::kFdThreads, 0); break;
+#define OSC_OCC(i, sub, minb) \
+      case i: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dev::k_fd_wave_fp64<sub, minb>, dev::kFdThreads, 0); break;
+      OSC_FP64_VARIANTS(OSC_OCC)
     }
   }
   return n > 0 ? n : 1;

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kMxThreads, MINB) k_fd_wave_mixed_pair(FdWaveA
       }
       if (SUB > 1) __syncthreads();
     }
-    if (A.fused) fused_unit_done_grouped<kMxThreads>(A, P, tile, n_act, &s_last, TE, &red[0][0][0]);
+    if (A.fused) fused_unit_done_grouped<kMxThreads>(A, P, tile, n_act, &s_last, TE, &red[0][0][0], P.spans);
   }
 }
 

@@ -223,6 +223,8 @@ extern "C" OSC_API int osc_flux_fixed_level_noalloc(int device, const double* tr
     FdWaveArgs a{};
     a.lev = lev; a.cap = cap; a.obs = obs; a.omega = omega; a.n_e = 1; a.n_items = n_obs;
     a.act = nullptr; a.n_act = nullptr; a.first = 1; a.level = level; a.tile_entries = 128; a.min_span = 32;
+    for (int i = 0; i < 3; ++i) a.x_start[i] = trajectory[(1 + i) * n];
+    a.t_abs = std::fmax(std::fabs(tstart), std::fabs(tstop)); a.t_len = tstop - tstart;
     a.target_units = 1; a.part = part; a.err = cnt + 2; a.work = c64 + 2;  // zeroed with the counters
     e = launch_fd_wave_fp64(a, (int)(plan.tiles * plan.spans), 0, st);
   }
