@@ -55,6 +55,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
+// Programmatic dependent launch: a wave lets the next one's CTAs become resident as soon as its own are
+// (launch_dependents), and a wave launched that way waits for its predecessor's end, with its memory
+// visible, before it touches anything the predecessor writes (wait).  Without the launch attribute both
+// do nothing.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Bulk copy `bytes` (multiple of 16, both addresses 16-byte aligned) from global to shared memory,
 // completing on `bar`.
 __device__ __forceinline__ void tma_load_1d(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar) {
@@ -173,4 +180,21 @@ __device__ __forceinline__ void sincos_fast(double phi, double* sn, double* cs) 
 static __device__ __noinline__ void sincos_far(double phi, double* sn, double* cs) { sincos(reduce_2pi(phi), sn, cs); }
 
 }  // namespace dev
+
+// Launch that may overlap its predecessor's tail on the stream (the kernel calls wait_predecessor()):
+// 2 to 3 us less between the waves of a request.
+template <class... P, class... A>
+inline cudaError_t launch_overlapped(void (*kernel)(P...), int grid, int threads, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)threads);
+  c.stream = st;
+  cudaLaunchAttribute a{};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &a;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 }  // namespace osc

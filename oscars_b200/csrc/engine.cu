@@ -405,6 +405,7 @@ int Engine::wave_grid(int kind, int variant) {
     check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "attr");
     const int per = kind == 2   ? mixed_blocks_per_sm(variant)
                     : kind == 4 ? pd_mixed_blocks_per_sm()
+                    : kind >= 5 ? lines_blocks_per_sm(kind == 6)
                                 : fp64_blocks_per_sm(kind == 1, variant);
     wave_grid_[kind][variant] = sms * per;
   }
@@ -504,12 +505,19 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
   const auto hist = prefill_hist_.find(hist_key);
   const int Lpre_want = hist != prefill_hist_.end() ? hist->second : kPrefillLevel;
   const int Lpre = std::min(lstop, std::max(Lfirst, Lpre_want));
-  const int variant = tuning_ ? current_variant_[kind]
+  // One observer: the line kernels, unless a variant of the general kernels is pinned (the mixed one from
+  // level 9 on, where every span is a whole number of its FP32 folds)
+  const bool lines = !rq.power_density && rq.n_obs == 1 && forced_variant[kind] < 0 && (!mixed || Lfirst == 9);
+  const int variant = lines ? 0 : tuning_ ? current_variant_[kind]
                               : pick_variant(kind, const_cast<RadRequest&>(rq), n_items, Lfirst, lstop, d_out, d_lvl, st);
-  const int resident = wave_grid(kind, variant);  // CTAs resident at once on the device
+  const int resident = wave_grid(lines ? (mixed ? 6 : 5) : kind, variant);  // CTAs resident at once on the device
   const int tile = rq.power_density ? (mixed ? pd_mixed_entries_per_cta() : 128)
+                   : lines ? lines_entries_per_cta()
                                     : (mixed ? mixed_entries_per_cta(variant) : fp64_entries_per_cta(variant));
-  const int min_span = rq.power_density ? kMinSpan : mixed ? kMinSpanSplit : kMinSpanFp64;
+  // At most 64 spans: beyond, the finalizer's pass over a tile's spans costs more than shorter units save.
+  auto min_span = [&](int L) {
+    return rq.power_density ? kMinSpan : std::max(mixed ? kMinSpanSplit : kMinSpanFp64, L > 6 ? 1 << (L - 6) : 1);
+  };
   const int64_t target = 4 * (int64_t)resident;   // >= 4 waves of equal units per launch
   const int64_t N = n_items;
   // Partial-sum buffer: a wave has tiles x spans units with spans the smallest power of two reaching
@@ -523,10 +531,10 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
   // which reaches the target (> resident) once t x (largest span count of the level) does.
   auto grid_for = [&](int L) -> int {
     if (L == Lfirst) {
-      const WavePlan pl = wave_plan(1, L, N, tile, target, min_span);
+      const WavePlan pl = wave_plan(1, L, N, tile, target, min_span(L));
       return (int)std::min<int64_t>(pl.tiles * pl.spans * pl.nseg, resident);
     }
-    const int64_t span_max = wave_spans(L, 1, INT64_MAX, min_span);
+    const int64_t span_max = wave_spans(L, 1, INT64_MAX, min_span(L));
     return (int)std::min<int64_t>(ntiles * span_max, resident);
   };
   part_.reserve(sizeof(double) * part_doubles);
@@ -614,7 +622,7 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
       w.lev = reinterpret_cast<const double*>(mrec_.p);
       w.cap = lev_cap_; w.obs = d_obs; w.normals = d_nrm; w.has_normal = d_nrm != nullptr;
       w.directional = rq.directional; w.n_items = N; w.act = act_in; w.n_act = nact_in;
-      w.first = first; w.level = L; w.tile_entries = tile; w.min_span = min_span; w.target_units = target;
+      w.first = first; w.level = L; w.tile_entries = tile; w.min_span = min_span(L); w.target_units = target;
       w.part = part_.as<double>(); w.err = cnt + kCntErr; w.work = fw + wv % 2;
       w.fused = 1;
       w.tile_done = fz3 + 16;
@@ -622,7 +630,7 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
       w.zero_u64 = fw + (wv + 1) % 2;
       PdFinalArgs& f = w.fin;
       f.part = part_.as<double>(); f.first = first; f.level = L; f.max_level = lstop; f.quantity = o.quantity;
-      f.directional = rq.directional; f.tile_entries = tile; f.min_span = min_span; f.target_units = target;
+      f.directional = rq.directional; f.tile_entries = tile; f.min_span = min_span(L); f.target_units = target;
       f.dt_prev = L >= 1 ? dt_inclusive(tstart_, tstop_, L - 1) : 0; f.dt_level = dt_inclusive(tstart_, tstop_, L);
       f.precision = o.precision; f.scale = scale; f.weight = weight; f.two_over_gamma = 2. / P.gamma;
       f.bdmax_levels = reinterpret_cast<const double*>(mrec_bd_.p);
@@ -642,7 +650,7 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
       w.lev = mixed ? reinterpret_cast<const double*>(mrec_.p) : lev_.as<double>();
       w.cap = lev_cap_; w.obs = d_obs; w.omega = omega_.as<double>();
       w.n_e = (int64_t)rq.omega.size(); w.n_items = N; w.act = act_in; w.n_act = nact_in;
-      w.first = first; w.level = L; w.tile_entries = tile; w.min_span = min_span; w.target_units = target;
+      w.first = first; w.level = L; w.tile_entries = tile; w.min_span = min_span(L); w.target_units = target;
       w.part = part_.as<double>(); w.err = cnt + kCntErr; w.work = fw + wv % 2;
       set_phase_reach(w);
       w.fused = 1;
@@ -651,7 +659,7 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
       w.zero_u64 = fw + (wv + 1) % 2;
       FdFinalArgs& f = w.fin;
       f.part = part_.as<double>(); f.first = first; f.level = L; f.max_level = lstop; f.quantity = o.quantity;
-      f.project = project; f.tile_entries = tile; f.min_span = min_span; f.target_units = target;
+      f.project = project; f.tile_entries = tile; f.min_span = min_span(L); f.target_units = target;
       f.dt_prev = L >= 1 ? dt_inclusive(tstart_, tstop_, L - 1) : 0; f.dt_level = dt_inclusive(tstart_, tstop_, L);
       f.precision = o.precision; f.c0 = c0; f.c2 = c2; f.weight = weight;
       for (int i = 0; i < 6; ++i) f.pol[i] = pol[i];
@@ -661,7 +669,9 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
       f.dmax_spans_joined = 1;  // the flux waves carry the step into each part across groups and spans
       auto ev = timed_begin(st);
       const int g = grid_for(L);
-      if (mixed) check(launch_fd_wave_mixed(w, frame_, g, variant, st), "flux wave (mixed)");
+      w.e_tiles = (w.n_e + tile - 1) / tile;
+      if (lines) check(launch_fd_lines(w, mixed ? &frame_ : nullptr, g, st), "spectrum wave");
+      else if (mixed) check(launch_fd_wave_mixed(w, frame_, g, variant, st), "flux wave (mixed)");
       else check(launch_fd_wave_fp64(w, g, variant, st), "flux wave");
       timed_end(ev, st);
       last_launches += 1;
@@ -673,7 +683,7 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
       w.lev = mixed ? reinterpret_cast<const double*>(mrec_.p) : lev_.as<double>();
       w.cap = lev_cap_; w.obs = d_obs; w.omega = omega_.as<double>();
       w.n_e = (int64_t)rq.omega.size(); w.n_items = N; w.act = act_in; w.n_act = nact_in;
-      w.first = first; w.level = L; w.tile_entries = tile; w.min_span = min_span; w.target_units = target;
+      w.first = first; w.level = L; w.tile_entries = tile; w.min_span = min_span(L); w.target_units = target;
       w.part = part_.as<double>(); w.err = cnt + kCntErr; w.work = c64 + 2;
       auto ev = timed_begin(st);
       const int g = grid_for(L);
@@ -682,7 +692,7 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
       timed_end(ev, st);
       FdFinalArgs f{};
       f.part = part_.as<double>(); f.first = first; f.level = L; f.max_level = lstop; f.quantity = o.quantity;
-      f.project = project; f.tile_entries = tile; f.min_span = min_span; f.target_units = target;
+      f.project = project; f.tile_entries = tile; f.min_span = min_span(L); f.target_units = target;
       f.dt_prev = L >= 1 ? dt_inclusive(tstart_, tstop_, L - 1) : 0; f.dt_level = dt_inclusive(tstart_, tstop_, L);
       f.precision = o.precision; f.c0 = c0; f.c2 = c2; f.weight = weight;
       for (int i = 0; i < 6; ++i) f.pol[i] = pol[i];
@@ -695,7 +705,7 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
       w.lev = mixed ? reinterpret_cast<const double*>(mrec_.p) : lev_.as<double>();
       w.cap = lev_cap_; w.obs = d_obs; w.normals = d_nrm; w.has_normal = d_nrm != nullptr;
       w.directional = rq.directional; w.n_items = N; w.act = act_in; w.n_act = nact_in;
-      w.first = first; w.level = L; w.tile_entries = tile; w.min_span = min_span; w.target_units = target;
+      w.first = first; w.level = L; w.tile_entries = tile; w.min_span = min_span(L); w.target_units = target;
       w.part = part_.as<double>(); w.err = cnt + kCntErr; w.work = c64 + 2;
       auto ev = timed_begin(st);
       if (mixed) check(launch_pd_wave_mixed(w, frame_, grid_for(L), st), "power density wave (mixed)");
@@ -703,7 +713,7 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
       timed_end(ev, st);
       PdFinalArgs f{};
       f.part = part_.as<double>(); f.first = first; f.level = L; f.max_level = lstop; f.quantity = o.quantity;
-      f.directional = rq.directional; f.tile_entries = tile; f.min_span = min_span; f.target_units = target;
+      f.directional = rq.directional; f.tile_entries = tile; f.min_span = min_span(L); f.target_units = target;
       f.dt_prev = L >= 1 ? dt_inclusive(tstart_, tstop_, L - 1) : 0; f.dt_level = dt_inclusive(tstart_, tstop_, L);
       f.precision = o.precision; f.scale = scale; f.weight = weight; f.two_over_gamma = 2. / P.gamma;
       f.bdmax_levels = reinterpret_cast<const double*>(mixed ? mrec_bd_.p : bd_bits_.p);

@@ -182,7 +182,7 @@ class Engine {
   std::vector<int> pending_;
   // kernel variants: kind 0 = FP64 flux, 1 = FP64 power density, 2 = mixed flux, 3 = batched mixed,
   // 4 = mixed power density
-  int wave_grid_[5][16] = {};
+  int wave_grid_[7][16] = {};  // kinds: 0 fp64, 1 power density, 2 mixed, 4 mixed power density, 5 / 6 fp64 / mixed lines
   int wave_grid(int kind, int variant);
   std::map<std::tuple<int, int, int, int>, int> tuned_;   // (kind, log2 entries, first level, last level) -> variant
   // (kind, entries, energies, last level, precision) -> highest level the last such request needed

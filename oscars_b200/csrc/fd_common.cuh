@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "device_common.cuh"
 #include "kernels.h"
 
 namespace osc {
@@ -60,6 +61,63 @@ __device__ __forceinline__ double level_time(double tstart, double tstop, int64_
   const double ts = __dadd_rn(tstart, __ddiv_rn(__dsub_rn(tstop, tstart), ldexp(1.0, L + 1)));
   const double sp = __ddiv_rn(__dsub_rn(tstop, tstart), L > ext_from ? __dsub_rn(ldexp(1.0, L), 1.0) : ldexp(1.0, L));
   return __dadd_rn(ts, __dmul_rn(sp, (double)i));
+}
+
+// ---------------------------------------------------------------------------------------------
+// FP64 sample term.
+// ---------------------------------------------------------------------------------------------
+// Retarded time t + D/c and phase -w (t + D/c) of one sample for an observer, with the operations of
+// fd_term below.
+__device__ __forceinline__ double fd_tau(double T, double X, double Y, double Z, double Ox, double Oy, double Oz) {
+  const double Rx = __dsub_rn(Ox, X), Ry = __dsub_rn(Oy, Y), Rz = __dsub_rn(Oz, Z);
+  const double s = __dadd_rn(__dadd_rn(__dmul_rn(Rx, Rx), __dmul_rn(Ry, Ry)), __dmul_rn(Rz, Rz));
+  return __dadd_rn(T, over_c(sqrt_by(s, rsqrt_near(s))));
+}
+__device__ __forceinline__ double fd_phase(double T, double X, double Y, double Z, double Ox, double Oy, double Oz,
+                                           double mw) {
+  return __dmul_rn(mw, fd_tau(T, X, Y, Z, Ox, Oy, Oz));
+}
+
+// Retarded time t + D/c and amplitude of one sample for an observer.  D, n and 1 - n.b round as the
+// reference's operations do (their last bits move the phase and the ill-conditioned 1 - n.b); the rest
+// is well conditioned and is formed with FMA from n x (u x a) = u (n.a) - a (n.u), u = n - b:
+//   e = u k1 - a k2,  k1 = ((1 - b^2) / D + n.a) / (D om^2),  k2 = (n.u) / (D om^2),  om = 1 - n.b.
+// 59 FP64 operations (with the library's square root and six divisions: ~115).
+struct FdTerm {
+  double tau, ex, ey, ez;
+};
+__device__ __forceinline__ FdTerm fd_term(double T, double X, double Y, double Z, double bx, double by, double bz,
+                                          double ax, double ay, double az, double ob2, double Ox, double Oy, double Oz) {
+  const double Rx = __dsub_rn(Ox, X), Ry = __dsub_rn(Oy, Y), Rz = __dsub_rn(Oz, Z);
+  const double s = __dadd_rn(__dadd_rn(__dmul_rn(Rx, Rx), __dmul_rn(Ry, Ry)), __dmul_rn(Rz, Rz));
+  const double y = rsqrt_near(s), D = sqrt_by(s, y);
+  FdTerm f;
+  f.tau = __dadd_rn(T, over_c(D));
+  const double nx = quot_by(Rx, D, y), ny = quot_by(Ry, D, y), nz = quot_by(Rz, D, y);
+  const double om =
+      __dsub_rn(1.0, __dadd_rn(__dadd_rn(__dmul_rn(nx, bx), __dmul_rn(ny, by)), __dmul_rn(nz, bz)));
+  const double ux = __dsub_rn(nx, bx), uy = __dsub_rn(ny, by), uz = __dsub_rn(nz, bz);
+  const double na = fma(nx, ax, fma(ny, ay, nz * az));
+  const double nu = fma(nx, ux, fma(ny, uy, nz * uz));
+  const double io = rcp_near(om);
+  const double f2 = y * io * io;
+  const double k1 = f2 * fma(ob2, y, na), k2 = -(f2 * nu);
+  f.ex = fma(ux, k1, ax * k2);
+  f.ey = fma(uy, k1, ay * k2);
+  f.ez = fma(uz, k1, az * k2);
+  return f;
+}
+
+// 1 - b^2 of a sample, in the reference's operations.
+__device__ __forceinline__ double one_minus_b2(double bx, double by, double bz) {
+  return __dsub_rn(1.0, __dadd_rn(__dadd_rn(__dmul_rn(bx, bx), __dmul_rn(by, by)), __dmul_rn(bz, bz)));
+}
+
+// Bound of |w (t + D/c)| over a trajectory: it starts at A.x_start, lasts A.t_len and its times lie
+// within A.t_abs of zero, and the particle is slower than light.
+__device__ __forceinline__ double phase_reach(const FdWaveArgs& A, double Ox, double Oy, double Oz, double mw) {
+  const double dx = Ox - A.x_start[0], dy = Oy - A.x_start[1], dz = Oz - A.x_start[2];
+  return fabs(mw) * (A.t_abs + A.t_len + sqrt(dx * dx + dy * dy + dz * dz) * kInvC1);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -202,15 +260,17 @@ __device__ __forceinline__ PairObs make_pair_obs(double fx, double fy, double fz
 
 // FP32 phase P32 of one sample with the per-lane operations of pair_sample (same value): the
 // quantity whose steps the stop rule bounds.
-__device__ __forceinline__ float pair_phase(float x, float y, float z, float tau, const PairObs& o) {
+__device__ __forceinline__ float pair_corr(float x, float y, float z, const PairObs& o) {  // D - R_z
   const float rx = fmaf(x, -1.f, o.ox.x), ry = fmaf(y, -1.f, o.oy.x), rz = fmaf(z, -1.f, o.oz.x);
   const float rho2 = fmaf(rx, rx, __fmul_rn(ry, ry));
   const float d2 = fmaf(rz, rz, rho2);
   const float iD = rsqrt_ftz(d2);
   const float ri = __fmul_rn(rho2, iD);
   const float q = __fmul_rn(ri, iD);
-  const float corr = __fmul_rn(ri, fmaf(0.125f, q, 0.5f));
-  return fmaf(o.wc.x, corr, __fmul_rn(o.w.x, tau));
+  return __fmul_rn(ri, fmaf(0.125f, q, 0.5f));
+}
+__device__ __forceinline__ float pair_phase(float x, float y, float z, float tau, const PairObs& o) {
+  return fmaf(o.wc.x, pair_corr(x, y, z, o), __fmul_rn(o.w.x, tau));
 }
 
 // P32 of sample b (0 or 1) of the pair record at `q` (shared or global memory).
@@ -231,16 +291,20 @@ __device__ __forceinline__ double nonneg_float_to_double(float x) {
 // |E|^2.  corr_f and half_iD = 1 / (2 D) are the sample's FP32 values.  v = 1.5 * 2^22 + turns lies
 // in [2^22, 2^23) (|turns| < 2^21), so bits 0..29 of its low word are the fraction of a turn in
 // units of 2^-30; bits 7..29, rounded, become the significand of a float in [1, 2).
-__device__ __forceinline__ float fp64_turns(double x, double y, double z, double tau, float corr_f, float half_iD,
-                                            const PairObs& o) {
+__device__ __forceinline__ double fp64_corr(double x, double y, double z, float corr_f, float half_iD, const PairObs& o) {
   const double Rx = o.dox - x, Ry = o.doy - y, Rz = o.doz - z;
   const double r2 = fma(Rx, Rx, Ry * Ry);
   const double c = nonneg_float_to_double(corr_f);
   const double f = fma(c, fma(2.0, Rz, c), -r2);
-  const double c1 = fma(-f, nonneg_float_to_double(half_iD), c);
-  const double v = fma(o.dwct, c1, fma(o.dwt, tau, kTurnBase));
+  return fma(-f, nonneg_float_to_double(half_iD), c);
+}
+__device__ __forceinline__ float turn_fraction(double v) {
   const unsigned lo = (unsigned)__double2loint(v) + 0x40u;  // round to 23 fraction bits (a carry wraps mod 1)
   return __uint_as_float(((lo >> 7) & 0x007FFFFFu) | 0x3F800000u) - 1.5f;
+}
+__device__ __forceinline__ float fp64_turns(double x, double y, double z, double tau, float corr_f, float half_iD,
+                                            const PairObs& o) {
+  return turn_fraction(fma(o.dwct, fp64_corr(x, y, z, corr_f, half_iD, o), fma(o.dwt, tau, kTurnBase)));
 }
 
 // Both samples of one pair record `q` for one entry: adds e (cos P, sin P) per lane to acc (x re,

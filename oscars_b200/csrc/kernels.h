@@ -101,6 +101,7 @@ struct FdWaveArgs {
   const double* obs;        // 3 * n_obs
   const double* omega;      // n_e
   int64_t n_e;
+  int64_t e_tiles;          // the line kernels without a list: tiles per observer
   int64_t n_items;          // n_obs * n_e (entry = obs_index * n_e + energy_index)
   const int* act;           // active entry ids (NULL: entries 0..n_items-1)
   const unsigned* n_act;    // device count of `act`
@@ -226,6 +227,12 @@ int mixed_blocks_per_sm(int variant);
 int fp64_blocks_per_sm(bool power_density, int variant);
 int fp64_entries_per_cta(int variant);
 const char* fp64_variant_name(int variant);
+
+// Many energies of one observer (kernels_lines.cu): a.lev = the FP64 level cache (F = NULL) or the
+// mixed records in frame *F; tile_entries = lines_entries_per_cta().
+int lines_entries_per_cta();
+int lines_blocks_per_sm(bool mixed);
+cudaError_t launch_fd_lines(const FdWaveArgs& a, const MixedFrame* F, int grid, cudaStream_t st);
 
 // FP64 level samples [s_begin, s_end) (10 SoA arrays of stride cap) and their per-level beta-difference
 // maxima; levels above ext_from are the reference's extended levels.

@@ -96,56 +96,6 @@ __device__ __forceinline__ void stage_issue(Stage<NARR, CH>& st, int b, const do
 constexpr int kFdThreads = 128;
 constexpr int kFdChunk = 128;
 
-// Phase -w (t + D/c) of one staged sample for an observer, with the operations of the sum below.
-__device__ __forceinline__ double fd_phase(double T, double X, double Y, double Z, double Ox, double Oy, double Oz,
-                                           double mw) {
-  const double Rx = __dsub_rn(Ox, X), Ry = __dsub_rn(Oy, Y), Rz = __dsub_rn(Oz, Z);
-  const double s = __dadd_rn(__dadd_rn(__dmul_rn(Rx, Rx), __dmul_rn(Ry, Ry)), __dmul_rn(Rz, Rz));
-  return __dmul_rn(mw, __dadd_rn(T, over_c(sqrt_by(s, rsqrt_near(s)))));
-}
-
-// Retarded time t + D/c and amplitude of one sample for an observer.  D, n and 1 - n.b round as the
-// reference's operations do (their last bits move the phase and the ill-conditioned 1 - n.b); the rest
-// is well conditioned and is formed with FMA from n x (u x a) = u (n.a) - a (n.u), u = n - b:
-//   e = u k1 - a k2,  k1 = ((1 - b^2) / D + n.a) / (D om^2),  k2 = (n.u) / (D om^2),  om = 1 - n.b.
-// 59 FP64 operations (with the library's square root and six divisions: ~115).
-struct FdTerm {
-  double tau, ex, ey, ez;
-};
-__device__ __forceinline__ FdTerm fd_term(double T, double X, double Y, double Z, double bx, double by, double bz,
-                                          double ax, double ay, double az, double ob2, double Ox, double Oy, double Oz) {
-  const double Rx = __dsub_rn(Ox, X), Ry = __dsub_rn(Oy, Y), Rz = __dsub_rn(Oz, Z);
-  const double s = __dadd_rn(__dadd_rn(__dmul_rn(Rx, Rx), __dmul_rn(Ry, Ry)), __dmul_rn(Rz, Rz));
-  const double y = rsqrt_near(s), D = sqrt_by(s, y);
-  FdTerm f;
-  f.tau = __dadd_rn(T, over_c(D));
-  const double nx = quot_by(Rx, D, y), ny = quot_by(Ry, D, y), nz = quot_by(Rz, D, y);
-  const double om =
-      __dsub_rn(1.0, __dadd_rn(__dadd_rn(__dmul_rn(nx, bx), __dmul_rn(ny, by)), __dmul_rn(nz, bz)));
-  const double ux = __dsub_rn(nx, bx), uy = __dsub_rn(ny, by), uz = __dsub_rn(nz, bz);
-  const double na = fma(nx, ax, fma(ny, ay, nz * az));
-  const double nu = fma(nx, ux, fma(ny, uy, nz * uz));
-  const double io = rcp_near(om);
-  const double f2 = y * io * io;
-  const double k1 = f2 * fma(ob2, y, na), k2 = -(f2 * nu);
-  f.ex = fma(ux, k1, ax * k2);
-  f.ey = fma(uy, k1, ay * k2);
-  f.ez = fma(uz, k1, az * k2);
-  return f;
-}
-
-// 1 - b^2 of a sample, in the reference's operations.
-__device__ __forceinline__ double one_minus_b2(double bx, double by, double bz) {
-  return __dsub_rn(1.0, __dadd_rn(__dadd_rn(__dmul_rn(bx, bx), __dmul_rn(by, by)), __dmul_rn(bz, bz)));
-}
-
-// Bound of |w (t + D/c)| over a trajectory: it starts at A.x_start, lasts A.t_len and its times lie
-// within A.t_abs of zero, and the particle is slower than light.
-__device__ __forceinline__ double phase_reach(const FdWaveArgs& A, double Ox, double Oy, double Oz, double mw) {
-  const double dx = Ox - A.x_start[0], dy = Oy - A.x_start[1], dz = Oz - A.x_start[2];
-  return fabs(mw) * (A.t_abs + A.t_len + sqrt(dx * dx + dy * dy + dz * dz) * kInvC1);
-}
-
 // Sample-split FP64 sum: the CTA's 128 threads form SUB groups of TE = 128 / SUB threads, one entry
 // per thread; group g takes the g-th of SUB equal parts of every staged chunk of the 10 level arrays.
 // Each part starts from the phase of the sample before it (the chunk's previous sample, the previous
@@ -179,17 +129,19 @@ __global__ void __launch_bounds__(kFdThreads, MINB) k_fd_wave_fp64(FdWaveArgs A)
   __shared__ WavePlan P;
   const int tid = threadIdx.x;
   const int grp = tid / TE, q = tid % TE;
+  launch_dependents();
+  if (tid == 0) {
+    mbar_init(&st.bar[0], 1);
+    mbar_init(&st.bar[1], 1);
+    fence_barrier_init();
+  }
+  wait_predecessor();
   if (A.fused && blockIdx.x == 0 && tid == 0) {  // counters of the following wave
     if (A.zero_u32) *A.zero_u32 = 0;
     if (A.zero_u64) *A.zero_u64 = 0;
   }
   const int64_t n_act = A.act ? (int64_t)*A.n_act : A.n_items;
-  if (tid == 0) {
-    P = wave_plan(A.first, A.level, n_act, TE, A.target_units, A.min_span);
-    mbar_init(&st.bar[0], 1);
-    mbar_init(&st.bar[1], 1);
-    fence_barrier_init();
-  }
+  if (tid == 0) P = wave_plan(A.first, A.level, n_act, TE, A.target_units, A.min_span);
   __syncthreads();
   // units (tile, segment, span), spans fastest: the first is the CTA's own, the others come from a
   // shared counter until the wave's units run out
@@ -583,10 +535,10 @@ const char* fp64_variant_name(int variant) {
 cudaError_t launch_fd_wave_fp64(const FdWaveArgs& a, int grid, int variant, cudaStream_t st) {
   switch (variant) {
 #define OSC_LAUNCH(i, sub, minb) \
-    case i: dev::k_fd_wave_fp64<sub, minb><<<grid, dev::kFdThreads, 0, st>>>(a); break;
+    case i: return launch_overlapped(dev::k_fd_wave_fp64<sub, minb>, grid, dev::kFdThreads, st, a);
     OSC_FP64_VARIANTS(OSC_LAUNCH)
   }
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_fd_finalize(const FdFinalArgs& a, int64_t n_act_bound, cudaStream_t st) {

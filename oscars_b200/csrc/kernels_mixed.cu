@@ -102,6 +102,8 @@ __global__ void __launch_bounds__(kMxThreads, MINB) k_fd_wave_mixed_pair(FdWaveA
   __shared__ int64_t next_unit;
   const int tid = threadIdx.x;
   const int grp = tid / TE, q = tid % TE;
+  launch_dependents();
+  wait_predecessor();
   if (A.fused && blockIdx.x == 0 && tid == 0) {  // counters of the following wave
     if (A.zero_u32) *A.zero_u32 = 0;
     if (A.zero_u64) *A.zero_u64 = 0;
@@ -317,6 +319,8 @@ __global__ void __launch_bounds__(kMxThreads, MINB) k_pd_wave_mixed(PdWaveArgs A
   __shared__ int s_last;
   const int tid = threadIdx.x;
   const int grp = tid / TE, q = tid % TE;
+  launch_dependents();
+  wait_predecessor();
   if (A.fused && blockIdx.x == 0 && tid == 0) {  // counters of the following wave
     if (A.zero_u32) *A.zero_u32 = 0;
     if (A.zero_u64) *A.zero_u64 = 0;
@@ -469,10 +473,10 @@ cudaError_t launch_fd_wave_mixed(const FdWaveArgs& a, const MixedFrame& F, int g
   const int T = dev::kMxThreads;
   switch (variant) {
 #define OSC_LAUNCH(i, sub, minb, cp, ssm) \
-    case i: dev::k_fd_wave_mixed_pair<sub, minb, cp, ssm><<<grid, T, 0, st>>>(a, F); break;
+    case i: return launch_overlapped(dev::k_fd_wave_mixed_pair<sub, minb, cp, ssm>, grid, T, st, a, F);
     OSC_MIXED_VARIANTS(OSC_LAUNCH)
   }
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 // The mixed power-density kernel: 4 groups of 32 entries, at least 4 CTAs per SM, 128 pair records
@@ -485,8 +489,7 @@ int pd_mixed_blocks_per_sm() {
   return n > 0 ? n : 1;
 }
 cudaError_t launch_pd_wave_mixed(const PdWaveArgs& a, const MixedFrame& F, int grid, cudaStream_t st) {
-  dev::k_pd_wave_mixed<kPdMxSub, 4, 128><<<grid, dev::kMxThreads, 0, st>>>(a, F);
-  return cudaGetLastError();
+  return launch_overlapped(dev::k_pd_wave_mixed<kPdMxSub, 4, 128>, grid, dev::kMxThreads, st, a, F);
 }
 
 }  // namespace osc

@@ -32,3 +32,28 @@ def test_fp64_flux_beyond_the_fast_phases():
     kw = dict(energy_eV=1e8, npoints=[3, 3], width=[0.004, 0.006], translation=[0, 0, 20], max_level=5)
     got, want = _both("calculate_flux_rectangle", kw)
     assert np.max(np.abs(got - want)) <= 1e-9 * np.max(np.abs(want))
+
+
+# The line kernels (one observer): tiles of 64 energies, spans of 64 samples, and the step test of the
+# stop rule at its precise bound (level 9 and up); the same roundings as above.
+@pytest.mark.parametrize("n, level", [(1, 0), (2, 3), (63, 8), (64, 9), (65, 10), (129, 12), (40, 13)])
+def test_fp64_spectrum_tiles_and_levels(n, level):
+    kw = dict(obs=[0.001, 0, 20], energy_range_eV=[200, 1900], npoints=n, max_level=level)
+    got, want = _both("calculate_spectrum", kw)
+    assert np.max(np.abs(got - want)) <= 1e-11 * np.max(np.abs(want))
+
+
+# Mixed: every phase, amplitude, sine, cosine and FP32 partial sum is the general kernel's; the order of
+# at most 2^9 FP64 additions differs (2^9 x 2^-53 of the sum of magnitudes, < 2000 peaks): 1e-10.
+@pytest.mark.parametrize("n, level", [(1, 9), (64, 10), (65, 11), (200, 14)])
+def test_mixed_spectrum_lines_match_general_kernel(n, level):
+    out = []
+    for variant in (0, -1):
+        s = sr(gpu=1)
+        s._ctx.call("osc_set_variant", 2, variant)
+        run_case(s, UND_SHORT_SETUP)
+        e, f = s.calculate_spectrum(obs=[0.001, 0, 20], energy_range_eV=[200, 1900], npoints=n, max_level=level,
+                                    compute="mixed", return_numpy=True)
+        out.append((f, s.last_levels.copy()))
+    assert np.array_equal(out[0][1], out[1][1])
+    assert np.max(np.abs(out[0][0] - out[1][0])) <= 1e-10 * np.max(np.abs(out[0][0]))
