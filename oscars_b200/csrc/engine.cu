@@ -389,7 +389,7 @@ void polarization_vector(const osc_rad_opts& o, double P[6], bool& project) {
 // Levels resident before a request starts: every wave up to this level is enqueued without any
 // host round trip; entries still unconverged after it make the host extend the cache.
 constexpr int kPrefillLevel = 14;
-constexpr int kMinSpan = 32;
+constexpr int kMinSpan = 64;
 // Sample-split mixed flux / spectrum waves: spans of at least one staged chunk, so that a
 // unit's fixed costs (its first copy, the partial store, the tile counter) stay small beside its
 // arithmetic.
@@ -511,12 +511,12 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
   const int variant = lines ? 0 : tuning_ ? current_variant_[kind]
                               : pick_variant(kind, const_cast<RadRequest&>(rq), n_items, Lfirst, lstop, d_out, d_lvl, st);
   const int resident = wave_grid(lines ? (mixed ? 6 : 5) : kind, variant);  // CTAs resident at once on the device
-  const int tile = rq.power_density ? (mixed ? pd_mixed_entries_per_cta() : 128)
+  const int tile = rq.power_density ? (mixed ? pd_mixed_entries_per_cta() : pd_fp64_entries_per_cta())
                    : lines ? lines_entries_per_cta()
                                     : (mixed ? mixed_entries_per_cta(variant) : fp64_entries_per_cta(variant));
   // At most 64 spans: beyond, the finalizer's pass over a tile's spans costs more than shorter units save.
   auto min_span = [&](int L) {
-    return rq.power_density ? kMinSpan : std::max(mixed ? kMinSpanSplit : kMinSpanFp64, L > 6 ? 1 << (L - 6) : 1);
+    return std::max(rq.power_density ? kMinSpan : mixed ? kMinSpanSplit : kMinSpanFp64, L > 6 ? 1 << (L - 6) : 1);
   };
   const int64_t target = 4 * (int64_t)resident;   // >= 4 waves of equal units per launch
   const int64_t N = n_items;
@@ -546,24 +546,19 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
   // [0] not converged, [1] samples, [2] unit counter of the running wave
   unsigned long long* c64 = reinterpret_cast<unsigned long long*>(cnt + 4);
   unsigned* level_max = cnt + 12;  // highest level at which an entry finished
-  // Flux / spectrum waves finalize their own tiles (one launch per level).  Wave w reads its active
-  // count from fz3[w % 3], appends survivors to fz3[(w + 1) % 3] and zeroes fz3[(w + 2) % 3] for the
-  // wave after; it takes units from fw[w % 2] and zeroes fw[(w + 1) % 2].
-  const bool fused = !rq.power_density || mixed;  // the FP64 power density keeps its finalize kernel
-  unsigned* fz3 = nullptr;
-  unsigned long long* fw = nullptr;
-  if (fused) {
-    fused_.reserve(64 + sizeof(unsigned) * (size_t)(ntiles + 1));
-    fz3 = fused_.as<unsigned>();
-    fw = reinterpret_cast<unsigned long long*>(fz3 + 4);
-  }
+  // Waves finalize their own tiles (one launch per level).  Wave w reads its active count from
+  // fz3[w % 3], appends survivors to fz3[(w + 1) % 3] and zeroes fz3[(w + 2) % 3] for the wave after; it
+  // takes units from fw[w % 2] and zeroes fw[(w + 1) % 2].
+  fused_.reserve(64 + sizeof(unsigned) * (size_t)(ntiles + 1));
+  unsigned* fz3 = fused_.as<unsigned>();
+  unsigned long long* fw = reinterpret_cast<unsigned long long*>(fz3 + 4);
   // One prologue launch zeroes the counters (words 0..12), the fused-finalize counters and the
   // beta-step maxima of the levels the prefill fills, and copies the staged frequencies.
   {
     if (mixed) reserve_mixed(Lpre);
     else reserve_levels(Lpre);
     const int filled = mixed ? mrec_filled_ : lev_filled_;
-    ZeroRange z0{cnt, 13}, z1{fz3, fused ? 16 + (ntiles + 1) : 0}, z2{nullptr, 0};
+    ZeroRange z0{cnt, 13}, z1{fz3, 16 + (ntiles + 1)}, z2{nullptr, 0};
     if (Lpre > filled) {
       if (mixed) {
         const int Lb = filled < 0 ? 0 : filled + 1;
@@ -614,17 +609,15 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
     else join_prefill();         // the levels filled on the side stream
     const int wv = L - Lfirst;
     const int* act_in = first ? nullptr : act_[cur_list].as<int>();
-    const unsigned* nact_in = first ? nullptr : (fused ? fz3 + wv % 3 : cnt + cur_list);
-    unsigned* n_next = fused ? fz3 + (wv + 1) % 3 : cnt + (cur_list ^ 1);
-    if (!fused) check(cudaMemsetAsync(n_next, 0, sizeof(unsigned), st), "memset");
-    if (fused && rq.power_density) {
+    const unsigned* nact_in = first ? nullptr : fz3 + wv % 3;
+    unsigned* n_next = fz3 + (wv + 1) % 3;
+    if (rq.power_density) {
       PdWaveArgs w{};
-      w.lev = reinterpret_cast<const double*>(mrec_.p);
+      w.lev = mixed ? reinterpret_cast<const double*>(mrec_.p) : lev_.as<double>();
       w.cap = lev_cap_; w.obs = d_obs; w.normals = d_nrm; w.has_normal = d_nrm != nullptr;
       w.directional = rq.directional; w.n_items = N; w.act = act_in; w.n_act = nact_in;
       w.first = first; w.level = L; w.tile_entries = tile; w.min_span = min_span(L); w.target_units = target;
       w.part = part_.as<double>(); w.err = cnt + kCntErr; w.work = fw + wv % 2;
-      w.fused = 1;
       w.tile_done = fz3 + 16;
       w.zero_u32 = fz3 + (wv + 2) % 3;
       w.zero_u64 = fw + (wv + 1) % 2;
@@ -633,96 +626,47 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
       f.directional = rq.directional; f.tile_entries = tile; f.min_span = min_span(L); f.target_units = target;
       f.dt_prev = L >= 1 ? dt_inclusive(tstart_, tstop_, L - 1) : 0; f.dt_level = dt_inclusive(tstart_, tstop_, L);
       f.precision = o.precision; f.scale = scale; f.weight = weight; f.two_over_gamma = 2. / P.gamma;
-      f.bdmax_levels = reinterpret_cast<const double*>(mrec_bd_.p);
+      f.bdmax_levels = reinterpret_cast<const double*>(mixed ? mrec_bd_.p : bd_bits_.p);
       f.n_items = N; f.act = act_in; f.n_act = nact_in; f.state = state_.as<double>();
       f.act_next = act_[cur_list ^ 1].as<int>(); f.n_next = n_next;
       f.out = d_out; f.level_out = d_lvl; f.not_converged = c64; f.samples = c64 + 1; f.level_max = level_max;
-      f.work_reset = nullptr;
-      auto ev = timed_begin(st);
-      check(launch_pd_wave_mixed(w, frame_, grid_for(L), st), "power density wave (mixed)");
-      timed_end(ev, st);
-      last_launches += 1;
-      cur_list ^= 1;
-      return;
-    }
-    if (fused) {
-      FdWaveArgs w{};
-      w.lev = mixed ? reinterpret_cast<const double*>(mrec_.p) : lev_.as<double>();
-      w.cap = lev_cap_; w.obs = d_obs; w.omega = omega_.as<double>();
-      w.n_e = (int64_t)rq.omega.size(); w.n_items = N; w.act = act_in; w.n_act = nact_in;
-      w.first = first; w.level = L; w.tile_entries = tile; w.min_span = min_span(L); w.target_units = target;
-      w.part = part_.as<double>(); w.err = cnt + kCntErr; w.work = fw + wv % 2;
-      set_phase_reach(w);
-      w.fused = 1;
-      w.tile_done = fz3 + 16;
-      w.zero_u32 = fz3 + (wv + 2) % 3;
-      w.zero_u64 = fw + (wv + 1) % 2;
-      FdFinalArgs& f = w.fin;
-      f.part = part_.as<double>(); f.first = first; f.level = L; f.max_level = lstop; f.quantity = o.quantity;
-      f.project = project; f.tile_entries = tile; f.min_span = min_span(L); f.target_units = target;
-      f.dt_prev = L >= 1 ? dt_inclusive(tstart_, tstop_, L - 1) : 0; f.dt_level = dt_inclusive(tstart_, tstop_, L);
-      f.precision = o.precision; f.c0 = c0; f.c2 = c2; f.weight = weight;
-      for (int i = 0; i < 6; ++i) f.pol[i] = pol[i];
-      f.n_items = N; f.act = act_in; f.n_act = nact_in; f.state = state_.as<double>();
-      f.act_next = act_[cur_list ^ 1].as<int>(); f.n_next = n_next;
-      f.out = d_out; f.level_out = d_lvl; f.not_converged = c64; f.samples = c64 + 1; f.level_max = level_max; f.work_reset = nullptr;
-      f.dmax_spans_joined = 1;  // the flux waves carry the step into each part across groups and spans
-      auto ev = timed_begin(st);
-      const int g = grid_for(L);
-      w.e_tiles = (w.n_e + tile - 1) / tile;
-      if (lines) check(launch_fd_lines(w, mixed ? &frame_ : nullptr, g, st), "spectrum wave");
-      else if (mixed) check(launch_fd_wave_mixed(w, frame_, g, variant, st), "flux wave (mixed)");
-      else check(launch_fd_wave_fp64(w, g, variant, st), "flux wave");
-      timed_end(ev, st);
-      last_launches += 1;
-      cur_list ^= 1;
-      return;
-    }
-    if (!rq.power_density) {
-      FdWaveArgs w{};
-      w.lev = mixed ? reinterpret_cast<const double*>(mrec_.p) : lev_.as<double>();
-      w.cap = lev_cap_; w.obs = d_obs; w.omega = omega_.as<double>();
-      w.n_e = (int64_t)rq.omega.size(); w.n_items = N; w.act = act_in; w.n_act = nact_in;
-      w.first = first; w.level = L; w.tile_entries = tile; w.min_span = min_span(L); w.target_units = target;
-      w.part = part_.as<double>(); w.err = cnt + kCntErr; w.work = c64 + 2;
-      auto ev = timed_begin(st);
-      const int g = grid_for(L);
-      if (mixed) check(launch_fd_wave_mixed(w, frame_, g, variant, st), "flux wave (mixed)");
-      else check(launch_fd_wave_fp64(w, g, variant, st), "flux wave");
-      timed_end(ev, st);
-      FdFinalArgs f{};
-      f.part = part_.as<double>(); f.first = first; f.level = L; f.max_level = lstop; f.quantity = o.quantity;
-      f.project = project; f.tile_entries = tile; f.min_span = min_span(L); f.target_units = target;
-      f.dt_prev = L >= 1 ? dt_inclusive(tstart_, tstop_, L - 1) : 0; f.dt_level = dt_inclusive(tstart_, tstop_, L);
-      f.precision = o.precision; f.c0 = c0; f.c2 = c2; f.weight = weight;
-      for (int i = 0; i < 6; ++i) f.pol[i] = pol[i];
-      f.n_items = N; f.act = act_in; f.n_act = nact_in; f.state = state_.as<double>();
-      f.act_next = act_[cur_list ^ 1].as<int>(); f.n_next = n_next;
-      f.out = d_out; f.level_out = d_lvl; f.not_converged = c64; f.samples = c64 + 1; f.level_max = level_max; f.work_reset = c64 + 2;
-      check(launch_fd_finalize(f, N, st), "flux finalize");
-    } else {
-      PdWaveArgs w{};
-      w.lev = mixed ? reinterpret_cast<const double*>(mrec_.p) : lev_.as<double>();
-      w.cap = lev_cap_; w.obs = d_obs; w.normals = d_nrm; w.has_normal = d_nrm != nullptr;
-      w.directional = rq.directional; w.n_items = N; w.act = act_in; w.n_act = nact_in;
-      w.first = first; w.level = L; w.tile_entries = tile; w.min_span = min_span(L); w.target_units = target;
-      w.part = part_.as<double>(); w.err = cnt + kCntErr; w.work = c64 + 2;
       auto ev = timed_begin(st);
       if (mixed) check(launch_pd_wave_mixed(w, frame_, grid_for(L), st), "power density wave (mixed)");
       else check(launch_pd_wave_fp64(w, grid_for(L), st), "power density wave");
       timed_end(ev, st);
-      PdFinalArgs f{};
-      f.part = part_.as<double>(); f.first = first; f.level = L; f.max_level = lstop; f.quantity = o.quantity;
-      f.directional = rq.directional; f.tile_entries = tile; f.min_span = min_span(L); f.target_units = target;
-      f.dt_prev = L >= 1 ? dt_inclusive(tstart_, tstop_, L - 1) : 0; f.dt_level = dt_inclusive(tstart_, tstop_, L);
-      f.precision = o.precision; f.scale = scale; f.weight = weight; f.two_over_gamma = 2. / P.gamma;
-      f.bdmax_levels = reinterpret_cast<const double*>(mixed ? mrec_bd_.p : bd_bits_.p);
-      f.n_items = N; f.act = act_in; f.n_act = nact_in; f.state = state_.as<double>();
-      f.act_next = act_[cur_list ^ 1].as<int>(); f.n_next = n_next;
-      f.out = d_out; f.level_out = d_lvl; f.not_converged = c64; f.samples = c64 + 1; f.level_max = level_max; f.work_reset = c64 + 2;
-      check(launch_pd_finalize(f, N, st), "power density finalize");
+      last_launches += 1;
+      cur_list ^= 1;
+      return;
     }
-    last_launches += 2;
+    FdWaveArgs w{};
+    w.lev = mixed ? reinterpret_cast<const double*>(mrec_.p) : lev_.as<double>();
+    w.cap = lev_cap_; w.obs = d_obs; w.omega = omega_.as<double>();
+    w.n_e = (int64_t)rq.omega.size(); w.n_items = N; w.act = act_in; w.n_act = nact_in;
+    w.first = first; w.level = L; w.tile_entries = tile; w.min_span = min_span(L); w.target_units = target;
+    w.part = part_.as<double>(); w.err = cnt + kCntErr; w.work = fw + wv % 2;
+    set_phase_reach(w);
+    w.fused = 1;
+    w.tile_done = fz3 + 16;
+    w.zero_u32 = fz3 + (wv + 2) % 3;
+    w.zero_u64 = fw + (wv + 1) % 2;
+    FdFinalArgs& f = w.fin;
+    f.part = part_.as<double>(); f.first = first; f.level = L; f.max_level = lstop; f.quantity = o.quantity;
+    f.project = project; f.tile_entries = tile; f.min_span = min_span(L); f.target_units = target;
+    f.dt_prev = L >= 1 ? dt_inclusive(tstart_, tstop_, L - 1) : 0; f.dt_level = dt_inclusive(tstart_, tstop_, L);
+    f.precision = o.precision; f.c0 = c0; f.c2 = c2; f.weight = weight;
+    for (int i = 0; i < 6; ++i) f.pol[i] = pol[i];
+    f.n_items = N; f.act = act_in; f.n_act = nact_in; f.state = state_.as<double>();
+    f.act_next = act_[cur_list ^ 1].as<int>(); f.n_next = n_next;
+    f.out = d_out; f.level_out = d_lvl; f.not_converged = c64; f.samples = c64 + 1; f.level_max = level_max; f.work_reset = nullptr;
+    f.dmax_spans_joined = 1;  // the flux waves carry the step into each part across groups and spans
+    auto ev = timed_begin(st);
+    const int g = grid_for(L);
+    w.e_tiles = (w.n_e + tile - 1) / tile;
+    if (lines) check(launch_fd_lines(w, mixed ? &frame_ : nullptr, g, st), "spectrum wave");
+    else if (mixed) check(launch_fd_wave_mixed(w, frame_, g, variant, st), "flux wave (mixed)");
+    else check(launch_fd_wave_fp64(w, g, variant, st), "flux wave");
+    timed_end(ev, st);
+    last_launches += 1;
     cur_list ^= 1;
   };
   for (int L = Lfirst; L <= Lpre; ++L) launch_wave(L);
@@ -730,7 +674,7 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
   for (int L = Lpre + 1; L <= lstop; ++L) {  // beyond the prefilled levels the host decides
     // a one-thread kernel writes the active count and the highest finished level into mapped host
     // memory behind a sequence word that the host polls (no copy engine, no stream wake-up)
-    const unsigned* active = fused ? fz3 + (L - Lfirst) % 3 : cnt + cur_list;
+    const unsigned* active = fz3 + (L - Lfirst) % 3;
     unsigned nn = 0, lmax = 0;
     // the report also stores the request's statistics into a ring slot, and the downloads of host
     // outputs go in behind it, before the host knows whether this was the last wave; if it was not,

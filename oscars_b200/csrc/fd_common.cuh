@@ -472,8 +472,8 @@ __device__ __forceinline__ void pd_entry_decide(const PdFinalArgs& A, int64_t it
   }
 }
 
-// Fused finalize of one tile of the mixed power-density wave by warp 0 (TE entries, 32 at a time):
-// each entry's span partials summed in span order from the tile-major layout
+// Fused finalize of one tile of a power-density wave by warp 0 (TE entries, 32 at a time): each
+// entry's span partials summed in span order from the tile-major layout
 // [tile][segment][span][entry in tile], the stop rule of pd_entry_decide, survivors appended.
 __device__ __forceinline__ void pd_tile_finalize(const PdFinalArgs& A, const WavePlan& P, int64_t tile, int64_t n_act,
                                                  int TE) {
@@ -485,8 +485,18 @@ __device__ __forceinline__ void pd_tile_finalize(const PdFinalArgs& A, const Wav
     const bool live = q < TE && slot < n_act;
     const int64_t item = live ? (A.act ? (int64_t)A.act[slot] : slot) : 0;
     auto seg_sum = [&](int g) {
+      constexpr int kBatch = 8;  // partials in flight at a time
+      const double* p = A.part + (tile * P.nseg + g) * P.spans * (int64_t)TE + q;
       double t = 0;
-      for (int sp = 0; sp < P.spans; ++sp) t += __ldcg(A.part + ((tile * P.nseg + g) * P.spans + sp) * TE + q);
+      int sp = 0;
+      for (; sp + kBatch <= P.spans; sp += kBatch) {
+        double v[kBatch];
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) v[b] = __ldcg(p + (int64_t)(sp + b) * TE);
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) t += v[b];
+      }
+      for (; sp < P.spans; ++sp) t += __ldcg(p + (int64_t)sp * TE);
       return t;
     };
     bool finished = false, unconverged = false, survive = false;
@@ -507,6 +517,24 @@ __device__ __forceinline__ void pd_tile_finalize(const PdFinalArgs& A, const Wav
     }
     finalize_bookkeeping(finished, unconverged, survive, item, A.level, A.act_next, A.n_next, A.not_converged,
                          A.samples, A.level_max);
+  }
+}
+
+// End of a unit of a power-density wave: publish this CTA's partial, count the tile's finished units,
+// and let the CTA that finished the last one finalize the tile.
+__device__ __forceinline__ void pd_unit_done(const PdWaveArgs& A, const WavePlan& P, int64_t tile, int64_t n_act,
+                                             int* s_last, int TE, int units) {
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned done = atomicAdd(&A.tile_done[tile], 1u);
+    *s_last = done == (unsigned)(units - 1);
+    if (*s_last) __threadfence();
+  }
+  __syncthreads();
+  if (*s_last) {
+    pd_tile_finalize(A.fin, P, tile, n_act, TE);
+    if (threadIdx.x == 0) A.tile_done[tile] = 0;
   }
 }
 

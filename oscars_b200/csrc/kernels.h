@@ -138,7 +138,6 @@ struct PdFinalArgs {
   int* level_out;
   unsigned long long* not_converged;
   unsigned long long* samples;
-  unsigned long long* work_reset;
   unsigned* level_max;      // highest level at which an entry finished (may be NULL)
 };
 
@@ -153,13 +152,12 @@ struct PdWaveArgs {
   const unsigned* n_act;
   int first, level, tile_entries, min_span;
   int64_t target_units;
-  double* part;             // partials, entry-major: [slot][seg][span]; fused: [tile][seg][span][entry in tile]
+  double* part;             // partials, [tile][seg][span][entry in tile]
   unsigned* err;
   unsigned long long* work;
-  // Fused finalize (the mixed kernel): the last CTA to finish a tile's spans applies the stop rule of
-  // `fin` to the tile's entries and appends survivors; zero_u32 / zero_u64 are the counters of the
-  // following wave, zeroed by block 0 at start.
-  int fused;
+  // The last CTA to finish a tile's spans applies the stop rule of `fin` to the tile's entries and
+  // appends survivors; zero_u32 / zero_u64 are the counters of the following wave, zeroed by block 0 at
+  // start.
   unsigned* tile_done;
   unsigned* zero_u32;
   unsigned long long* zero_u64;
@@ -242,11 +240,11 @@ cudaError_t launch_level_fill(const double* knots, int64_t n, double tstart, dou
 cudaError_t launch_fd_wave_fp64(const FdWaveArgs& a, int grid, int variant, cudaStream_t st);
 cudaError_t launch_fd_finalize(const FdFinalArgs& a, int64_t n_act_bound, cudaStream_t st);
 cudaError_t launch_pd_wave_fp64(const PdWaveArgs& a, int grid, cudaStream_t st);
+int pd_fp64_entries_per_cta();
 // Mixed-precision power density over the pair records (kernels_mixed.cu): a.lev = the records,
-// partials entry-major like the FP64 kernel's, tile_entries = pd_mixed_entries_per_cta().
+// tile_entries = pd_mixed_entries_per_cta().
 cudaError_t launch_pd_wave_mixed(const PdWaveArgs& a, const MixedFrame& F, int grid, cudaStream_t st);
 int pd_mixed_entries_per_cta();
 int pd_mixed_blocks_per_sm();
-cudaError_t launch_pd_finalize(const PdFinalArgs& a, int64_t n_act_bound, cudaStream_t st);
 
 }  // namespace osc

@@ -16,6 +16,7 @@
 // reference's stop rule and compacts the still-active entries for the next wave.
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <type_traits>
 
 #include "device_common.cuh"
 #include "fd_common.cuh"
@@ -358,144 +359,156 @@ __global__ void k_fd_finalize(FdFinalArgs A) {
 // ---------------------------------------------------------------------------------------------
 // Power density (src/OSCARSSR.cc:2869-2922):
 //   sum += [(N1 x ((N1 - b) x a/c)) . Nk]^2 / (1 - b.N1)^5 / |O - X|^2 * (N1 . normal),  k = 2, 3
-// N1 and 1 - b.N1 keep the reference's operations (the difference is ill-conditioned, so its value
-// depends on them); the well-conditioned rest is summed as |N1 x W|^2 / ((1 - b.N1)^5 |O - X|^2),
-// equal to the two projections to rounding.
+// N1, N1 . normal and 1 - b.N1 round as the reference's operations do (the difference is
+// ill-conditioned, and the directional cut is a sign); the well-conditioned rest is
+// |u (N1.a) - a (N1.u)|^2, u = N1 - b, the squared norm of the numerator, which lies across N1 and so
+// equals the sum of its squared projections on N2 and N3, times the fifth power of 1 / (1 - b.N1) and
+// 1 / |O - X|^2.
+// Sample-split and fused like the flux waves; 67 FP64 instructions per (entry, sample) (with the
+// library's square root and four divisions: ~130, a separate finalize launch and 128 entries per CTA).
 // ---------------------------------------------------------------------------------------------
 constexpr int kPdThreads = 128;
 constexpr int kPdChunk = 128;
+constexpr int kPdSub = 4;                       // groups of a CTA
+constexpr int kPdTile = kPdThreads / kPdSub;    // entries per CTA
 
-__device__ __forceinline__ void unit3(double x, double y, double z, double& ux, double& uy, double& uz) {
-  const double m = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z)));
-  ux = __ddiv_rn(x, m); uy = __ddiv_rn(y, m); uz = __ddiv_rn(z, m);
+template <bool NORMAL, bool DIRECTIONAL>
+__device__ __forceinline__ double pd_term(double X, double Y, double Z, double bx, double by, double bz, double ax,
+                                          double ay, double az, double Ox, double Oy, double Oz, double Nx, double Ny,
+                                          double Nz) {
+  const double Rx = __dsub_rn(Ox, X), Ry = __dsub_rn(Oy, Y), Rz = __dsub_rn(Oz, Z);
+  const double s = __dadd_rn(__dadd_rn(__dmul_rn(Rx, Rx), __dmul_rn(Ry, Ry)), __dmul_rn(Rz, Rz));
+  const double y = rsqrt_near(s), D = sqrt_by(s, y);
+  const double nx = quot_by(Rx, D, y), ny = quot_by(Ry, D, y), nz = quot_by(Rz, D, y);
+  const double om =
+      __dsub_rn(1.0, __dadd_rn(__dadd_rn(__dmul_rn(bx, nx), __dmul_rn(by, ny)), __dmul_rn(bz, nz)));
+  const double ux = __dsub_rn(nx, bx), uy = __dsub_rn(ny, by), uz = __dsub_rn(nz, bz);
+  const double na = fma(nx, ax, fma(ny, ay, nz * az));
+  const double nu = fma(nx, ux, fma(ny, uy, nz * uz));
+  const double mx = fma(ux, na, -(ax * nu)), my = fma(uy, na, -(ay * nu)), mz = fma(uz, na, -(az * nu));
+  const double io = rcp_near(om), io2 = io * io;
+  double t = fma(mx, mx, fma(my, my, mz * mz)) * (io2 * io2 * io) * (y * y);
+  if (NORMAL) {
+    const double n1dn = __dadd_rn(__dadd_rn(__dmul_rn(nx, Nx), __dmul_rn(ny, Ny)), __dmul_rn(nz, Nz));
+    t = DIRECTIONAL && n1dn <= 0 ? 0.0 : t * n1dn;
+  }
+  return t;
 }
 
-__global__ void __launch_bounds__(kPdThreads) k_pd_wave_fp64(PdWaveArgs A) {
-  __shared__ __align__(16) Stage<10, kPdChunk> st;
-  const int tid = threadIdx.x;
-  const int64_t n_act = A.act ? (int64_t)*A.n_act : A.n_items;
-  // the plan is uniform over the CTA; keeping it in shared memory frees the registers its
-  // fields would otherwise hold across the sample loop
+__global__ void __launch_bounds__(kPdThreads, 5) k_pd_wave_fp64(PdWaveArgs A) {
+  constexpr int TE = kPdTile, SUB = kPdSub;
+  if (A.tile_entries != TE) {  // the host sized the partials for another tile
+    if (threadIdx.x == 0) atomicOr(A.err, kErrPlan);
+    return;
+  }
+  __shared__ __align__(16) Stage<9, kPdChunk> st;  // x y z beta a/c: the times are not needed
+  __shared__ double red[SUB - 1][TE];
   __shared__ WavePlan P;
-  if (threadIdx.x == 0) P = wave_plan(A.first, A.level, n_act, kPdThreads, A.target_units, A.min_span);
-  __syncthreads();
-  const int64_t units = P.tiles * P.spans;
+  __shared__ int64_t next_unit;
+  __shared__ int s_last;
+  const int tid = threadIdx.x;
+  const int grp = tid / TE, q = tid % TE;
+  launch_dependents();
   if (tid == 0) {
     mbar_init(&st.bar[0], 1);
     mbar_init(&st.bar[1], 1);
     fence_barrier_init();
   }
+  wait_predecessor();
+  if (blockIdx.x == 0 && tid == 0) {  // counters of the following wave
+    if (A.zero_u32) *A.zero_u32 = 0;
+    if (A.zero_u64) *A.zero_u64 = 0;
+  }
+  const int64_t n_act = A.act ? (int64_t)*A.n_act : A.n_items;
+  if (tid == 0) P = wave_plan(A.first, A.level, n_act, TE, A.target_units, A.min_span);
   __syncthreads();
-  uint32_t phase_bits = 0;
-  __shared__ int64_t next_unit;
-  for (;;) {  // CTAs take (tile, span) units from a shared counter until the wave's units run out
-    if (tid == 0) next_unit = (int64_t)atomicAdd(A.work, 1ull);
-    __syncthreads();
-    const int64_t u = next_unit;
-    __syncthreads();
-    if (u >= units) break;
-    const int64_t tile = u / P.spans;
-    const int span = (int)(u % P.spans);
-    const int64_t slot = tile * kPdThreads + tid;
+  // units (tile, segment, span) and their early requests as in k_fd_wave_fp64
+  const int64_t units = (P.tiles * P.nseg) << P.log2_spans;
+  auto unit_range = [&](int64_t u, int64_t& b0, int64_t& b1) {
+    const int64_t r = u >> P.log2_spans;
+    const int g = P.nseg == 2 ? (int)(r & 1) : 0;
+    b0 = seg_begin(P, g) + (u & (P.spans - 1)) * seg_span(P, g);
+    b1 = min(seg_end(P, g), b0 + seg_span(P, g));
+  };
+  auto issue = [&](int64_t lo, int64_t end, int b) {
+    const int64_t hi = min(end, lo + kPdChunk);
+    stage_issue<9, kPdChunk>(st, b, A.lev + A.cap, A.cap, lo & ~(int64_t)1, (hi + 1) & ~(int64_t)1);
+  };
+  uint32_t staged = 0;
+  int64_t u = blockIdx.x;
+  if (tid == 0 && u < units) {
+    int64_t b0, b1;
+    unit_range(u, b0, b1);
+    if (b0 < b1) issue(b0, b1, 0);
+  }
+  while (u < units) {
+    int64_t after = 0;
+    if (tid == 0) after = (int64_t)gridDim.x + (int64_t)atomicAdd(A.work, 1ull);
+    int64_t b0, b1;
+    unit_range(u, b0, b1);
+    const int64_t nchunks = b1 > b0 ? (b1 - b0 + kPdChunk - 1) / kPdChunk : 0;
+    const int span = (int)u & (P.spans - 1);
+    const int g = P.nseg == 2 ? (int)(u >> P.log2_spans) & 1 : 0;
+    const int64_t tile = u >> (P.log2_spans + P.nseg - 1);
+    const int64_t slot = tile * TE + q;
     const bool live = slot < n_act;
     const int64_t item = live ? (A.act ? (int64_t)A.act[slot] : slot) : 0;
     const double Ox = A.obs[3 * item], Oy = A.obs[3 * item + 1], Oz = A.obs[3 * item + 2];
     double Nx = 0, Ny = 0, Nz = 0;
     if (A.has_normal) { Nx = A.normals[3 * item]; Ny = A.normals[3 * item + 1]; Nz = A.normals[3 * item + 2]; }
-    for (int g = 0; g < P.nseg; ++g) {
-      const int64_t b0 = seg_begin(P, g) + (int64_t)span * seg_span(P, g);
-      const int64_t b1 = min(seg_end(P, g), b0 + seg_span(P, g));
-      double sum = 0;
-      const int64_t nchunks = b1 > b0 ? (b1 - b0 + kPdChunk - 1) / kPdChunk : 0;
-      if (tid == 0 && nchunks > 0) {
-        const int64_t lo = b0, hi = min(b1, b0 + kPdChunk);
-        stage_issue<10, kPdChunk>(st, 0, A.lev, A.cap, lo & ~(int64_t)1, (hi + 1) & ~(int64_t)1);
+    double sum = 0;
+    for (int64_t c = 0; c < nchunks; ++c, ++staged) {
+      const int buf = (int)(staged & 1u);
+      const int64_t lo = b0 + c * kPdChunk, hi = min(b1, lo + kPdChunk);
+      if (tid == 0) {
+        if (c + 1 < nchunks) {
+          issue(lo + kPdChunk, b1, buf ^ 1);
+        } else if (after < units) {
+          int64_t n0, n1;
+          unit_range(after, n0, n1);
+          if (n0 < n1) issue(n0, n1, buf ^ 1);
+        }
       }
-      for (int64_t c = 0; c < nchunks; ++c) {
-        const int buf = (int)(c & 1);
-        const int64_t lo = b0 + c * kPdChunk, hi = min(b1, lo + kPdChunk);
-        if (tid == 0 && c + 1 < nchunks) {
-          const int64_t lo2 = lo + kPdChunk, hi2 = min(b1, lo2 + kPdChunk);
-          stage_issue<10, kPdChunk>(st, buf ^ 1, A.lev, A.cap, lo2 & ~(int64_t)1, (hi2 + 1) & ~(int64_t)1);
-        }
-        if (!mbar_wait(&st.bar[buf], (phase_bits >> buf) & 1u)) {
-          if (tid == 0) atomicOr(A.err, kErrTmaTimeout);
-          return;
-        }
-        phase_bits ^= 1u << buf;
-        const int64_t lo_al = lo & ~(int64_t)1;
-        const int j0 = (int)(max(lo, (int64_t)1) - lo_al), j1 = (int)(hi - lo_al);
-        if (live) {
-          for (int j = j0; j < j1; ++j) {
-            const double Rx = __dsub_rn(Ox, st.v[buf][1][j]), Ry = __dsub_rn(Oy, st.v[buf][2][j]), Rz = __dsub_rn(Oz, st.v[buf][3][j]);
-            // N1 and 1 - B.N1 with the reference's operations: the difference 1 - B.N1 (~1e-8) carries
-            // the rounding of B.N1, which its result shares
-            double n1x, n1y, n1z;
-            unit3(Rx, Ry, Rz, n1x, n1y, n1z);
-            const double n1dn = A.has_normal
-                                    ? __dadd_rn(__dadd_rn(__dmul_rn(n1x, Nx), __dmul_rn(n1y, Ny)), __dmul_rn(n1z, Nz))
-                                    : 1.0;
-            if (A.directional && n1dn <= 0) continue;
-            const double bx = st.v[buf][4][j], by = st.v[buf][5][j], bz = st.v[buf][6][j];
-            const double ax = st.v[buf][7][j], ay = st.v[buf][8][j], az = st.v[buf][9][j];
-            const double ux = __dsub_rn(n1x, bx), uy = __dsub_rn(n1y, by), uz = __dsub_rn(n1z, bz);
-            const double wx = __dsub_rn(__dmul_rn(uy, az), __dmul_rn(ay, uz));
-            const double wy = __dsub_rn(__dmul_rn(uz, ax), __dmul_rn(az, ux));
-            const double wz = __dsub_rn(__dmul_rn(ux, ay), __dmul_rn(ax, uy));
-            const double mx = __dsub_rn(__dmul_rn(n1y, wz), __dmul_rn(wy, n1z));
-            const double my = __dsub_rn(__dmul_rn(n1z, wx), __dmul_rn(wz, n1x));
-            const double mz = __dsub_rn(__dmul_rn(n1x, wy), __dmul_rn(wx, n1y));
-            const double bdn = __dadd_rn(__dadd_rn(__dmul_rn(bx, n1x), __dmul_rn(by, n1y)), __dmul_rn(bz, n1z));
-            // the rest is well conditioned: the squared projections on N2 and N3 (an orthonormal pair
-            // across N1) sum to |N1 x W|^2, which is across N1; (1 - B.N1)^5 by products; one division
-            const double om = __dsub_rn(1.0, bdn), om2 = om * om;
-            const double m2 = __dadd_rn(__dadd_rn(__dmul_rn(Rx, Rx), __dmul_rn(Ry, Ry)), __dmul_rn(Rz, Rz));
-            const double num = fma(mx, mx, fma(my, my, mz * mz));
-            sum = fma(num / (om2 * om2 * om * m2), n1dn, sum);
-          }
-        }
-        __syncthreads();
+      if (!mbar_wait(&st.bar[buf], (staged >> 1) & 1u)) {
+        if (tid == 0) atomicOr(A.err, kErrTmaTimeout);
+        return;
       }
-      if (live) A.part[slot * P.nseg * P.spans + g * P.spans + span] = sum;
+      const int64_t lo_al = lo & ~(int64_t)1;
+      const int ja = (int)(max(lo, (int64_t)1) - lo_al), jb = (int)(hi - lo_al);  // sample 0 is the unused slot
+      const int j0 = ja + ((jb - ja) * grp) / SUB, j1 = ja + ((jb - ja) * (grp + 1)) / SUB;  // this group's part
+      auto add = [&](auto normal, auto directional) {
+#pragma unroll 2
+        for (int j = j0; j < j1; ++j)
+          sum += pd_term<normal.value, directional.value>(
+              st.v[buf][0][j], st.v[buf][1][j], st.v[buf][2][j], st.v[buf][3][j], st.v[buf][4][j], st.v[buf][5][j],
+              st.v[buf][6][j], st.v[buf][7][j], st.v[buf][8][j], Ox, Oy, Oz, Nx, Ny, Nz);
+      };
+      if (live) {
+        if (A.has_normal && A.directional) add(std::true_type{}, std::true_type{});
+        else if (A.has_normal) add(std::true_type{}, std::false_type{});
+        else add(std::false_type{}, std::false_type{});
+      }
+      __syncthreads();  // everyone is done with `buf` before it is refilled
     }
+    if (nchunks == 0) {  // (no unit of a planned wave is empty)
+      if (tid == 0 && after < units) {
+        int64_t n0, n1;
+        unit_range(after, n0, n1);
+        if (n0 < n1) issue(n0, n1, (int)(staged & 1u));
+      }
+      __syncthreads();
+    }
+    // the groups' sums in group order; group 0 stores the span's partial
+    if (grp > 0) red[grp - 1][q] = sum;
+    __syncthreads();
+    if (grp == 0 && live) {
+      for (int o = 0; o < SUB - 1; ++o) sum += red[o][q];
+      A.part[((tile * P.nseg + g) * P.spans + span) * TE + q] = sum;
+    }
+    if (tid == 0) next_unit = after;
+    pd_unit_done(A, P, tile, n_act, &s_last, TE, P.nseg * P.spans);
+    u = next_unit;
   }
-}
-
-// src/OSCARSSR.cc:2924-2968
-__global__ void k_pd_finalize(PdFinalArgs A) {
-  if (blockIdx.x == 0 && threadIdx.x == 0 && A.work_reset) *A.work_reset = 0;
-  const int64_t n_act = A.act ? (int64_t)*A.n_act : A.n_items;
-  const int lane = threadIdx.x % kFinLanes;
-  const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kFinLanes;
-  if ((int64_t)blockIdx.x * blockDim.x / kFinLanes >= n_act) return;
-  const bool live = slot < n_act;
-  const WavePlan P = wave_plan(A.first, A.level, n_act, A.tile_entries, A.target_units, A.min_span);
-  const int64_t item = live ? (A.act ? (int64_t)A.act[slot] : slot) : 0;
-  const int64_t N = A.n_items;
-  auto seg_sum = [&](int g) {
-    double t = 0;
-    if (live)
-      for (int sp = lane; sp < P.spans; sp += kFinLanes) t += A.part[slot * P.nseg * P.spans + g * P.spans + sp];
-    return group_sum(t);
-  };
-  double sum = 0, last_sum = -1;
-  if (A.first) {
-    if (P.nseg == 2) {
-      sum += seg_sum(0);
-      last_sum = sum * A.dt_prev;
-    }
-    sum += seg_sum(P.nseg - 1);
-  } else {
-    if (live) {
-      sum = A.state[item];
-      last_sum = A.state[N + item];
-    }
-    sum += seg_sum(0);
-  }
-  bool finished = false, unconverged = false, survive = false;
-  if (live && lane == 0) pd_entry_decide(A, item, sum, last_sum, finished, unconverged, survive);
-  finalize_bookkeeping(finished, unconverged, survive, item, A.level, A.act_next, A.n_next, A.not_converged, A.samples,
-                       A.level_max);
 }
 
 }  // namespace dev
@@ -549,17 +562,9 @@ cudaError_t launch_fd_finalize(const FdFinalArgs& a, int64_t n_act_bound, cudaSt
   return cudaGetLastError();
 }
 
+int pd_fp64_entries_per_cta() { return dev::kPdTile; }
 cudaError_t launch_pd_wave_fp64(const PdWaveArgs& a, int grid, cudaStream_t st) {
-  dev::k_pd_wave_fp64<<<grid, dev::kPdThreads, 0, st>>>(a);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_pd_finalize(const PdFinalArgs& a, int64_t n_act_bound, cudaStream_t st) {
-  if (n_act_bound == 0) return cudaSuccess;
-  const int T = 256;
-  const int64_t threads = n_act_bound * dev::kFinLanes;
-  dev::k_pd_finalize<<<(unsigned)((threads + T - 1) / T), T, 0, st>>>(a);
-  return cudaGetLastError();
+  return launch_overlapped(dev::k_pd_wave_fp64, grid, dev::kPdThreads, st, a);
 }
 
 int fp64_blocks_per_sm(bool power_density, int variant) {

@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(kMxThreads, MINB) k_fd_wave_mixed_pair(FdWaveA
 // for any direction) and the numerator run on packed f32x2 operands in the particle frame; the fifth
 // power of 1 / (1 - b.N1) (~1e40 near the axis, beyond FP32) and the sums in FP64.  Sample-split like
 // the flux kernel: SUB groups of TE = 128 / SUB entries, each taking 1/SUB of every staged chunk, the
-// groups' sums reduced in group order; entry-major partials for k_pd_finalize.
+// groups' sums reduced in group order; the CTA that finishes a tile's last span finalizes it.
 // ---------------------------------------------------------------------------------------------
 struct PdObsMx {
   float2 ox, oy, oz;  // observer in the particle frame (both lanes)
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kMxThreads, MINB) k_pd_wave_mixed(PdWaveArgs A
   const int grp = tid / TE, q = tid % TE;
   launch_dependents();
   wait_predecessor();
-  if (A.fused && blockIdx.x == 0 && tid == 0) {  // counters of the following wave
+  if (blockIdx.x == 0 && tid == 0) {  // counters of the following wave
     if (A.zero_u32) *A.zero_u32 = 0;
     if (A.zero_u64) *A.zero_u64 = 0;
   }
@@ -397,33 +397,18 @@ __global__ void __launch_bounds__(kMxThreads, MINB) k_pd_wave_mixed(PdWaveArgs A
         }
         __syncthreads();  // everyone is done with `buf` before it is refilled
       }
-      // reduce the groups' sums in group order; group 0 stores the span's partial (entry-major, or
-      // tile-major for the fused finalize)
+      // reduce the groups' sums in group order; group 0 stores the span's partial, tile-major
       if (SUB > 1 && grp > 0) red[grp - 1][q] = S;
       if (SUB > 1) __syncthreads();
       if (grp == 0) {
         for (int o2 = 0; o2 < SUB - 1; ++o2) S += red[o2][q];
         if (live) {
-          if (A.fused) A.part[((tile * P.nseg + g) * P.spans + span) * TE + q] = S;
-          else A.part[slot * P.nseg * P.spans + g * P.spans + span] = S;
+          A.part[((tile * P.nseg + g) * P.spans + span) * TE + q] = S;
         }
       }
       if (SUB > 1) __syncthreads();
     }
-    if (A.fused) {  // the CTA that finishes a tile's last span finalizes the tile
-      __threadfence();
-      __syncthreads();
-      if (tid == 0) {
-        const unsigned done = atomicAdd(&A.tile_done[tile], 1u);
-        s_last = done == (unsigned)(P.spans - 1);
-        if (s_last) __threadfence();
-      }
-      __syncthreads();
-      if (s_last) {
-        pd_tile_finalize(A.fin, P, tile, n_act, TE);
-        if (tid == 0) A.tile_done[tile] = 0;
-      }
-    }
+    pd_unit_done(A, P, tile, n_act, &s_last, TE, P.spans);
   }
 }
 

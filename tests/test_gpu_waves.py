@@ -57,3 +57,13 @@ def test_mixed_spectrum_lines_match_general_kernel(n, level):
         out.append((f, s.last_levels.copy()))
     assert np.array_equal(out[0][1], out[1][1])
     assert np.max(np.abs(out[0][0] - out[1][0])) <= 1e-10 * np.max(np.abs(out[0][0]))
+
+
+# Power density: N1, N1 . normal and 1 - b.N1 have the oracle's bits, the rest of a term about 40 roundings
+# (5e-15), and the terms of a point have one sign: 1e-12.
+@pytest.mark.parametrize("nx, ny, normal, plane, level", [(1, 1, 0, "XY", 0), (31, 1, 1, "XY", 3), (3, 11, -1, "XY", 9),
+                                                          (5, 13, 0, "XY", 10), (9, 7, 1, "XZ", 11), (8, 16, -1, "YZ", 12)])
+def test_fp64_power_density_tiles_and_levels(nx, ny, normal, plane, level):
+    kw = dict(npoints=[nx, ny], plane=plane, width=[0.02, 0.03], normal=normal, translation=[0, 0.01, 20], max_level=level)
+    got, want = _both("calculate_power_density_rectangle", kw)
+    assert np.max(np.abs(got - want)) <= 1e-12 * max(np.max(np.abs(want)), 1e-300)
