@@ -275,6 +275,19 @@ OSC_API int osc_power_density(osc_ctx* ctx, const double* obs_xyz, const double*
  * out / level_out: n values / stop levels; a facet that does not stop reports the level of the last
  * facet before it that did (the reference's Result_Level), counted in n_not_converged.  opts: the
  * precision, levels, nparticles and quantity fields are used. */
+/* The same on a rectangle given by its description (osc_surface_rectangle): the observers (and the
+ * normals of the power density) are formed on the device, so nothing is uploaded, and the positions the
+ * caller asks for (xyz, x1x2: 3 x nx1 x nx2 doubles each, either may be NULL) are written on the host
+ * while the device computes. */
+OSC_API int osc_flux_rectangle(osc_ctx* ctx, const char* plane, int nx1, int nx2, double width1, double width2,
+                               const double rotations[3], const double translation[3], int normal,
+                               double energy_eV, const osc_rad_opts* opts, double* xyz, double* x1x2,
+                               double* out, int32_t* level_out, long long* n_not_converged);
+OSC_API int osc_power_density_rectangle(osc_ctx* ctx, const char* plane, int nx1, int nx2, double width1,
+                                        double width2, const double rotations[3], const double translation[3],
+                                        int normal, int directional, const osc_rad_opts* opts, double* xyz,
+                                        double* x1x2, double* out, int32_t* level_out,
+                                        long long* n_not_converged);
 OSC_API int osc_power_density_stl(osc_ctx* ctx, const double* facets, const double* centers, long long n,
                                   const osc_rad_opts* opts, double* out, int32_t* level_out,
                                   long long* n_not_converged);

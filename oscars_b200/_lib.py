@@ -84,6 +84,10 @@ SIGNATURES = {
     "osc_surface_x0x1x2": (I, [I, I, DP, DP, DP, I, DP, DP, DP]),
     "osc_surface_points": (I, [LL, DP, DP, DP, DP, I, DP, DP]),
     "osc_flux": (I, [VP, DP, LL, D, ctypes.POINTER(RadOpts), DP, I32P, LLP]),
+    "osc_flux_rectangle": (I, [VP, ctypes.c_char_p, I, I, D, D, DP, DP, I, D, ctypes.POINTER(RadOpts), DP, DP, DP,
+                               I32P, LLP]),
+    "osc_power_density_rectangle": (I, [VP, ctypes.c_char_p, I, I, D, D, DP, DP, I, I, ctypes.POINTER(RadOpts), DP, DP,
+                                        DP, I32P, LLP]),
     "osc_spectrum": (I, [VP, DP, DP, LL, ctypes.POINTER(RadOpts), DP, I32P, LLP]),
     "osc_flux_multi": (I, [VP, DP, LL, DP, LL, ctypes.POINTER(RadOpts), I, DP, I32P, LLP]),
     "osc_power_density": (I, [VP, DP, DP, LL, I, ctypes.POINTER(RadOpts), DP, I32P, LLP]),

@@ -578,6 +578,42 @@ OSC_API int osc_flux(osc_ctx* ctx, const double* obs_xyz, long long n_obs, doubl
   });
 }
 
+// The rectangle calls: observers formed on the device, the caller's position arrays filled and its
+// result pages touched on the host meanwhile.
+static void rectangle_request(osc_ctx* ctx, osc::RadRequest& rq, const char* plane, int nx1, int nx2, double w1, double w2,
+                              const double* rotations, const double* translation, int normal, const osc_rad_opts* opts,
+                              double* xyz, double* x1x2, double* out, int32_t* level_out, long long* n_not_converged) {
+  check_opts(opts);
+  if (!plane || !out) throw osc::Error{OSC_ERR_INVALID, "bad buffers"};
+  if (nx1 <= 0 || nx2 <= 0) throw osc::Error{OSC_ERR_INVALID, "an entry in 'npoints' is <= 0"};
+  const osc::RectSurface rect = osc::rectangle_layout(plane, nx1, nx2, w1, w2, V3(rotations), V3(translation), normal);
+  const long long n = (long long)nx1 * nx2;
+  rq.rect = &rect;
+  rq.n_obs = n;
+  rq.opts = *opts;
+  rq.out = out;
+  rq.level_out = level_out;
+  rq.meanwhile = [&] {
+    if (xyz || x1x2) osc::rectangle_points(rect, xyz, nullptr, x1x2);
+    std::memset(out, 0, sizeof(double) * n);
+    if (level_out) std::memset(level_out, 0, sizeof(int32_t) * n);
+  };
+  ctx->eng->radiation(rq);
+  if (n_not_converged) *n_not_converged = ctx->eng->last_not_converged;
+}
+
+OSC_API int osc_flux_rectangle(osc_ctx* ctx, const char* plane, int nx1, int nx2, double width1, double width2,
+                               const double rotations[3], const double translation[3], int normal, double energy_eV,
+                               const osc_rad_opts* opts, double* xyz, double* x1x2, double* out, int32_t* level_out,
+                               long long* n_not_converged) {
+  return guarded(ctx, [&] {
+    osc::RadRequest rq;
+    rq.omega = {osc::ev_to_omega(energy_eV)};
+    rectangle_request(ctx, rq, plane, nx1, nx2, width1, width2, rotations, translation, normal, opts, xyz, x1x2, out,
+                      level_out, n_not_converged);
+  });
+}
+
 OSC_API int osc_spectrum(osc_ctx* ctx, const double obs[3], const double* energies_eV, long long n_energies,
                          const osc_rad_opts* opts, double* out, int32_t* level_out, long long* n_not_converged) {
   return guarded(ctx, [&] {
@@ -774,6 +810,19 @@ OSC_API int osc_power_density(osc_ctx* ctx, const double* obs_xyz, const double*
     rq.level_out = level_out;
     ctx->eng->radiation(rq);
     if (n_not_converged) *n_not_converged = ctx->eng->last_not_converged;
+  });
+}
+
+OSC_API int osc_power_density_rectangle(osc_ctx* ctx, const char* plane, int nx1, int nx2, double width1, double width2,
+                                        const double rotations[3], const double translation[3], int normal,
+                                        int directional, const osc_rad_opts* opts, double* xyz, double* x1x2, double* out,
+                                        int32_t* level_out, long long* n_not_converged) {
+  return guarded(ctx, [&] {
+    osc::RadRequest rq;
+    rq.power_density = true;
+    rq.directional = directional != 0;
+    rectangle_request(ctx, rq, plane, nx1, nx2, width1, width2, rotations, translation, normal, opts, xyz, x1x2, out,
+                      level_out, n_not_converged);
   });
 }
 

@@ -15,6 +15,7 @@
 #include <mutex>
 #include <thread>
 
+#include "device_common.cuh"
 #include "kernels.h"
 
 namespace osc {
@@ -58,13 +59,17 @@ Engine::Engine(int dev) : device(dev) {
   mrec_bd_.reserve(32 * sizeof(unsigned long long));
   cnt_.reserve(64);
   check(cudaMemset(cnt_.p, 0, 64), "memset");
-  check(cudaHostAlloc(reinterpret_cast<void**>(&stats_host_), kStatWords * kStatSlots * sizeof(unsigned long long),
-                      cudaHostAllocMapped),
-        "cudaHostAlloc");
-  check(cudaHostAlloc(reinterpret_cast<void**>(&stage_host_), kStageDoubles * sizeof(double), cudaHostAllocMapped),
-        "cudaHostAlloc");
-  check(cudaHostAlloc(reinterpret_cast<void**>(&ctl_host_), 16 * sizeof(unsigned), cudaHostAllocMapped),
-        "cudaHostAlloc");
+  {  // one mapped page-locked block: statistics ring, staging, control words, small results
+    const size_t b_stat = kStatWords * kStatSlots * sizeof(unsigned long long), b_stage = kStageDoubles * sizeof(double);
+    const size_t b_ctl = 64, b_tail = kTailEntries * (sizeof(double) + sizeof(int32_t));
+    check(cudaHostAlloc(reinterpret_cast<void**>(&mapped_), b_stat + b_stage + b_ctl + b_tail, cudaHostAllocMapped),
+          "cudaHostAlloc");
+    stats_host_ = reinterpret_cast<unsigned long long*>(mapped_);
+    stage_host_ = reinterpret_cast<double*>(mapped_ + b_stat);
+    ctl_host_ = reinterpret_cast<unsigned*>(mapped_ + b_stat + b_stage);
+    tail_host_ = reinterpret_cast<double*>(mapped_ + b_stat + b_stage + b_ctl);
+    std::memset(ctl_host_, 0, b_ctl);
+  }
   for (int i = 0; i < kStatSlots; ++i) check(cudaEventCreateWithFlags(&stats_ev_[i], cudaEventDisableTiming), "event");
   check(cudaEventCreateWithFlags(&stage_ev_, cudaEventDisableTiming), "event");
   check(cudaEventCreateWithFlags(&order_ev_, cudaEventDisableTiming), "event");
@@ -97,9 +102,8 @@ Engine::~Engine() {
   for (cudaEvent_t e : {in_fork_ev_, in_ev_})
     if (e) cudaEventDestroy(e);
   if (last_stream_valid_ && last_stream_ != stream) cudaStreamSynchronize(last_stream_);
-  if (stats_host_) cudaFreeHost(stats_host_);
-  if (stage_host_) cudaFreeHost(stage_host_);
-  if (ctl_host_) cudaFreeHost(ctl_host_);
+  if (mapped_) cudaFreeHost(mapped_);
+  if (bounce_) cudaFreeHost(bounce_);
   for (PinnedStage& p : pin_pool_) {
     if (p.copied) {
       cudaEventSynchronize(p.copied);
@@ -431,20 +435,42 @@ __global__ void k_stats_out(const unsigned long long* __restrict__ c64, const un
 }
 
 // Start of a request in one launch: zero up to three ranges of 32-bit words (the request's counters,
-// the fused-finalize counters, the beta-step maxima of the levels to fill) and copy the frequencies
-// from the mapped staging buffer.
+// the fused-finalize counters, the beta-step maxima of the levels to fill), copy what is staged in
+// mapped memory (frequencies, then the observers and normals of small requests) and form the points of
+// a rectangle (the host's operations on its start and step vectors, so the same bits).
 struct ZeroRange {
   unsigned* p;
   int64_t words;
 };
-__global__ void k_request_prologue(ZeroRange z0, ZeroRange z1, ZeroRange z2, const double* __restrict__ om_src,
-                                   double* __restrict__ om_dst, int64_t n_om) {
+struct PrologueCopy {
+  const double* src;
+  double *om, *obs, *nrm;
+  int64_t n_om, n_obs, n_nrm;  // doubles
+};
+struct PrologueRect {
+  int64_t n;  // points (0: none)
+  int nx2;
+  double start[3], v1[3], v2[3], normal[3];
+  double *obs, *nrm;
+};
+__global__ void k_request_prologue(ZeroRange z0, ZeroRange z1, ZeroRange z2, PrologueCopy c, PrologueRect r) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   for (int64_t i = t0; i < z0.words; i += stride) z0.p[i] = 0u;
   for (int64_t i = t0; i < z1.words; i += stride) z1.p[i] = 0u;
   for (int64_t i = t0; i < z2.words; i += stride) z2.p[i] = 0u;
-  for (int64_t i = t0; i < n_om; i += stride) om_dst[i] = om_src[i];
+  for (int64_t i = t0; i < c.n_om; i += stride) c.om[i] = c.src[i];
+  for (int64_t i = t0; i < c.n_obs; i += stride) c.obs[i] = c.src[c.n_om + i];
+  for (int64_t i = t0; i < c.n_nrm; i += stride) c.nrm[i] = c.src[c.n_om + c.n_obs + i];
+  for (int64_t i = t0; i < r.n; i += stride) {
+    const int64_t i1 = i / r.nx2;
+    const double x1 = (double)i1, x2 = (double)(i - i1 * r.nx2);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      r.obs[3 * i + k] = __dadd_rn(__dadd_rn(r.start[k], __dmul_rn(r.v1[k], x1)), __dmul_rn(r.v2[k], x2));
+      if (r.nrm) r.nrm[3 * i + k] = r.normal[k];
+    }
+  }
 }
 
 int Engine::pick_variant(int kind, RadRequest& rq, int64_t n_items, int Lfirst, int lstop, double* d_out,
@@ -567,21 +593,38 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
         z2 = ZeroRange{bd_bits_.as<unsigned>(), 64};
       }
     }
-    const int64_t n_om = omega_staged_;
-    const int64_t words = std::max<int64_t>(std::max<int64_t>(z0.words, z1.words), std::max<int64_t>(z2.words, n_om));
-    const int blocks = (int)std::min<int64_t>((words + 255) / 256, 148);
-    k_request_prologue<<<blocks, 256, 0, st>>>(z0, z1, z2, stage_host_, omega_.as<double>(), n_om);
+    PrologueCopy cp{stage_host_, omega_.as<double>(), obs_.as<double>(), nrm_.as<double>(),
+                    omega_staged_, obs_staged_, nrm_staged_};
+    PrologueRect pr{};
+    if (rect_pending_) {
+      const RectSurface& q = *rect_pending_;
+      const Vec3 v[4] = {q.start, q.v1, q.v2, q.normal};
+      double* d[4] = {pr.start, pr.v1, pr.v2, pr.normal};
+      for (int i = 0; i < 4; ++i) {
+        d[i][0] = v[i].x;
+        d[i][1] = v[i].y;
+        d[i][2] = v[i].z;
+      }
+      pr.n = (int64_t)q.nx1 * q.nx2;
+      pr.nx2 = q.nx2;
+      pr.obs = obs_.as<double>();
+      pr.nrm = rq.power_density ? nrm_.as<double>() : nullptr;
+      rect_pending_ = nullptr;
+    }
+    const int64_t words = std::max({z0.words, z1.words, z2.words, cp.n_om, cp.n_obs, pr.n});
+    const int blocks = (int)std::min<int64_t>((words + 255) / 256, 296);
+    k_request_prologue<<<blocks, 256, 0, st>>>(z0, z1, z2, cp, pr);
     check(cudaGetLastError(), "request prologue");
     ++last_launches;
-    if (n_om > 0) {  // the staging buffer is free again once the prologue has run
+    if (cp.n_om + cp.n_obs + cp.n_nrm > 0) {  // the staging buffer is free again once the prologue has run
       check(cudaEventRecord(stage_ev_, st), "event");
-      omega_staged_ = 0;
+      omega_staged_ = obs_staged_ = nrm_staged_ = 0;
     }
   }
   prefill(mixed, Lfirst, Lpre, true);
 
   const double* d_obs = req_obs_;
-  const double* d_nrm = rq.normals ? req_nrm_ : nullptr;
+  const double* d_nrm = req_nrm_;
   double pol[6];
   bool project = false;
   double c0 = 0, c2 = 0, scale = 0;
@@ -670,6 +713,13 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
     cur_list ^= 1;
   };
   for (int L = Lfirst; L <= Lpre; ++L) launch_wave(L);
+  // the caller's own host work, while the device computes
+  auto overlap = [&]() {
+    if (tuning_ || !rq.meanwhile) return;
+    const std::function<void()> work = std::move(const_cast<RadRequest&>(rq).meanwhile);
+    const_cast<RadRequest&>(rq).meanwhile = nullptr;
+    work();
+  };
   bool finished = false;  // statistics (and result downloads) already enqueued behind the last wave
   for (int L = Lpre + 1; L <= lstop; ++L) {  // beyond the prefilled levels the host decides
     // a one-thread kernel writes the active count and the highest finished level into mapped host
@@ -680,24 +730,31 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
     // outputs go in behind it, before the host knows whether this was the last wave; if it was not,
     // both are superseded by those the request ends with
     const bool speculate = !tuning_;
+    const bool small = speculate && tail_.active && tail_.small;
     const int slot = speculate ? claim_stat_slot() : -1;
     const unsigned seq = report_launch(active, level_max, st, speculate ? c64 : nullptr,
-                                       speculate ? stats_host_ + kStatWords * slot : nullptr);
-    if (speculate) finish_request(slot, st);
+                                       speculate ? stats_host_ + kStatWords * slot : nullptr, small);
+    if (speculate && !small) finish_request(slot, st);
+    overlap();
     report_wait(seq, &nn, &lmax, st);
     if (nn == 0) {
       if (!tuning_) prefill_hist_[hist_key] = std::max<int>(Lfirst, (int)lmax);
       finished = speculate;
+      if (small) {  // results and statistics are in mapped memory: no copies, no event
+        std::memcpy(tail_.h_out, tail_host_, sizeof(double) * tail_.n);
+        if (tail_.h_lvl) std::memcpy(tail_.h_lvl, tail_host_ + kTailEntries, sizeof(int32_t) * tail_.n);
+        tail_.emitted = tail_.done = true;
+        take_stats(slot);
+      }
       break;
     }
-    if (speculate) {
-      pending_.pop_back();
-      tail_.emitted = false;
-    }
+    if (speculate && !small) pending_.pop_back();
+    tail_.emitted = false;
     if (mixed) ensure_mixed(L);
     else ensure_levels(L);
     launch_wave(L);
   }
+  overlap();
   join_prefill();
   wait_inputs(st);  // no upload into the request's buffers stays in flight past the request
   if (!finished) {
@@ -721,11 +778,46 @@ void Engine::finish_request(int slot, cudaStream_t st) {
   check(cudaEventRecord(stats_ev_[slot], st), "event");
   pending_.push_back(slot);
   if (!tail_.active || tuning_) return;
-  check(cudaMemcpyAsync(tail_.h_out, tail_.d_out, sizeof(double) * tail_.n, cudaMemcpyDeviceToHost, st), "download");
+  void* h_out = tail_.bounce ? (void*)bounce_ : (void*)tail_.h_out;
+  void* h_lvl = tail_.bounce ? (void*)(bounce_ + sizeof(double) * tail_.n) : (void*)tail_.h_lvl;
+  check(cudaMemcpyAsync(h_out, tail_.d_out, sizeof(double) * tail_.n, cudaMemcpyDeviceToHost, st), "download");
   if (tail_.h_lvl)
-    check(cudaMemcpyAsync(tail_.h_lvl, tail_.d_lvl, sizeof(int32_t) * tail_.n, cudaMemcpyDeviceToHost, st),
-          "download");
+    check(cudaMemcpyAsync(h_lvl, tail_.d_lvl, sizeof(int32_t) * tail_.n, cudaMemcpyDeviceToHost, st), "download");
   tail_.emitted = true;
+}
+
+// Whether downloads into `p` go through bounce_ (pageable memory: the driver would stage them in small
+// pieces while the host waits), growing it to `bytes`; larger results keep the driver's path.
+bool Engine::reserve_bounce(const void* p, size_t bytes) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (at.type != cudaMemoryTypeUnregistered || bytes > kBounceBytes) return false;
+  if (bounce_bytes_ < bytes) {
+    if (bounce_) cudaFreeHost(bounce_);
+    bounce_ = nullptr;
+    bounce_bytes_ = 0;
+    const size_t want = std::min(kBounceBytes, std::max(2 * bytes, (size_t)1 << 20));
+    if (cudaHostAlloc(reinterpret_cast<void**>(&bounce_), want, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      bounce_ = nullptr;
+      return false;
+    }
+    bounce_bytes_ = want;
+  }
+  return true;
+}
+
+// Adds the statistics in ring slot `slot` to the request's; returns its error word.
+unsigned Engine::take_stats(int slot) {
+  const volatile unsigned long long* w = stats_host_ + kStatWords * slot;
+  last_not_converged += (long long)w[0];
+  last_samples += (long long)w[1];
+  if (profiling) prof_samples += (long long)w[1];
+  early_err_ |= (unsigned)w[2];
+  return (unsigned)w[2];
 }
 
 void Engine::wait_inputs(cudaStream_t st) {
@@ -740,16 +832,14 @@ void Engine::collect() {
   // the error word rides in the slots (the last one has every earlier error: the word is sticky);
   // with no slot pending it is read directly
   unsigned err = 0;
-  const bool direct = pending_.empty();
+  const bool direct = pending_.empty() && !tail_.done;
   for (int slot : pending_) {
     check(cudaEventSynchronize(stats_ev_[slot]), "radiation");
-    const volatile unsigned long long* w = stats_host_ + kStatWords * slot;
-    last_not_converged += (long long)w[0];
-    last_samples += (long long)w[1];
-    err |= (unsigned)w[2];
-    if (profiling) prof_samples += (long long)w[1];
+    take_stats(slot);
   }
   pending_.clear();
+  err = early_err_;
+  early_err_ = 0;
   if (profiling) collect_timings();
   if (direct) check(cudaMemcpy(&err, cnt_.as<unsigned>() + kCntErr, sizeof err, cudaMemcpyDeviceToHost), "error word");
   if (err) {
@@ -898,9 +988,22 @@ class TrajectoryPipeline {
   bool stop_ = false;
 };
 
-__global__ void k_report_counts(const unsigned* __restrict__ a, const unsigned* __restrict__ b,
-                                volatile unsigned* host, unsigned seq, const unsigned long long* __restrict__ c64,
-                                const unsigned* __restrict__ err, volatile unsigned long long* slot) {
+// n > 0: the results too (n values and levels), before the sequence number.
+__global__ void __launch_bounds__(1024) k_report_counts(const unsigned* __restrict__ a, const unsigned* __restrict__ b,
+                                                        volatile unsigned* host, unsigned seq,
+                                                        const unsigned long long* __restrict__ c64,
+                                                        const unsigned* __restrict__ err,
+                                                        volatile unsigned long long* slot, int n,
+                                                        const double* __restrict__ out, const int* __restrict__ lvl,
+                                                        double* h_out, int* h_lvl) {
+  dev::wait_predecessor();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) h_out[i] = out[i];
+  for (int i = threadIdx.x; i < n; i += blockDim.x) h_lvl[i] = lvl[i];
+  if (n > 0) {
+    __threadfence_system();
+    __syncthreads();
+  }
+  if (threadIdx.x != 0) return;
   if (slot) k_stats_store(c64, err, slot);
   host[1] = *a;
   host[2] = *b;
@@ -917,10 +1020,13 @@ void Engine::report_counts(const unsigned* a, const unsigned* b, unsigned* va, u
 }
 
 unsigned Engine::report_launch(const unsigned* a, const unsigned* b, cudaStream_t st, const unsigned long long* c64,
-                               unsigned long long* slot) {
+                               unsigned long long* slot, bool results) {
   const unsigned seq = ++report_seq_;
-  k_report_counts<<<1, 1, 0, st>>>(a, b, ctl_host_, seq, c64, cnt_.as<unsigned>() + kCntErr, slot);
-  check(cudaGetLastError(), "count");
+  const int n = results ? (int)tail_.n : 0;
+  check(launch_overlapped(k_report_counts, 1, n > 0 ? 1024 : 1, st, a, b, ctl_host_, seq, c64,
+                          cnt_.as<unsigned>() + kCntErr, slot, n, tail_.d_out, tail_.d_lvl, tail_host_,
+                          reinterpret_cast<int*>(tail_host_ + kTailEntries)),
+        "count");
   ++last_launches;
   return seq;
 }
@@ -960,9 +1066,30 @@ void Engine::radiation(RadRequest& rq) {
   // slower than the upload it saves.)  Up to kStageDoubles frequencies are staged in mapped
   // page-locked memory for the request prologue to copy; more go up directly.
   const int np = rq.opts.nparticles;
+  omega_staged_ = obs_staged_ = nrm_staged_ = 0;
+  rect_pending_ = nullptr;
+  early_err_ = 0;
+  const int64_t n_stage = (rq.power_density ? 0 : n_e) + 3 * rq.n_obs * (rq.normals ? 2 : 1);
   if (rq.obs_on_device) {
     req_obs_ = rq.obs;
     req_nrm_ = rq.normals;
+  } else if (rq.rect || n_stage <= kStageDoubles) {
+    // a rectangle's points are formed by the prologue, a few observers staged for it to copy: no upload
+    obs_.reserve(sizeof(double) * 3 * rq.n_obs);
+    if (rq.rect ? rq.power_density : rq.normals != nullptr) nrm_.reserve(sizeof(double) * 3 * rq.n_obs);
+    rect_pending_ = rq.rect;
+    req_obs_ = obs_.as<double>();
+    req_nrm_ = (rq.rect ? rq.power_density : rq.normals != nullptr) ? nrm_.as<double>() : nullptr;
+    if (!rq.rect) {
+      check(cudaEventSynchronize(stage_ev_), "stage");
+      double* q = stage_host_ + (rq.power_density ? 0 : n_e);
+      std::memcpy(q, rq.obs, sizeof(double) * 3 * rq.n_obs);
+      obs_staged_ = 3 * rq.n_obs;
+      if (rq.normals) {
+        std::memcpy(q + obs_staged_, rq.normals, sizeof(double) * 3 * rq.n_obs);
+        nrm_staged_ = 3 * rq.n_obs;
+      }
+    }
   } else {
     check(cudaEventRecord(in_fork_ev_, st), "event");
     check(cudaStreamWaitEvent(copy_, in_fork_ev_, 0), "stream wait");
@@ -978,7 +1105,6 @@ void Engine::radiation(RadRequest& rq) {
     req_obs_ = obs_.as<double>();
     req_nrm_ = rq.normals ? nrm_.as<double>() : nullptr;
   }
-  omega_staged_ = 0;
   if (!rq.power_density) {
     omega_.reserve(sizeof(double) * n_e);
     if (n_e <= kStageDoubles) {
@@ -1015,7 +1141,16 @@ void Engine::radiation(RadRequest& rq) {
     model.ensure_trajectory();
     upload_trajectory();
     tail_ = ResultTail{};
-    if (!rq.out_on_device) tail_ = ResultTail{true, false, d_out, d_lvl, rq.out, rq.level_out, N};
+    if (!rq.out_on_device) {
+      tail_.active = true;
+      tail_.d_out = d_out;
+      tail_.d_lvl = d_lvl;
+      tail_.h_out = rq.out;
+      tail_.h_lvl = rq.level_out;
+      tail_.n = N;
+      tail_.small = N <= kTailEntries;
+      tail_.bounce = !tail_.small && reserve_bounce(rq.out, (size_t)N * (sizeof(double) + sizeof(int32_t)));
+    }
     try {
       run_single(rq, N, 1.0, d_out, d_lvl, st);
     } catch (...) {
@@ -1066,9 +1201,15 @@ void Engine::radiation(RadRequest& rq) {
       if (rq.level_out)
         check(cudaMemcpyAsync(rq.level_out, d_lvl, sizeof(int32_t) * N, cudaMemcpyDeviceToHost, st), "download");
     }
-    tail_ = ResultTail{};
-    check(cudaStreamSynchronize(st), "download");
+    if (!tail_.done) {
+      check(cudaStreamSynchronize(st), "download");
+      if (tail_.emitted && tail_.bounce) {
+        std::memcpy(rq.out, bounce_, sizeof(double) * N);
+        if (rq.level_out) std::memcpy(rq.level_out, bounce_ + sizeof(double) * N, sizeof(int32_t) * N);
+      }
+    }
     collect();
+    tail_ = ResultTail{};
   }
 }
 
@@ -1080,7 +1221,12 @@ void Engine::radiation_beam_mixed(RadRequest& rq, int64_t N) {
   const int64_t n_e = (int64_t)rq.omega.size();
   std::vector<double> obs_h;
   const double* obs = rq.obs;
-  if (rq.obs_on_device) {
+  if (rq.meanwhile) rq.meanwhile();
+  if (rq.rect) {
+    obs_h.resize(3 * rq.n_obs);
+    rectangle_points(*rq.rect, obs_h.data(), nullptr, nullptr);
+    obs = obs_h.data();
+  } else if (rq.obs_on_device) {
     obs_h.resize(3 * rq.n_obs);
     check(cudaMemcpy(obs_h.data(), rq.obs, sizeof(double) * 3 * rq.n_obs, cudaMemcpyDeviceToHost), "observers");
     obs = obs_h.data();

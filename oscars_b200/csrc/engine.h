@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <map>
 #include <tuple>
@@ -37,6 +38,8 @@ struct RadRequest {
   bool power_density = false;
   const double* obs = nullptr;      // 3*n_obs
   const double* normals = nullptr;  // 3*n_obs or NULL
+  const RectSurface* rect = nullptr;  // observers (and normals) of a rectangle, formed on the device instead
+  std::function<void()> meanwhile;    // host work of the caller, run once while the device computes
   int64_t n_obs = 0;
   std::vector<double> omega;        // n_e angular frequencies
   bool obs_on_device = false;
@@ -160,6 +163,14 @@ class Engine {
   static constexpr int kStatWords = 4;
   unsigned long long* stats_host_ = nullptr;
   double* stage_host_ = nullptr;
+  // results of requests of up to kTailEntries entries, stored by the report kernel; larger ones are
+  // downloaded through bounce_ when the caller's buffers are pageable
+  static constexpr int64_t kTailEntries = 8192;
+  static constexpr size_t kBounceBytes = (size_t)64 << 20;
+  double* tail_host_ = nullptr;
+  unsigned char* mapped_ = nullptr;  // one page-locked block: stats, stage, control words, tail
+  unsigned char* bounce_ = nullptr;
+  size_t bounce_bytes_ = 0;
   // Device counter block cnt_ (16 words): [0], [1] survivor-list counts, [4..9] three 64-bit counters
   // (not converged, samples, unit counter of the running wave), [12] highest finished level -- all
   // zeroed by one memset of words 0..12 per request -- and [kCntErr] the sticky error word.
@@ -173,7 +184,7 @@ class Engine {
   // its sequence number; with `slot`, the kernel also stores the request's statistics there (c64[0..1]
   // and the error word)
   unsigned report_launch(const unsigned* a, const unsigned* b, cudaStream_t st, const unsigned long long* c64 = nullptr,
-                         unsigned long long* slot = nullptr);
+                         unsigned long long* slot = nullptr, bool results = false);
   void report_wait(unsigned seq, unsigned* va, unsigned* vb, cudaStream_t st);
   static constexpr int kStatSlots = 64;
   cudaEvent_t stats_ev_[kStatSlots] = {};
@@ -272,6 +283,8 @@ class Engine {
   const double* req_nrm_ = nullptr;
   // frequencies staged in mapped page-locked memory (stage_host_) for the request prologue to copy
   int64_t omega_staged_ = 0;
+  int64_t obs_staged_ = 0, nrm_staged_ = 0;  // observer / normal doubles staged behind the frequencies
+  const RectSurface* rect_pending_ = nullptr;  // rectangle the next prologue forms
   void wait_inputs(cudaStream_t st);
   // Result downloads of a single-particle request with host outputs, enqueued by run_single right
   // behind its statistics -- ahead of the host's last poll, so the copies need no extra round trip.
@@ -282,9 +295,15 @@ class Engine {
     double* h_out = nullptr;
     int32_t* h_lvl = nullptr;
     int64_t n = 0;
+    bool small = false;  // the report kernel stores the results into tail_host_
+    bool done = false;   // they are in the caller's buffers
+    bool bounce = false; // the downloads go to page-locked memory first
   } tail_;
   int claim_stat_slot();
   void finish_request(int slot, cudaStream_t st);
+  bool reserve_bounce(const void* p, size_t bytes);
+  unsigned take_stats(int slot);
+  unsigned early_err_ = 0;  // error words of statistics taken without their event
   void run_single(const RadRequest& rq, int64_t n_items, double weight, double* d_out, int32_t* d_lvl,
                   cudaStream_t st);
   void check(cudaError_t e, const char* what);

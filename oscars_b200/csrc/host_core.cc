@@ -994,8 +994,8 @@ void spline_second_derivatives(Knots& k, bool threads) {
 // ---------------------------------------------------------------------------------------------
 // Rectangle surface (src/TSurfacePoints_Rectangle.cc:140-315)
 // ---------------------------------------------------------------------------------------------
-void surface_rectangle(const std::string& plane_in, int nx1, int nx2, double w1, double w2, Vec3 rot,
-                       Vec3 trans, int normal, double* xyz, double* normals, double* x1x2) {
+RectSurface rectangle_layout(const std::string& plane_in, int nx1, int nx2, double w1, double w2, Vec3 rot, Vec3 trans,
+                             int normal) {
   std::string P = plane_in;
   std::transform(P.begin(), P.end(), P.begin(), ::toupper);
   const double s1 = nx1 > 1 ? w1 / (nx1 - 1) : 0;
@@ -1017,21 +1017,33 @@ void surface_rectangle(const std::string& plane_in, int nx1, int nx2, double w1,
   Vec3 nv = rotate_xyz(L.n, rot);
   if (normal == -1) nv = nv * -1;
   else if (normal != 0 && normal != 1) throw Error{OSC_ERR_INVALID, "normal must be -1, 0, or 1"};
-  const double m1 = mag(v1), m2 = mag(v2);
-  const int64_t n = (int64_t)nx1 * nx2;
-  for (int64_t i = 0; i < n; ++i) {
-    const int ix1 = (int)(i / nx2), ix2 = (int)(i % nx2);
-    if (xyz) {
-      const Vec3 p = (st + v1 * (double)ix1) + v2 * (double)ix2;
-      xyz[3 * i] = p.x; xyz[3 * i + 1] = p.y; xyz[3 * i + 2] = p.z;
-    }
-    if (normals) { normals[3 * i] = nv.x; normals[3 * i + 1] = nv.y; normals[3 * i + 2] = nv.z; }
-    if (x1x2) {
-      x1x2[3 * i] = s1 * ix1 - m1 * (nx1 - 1) / 2.;
-      x1x2[3 * i + 1] = s2 * ix2 - m2 * (nx2 - 1) / 2.;
-      x1x2[3 * i + 2] = 0;
+  return {nx1, nx2, st, v1, v2, nv, s1, s2, mag(v1), mag(v2)};
+}
+
+void rectangle_points(const RectSurface& r, double* xyz, double* normals, double* x1x2) {
+  for (int ix1 = 0; ix1 < r.nx1; ++ix1) {
+    const int64_t row = 3 * (int64_t)ix1 * r.nx2;
+    const Vec3 a = r.start + r.v1 * (double)ix1;
+    const double c1 = r.s1 * ix1 - r.m1 * (r.nx1 - 1) / 2.;
+    for (int ix2 = 0; ix2 < r.nx2; ++ix2) {
+      const int64_t i = row + 3 * ix2;
+      if (xyz) {
+        const Vec3 p = a + r.v2 * (double)ix2;
+        xyz[i] = p.x; xyz[i + 1] = p.y; xyz[i + 2] = p.z;
+      }
+      if (normals) { normals[i] = r.normal.x; normals[i + 1] = r.normal.y; normals[i + 2] = r.normal.z; }
+      if (x1x2) {
+        x1x2[i] = c1;
+        x1x2[i + 1] = r.s2 * ix2 - r.m2 * (r.nx2 - 1) / 2.;
+        x1x2[i + 2] = 0;
+      }
     }
   }
+}
+
+void surface_rectangle(const std::string& plane, int nx1, int nx2, double w1, double w2, Vec3 rot, Vec3 trans, int normal,
+                       double* xyz, double* normals, double* x1x2) {
+  rectangle_points(rectangle_layout(plane, nx1, nx2, w1, w2, rot, trans, normal), xyz, normals, x1x2);
 }
 
 // Rectangle from three points (TSurfacePoints_Rectangle::Init(NX1, NX2, X0, X1, X2, Normal) and

@@ -200,6 +200,16 @@ void spline_second_derivatives(Knots& k, bool threads = true);
 void parallel_tasks(int n, const std::function<void(int)>& fn);
 
 // Rectangle surface (TSurfacePoints_Rectangle).  Throws osc::Error.
+// A rectangle's points: start + v1 ix1 + v2 ix2 (ix2 fastest), the in-plane steps and their magnitudes,
+// and the common normal.
+struct RectSurface {
+  int nx1, nx2;
+  Vec3 start, v1, v2, normal;
+  double s1, s2, m1, m2;
+};
+RectSurface rectangle_layout(const std::string& plane, int nx1, int nx2, double w1, double w2, Vec3 rot, Vec3 trans,
+                             int normal);
+void rectangle_points(const RectSurface& r, double* xyz, double* normals, double* x1x2);  // any may be NULL
 void surface_rectangle(const std::string& plane, int nx1, int nx2, double w1, double w2, Vec3 rot,
                        Vec3 trans, int normal, double* xyz, double* normals, double* x1x2);
 // Rectangle from three points (TSurfacePoints_Rectangle x0x1x2 form).  Throws osc::Error.

@@ -437,7 +437,13 @@ class sr:
         if energy_points_eV is not None:
             if len(energy_points_eV) == 0:
                 raise ValueError("Number of points to calculate is zero.  Check input.")
-            return np.array([float(e) for e in energy_points_eV])
+            try:
+                e = np.array(energy_points_eV, dtype=np.float64)
+                if e.ndim == 1 and not np.isnan(e).any():
+                    return e
+            except (TypeError, ValueError):
+                pass
+            return np.array([float(e) for e in energy_points_eV])  # nested, None and the like, point by point
         e0 = e1 = 0.0
         if energy_range_eV is not None:
             if len(energy_range_eV) != 2:
@@ -479,6 +485,18 @@ class sr:
         return [[float(E[i]), float(out[i])] for i in range(E.size)]
 
     def _rectangle(self, npoints, plane, width, x0x1x2, rotations, translation, normal, pd):
+        """(xyz, normals, in-plane coordinates) of a rectangle's points, 3 values each."""
+        a = self._rectangle_args(npoints, plane, width, x0x1x2, rotations, translation, normal, pd)
+        n = a[1] * a[2]
+        xyz, nrm, x12 = np.zeros(3 * n), np.zeros(3 * n), np.zeros(3 * n)
+        f = _lib.lib().osc_surface_rectangle if x0x1x2 is None else _lib.lib().osc_surface_x0x1x2
+        if f(*(a if x0x1x2 is None else a[1:]), dptr(xyz), dptr(nrm), dptr(x12)) != 0:
+            raise ValueError(_lib.lib().osc_last_error(None).decode())
+        return xyz, nrm, x12
+
+    def _rectangle_args(self, npoints, plane, width, x0x1x2, rotations, translation, normal, pd):
+        """Checked arguments of a rectangle: (plane, nx1, nx2, w1, w2, rotations, translation, normal), or with
+        x0x1x2 (None, nx1, nx2, points, rotations, translation, normal), arrays as pointers."""
         if len(npoints) != 2:
             raise ValueError("'npoints' must be [int, int]")
         nx1, nx2 = int(npoints[0]), int(npoints[1])
@@ -491,25 +509,46 @@ class sr:
             w1, w2 = float(width[0]), float(width[1])
         if abs(normal) > 1:
             raise ValueError("'normal' must be -1, 0, or 1")
-        n = nx1 * nx2
         if x0x1x2 is not None:  # the three-point form (src/OSCARSSR_Python.cc:6633-6658, 8146-8172)
             if len(x0x1x2) != 3:
                 raise ValueError("'x0x1x2' must have 3 XYZ points defined correctly")
             pts = np.array([_vec3(p, "x0x1x2") for p in x0x1x2], dtype=np.float64).ravel()
-            xyz, nrm, x12 = np.zeros(3 * n), np.zeros(3 * n), np.zeros(3 * n)
-            rc = _lib.lib().osc_surface_x0x1x2(nx1, nx2, dptr(pts), dptr(r), dptr(t), int(normal), dptr(xyz), dptr(nrm),
-                                               dptr(x12))
-            if rc != 0:
+            form = dptr(pts), dptr(r), dptr(t), int(normal)
+            if _lib.lib().osc_surface_x0x1x2(min(nx1, 2), min(nx2, 2), *form, None, None, None):
                 raise ValueError(_lib.lib().osc_last_error(None).decode())
-            return xyz, nrm, x12
+            return (None, nx1, nx2) + form
         if w1 <= 0 or w2 <= 0:
             raise ValueError("'width' must be > 0" if pd else "'width' must be given as [w1, w2] with both > 0")
-        xyz, nrm, x12 = np.zeros(3 * n), np.zeros(3 * n), np.zeros(3 * n)
-        rc = _lib.lib().osc_surface_rectangle(plane.encode(), nx1, nx2, w1, w2, dptr(r), dptr(t), int(normal),
-                                              dptr(xyz), dptr(nrm), dptr(x12))
-        if rc != 0:
+        # one point's worth of work checks the plane and the normal
+        if _lib.lib().osc_surface_rectangle(plane.encode(), 1, 1, w1, w2, dptr(r), dptr(t), int(normal), None, None, None):
             raise ValueError(_lib.lib().osc_last_error(None).decode())
-        return xyz, nrm, x12
+        return plane.encode(), nx1, nx2, w1, w2, dptr(r), dptr(t), int(normal)
+
+    def _rectangle_run(self, args, x0x1x2, dim, kind, what, o):
+        """Positions and values of a rectangle request: kind 'flux' (what = the energy) or 'power_density'
+        (what = directional).  The library forms a rectangle's observers itself and fills the positions while
+        the device computes; the three-point form uploads them."""
+        n = args[1] * args[2]
+        nnc = ctypes.c_longlong()
+        out = np.empty(n)
+        lv = np.empty(n, dtype=np.int32)
+        if x0x1x2 is None:
+            pos = np.empty(3 * n)
+            self._ctx.call("osc_%s_rectangle" % kind, *args, what, ctypes.byref(o), dptr(pos) if dim == 3 else None,
+                           None if dim == 3 else dptr(pos), dptr(out), i32ptr(lv), ctypes.byref(nnc))
+        else:
+            xyz, nrm, x12 = np.empty(3 * n), np.empty(3 * n), np.empty(3 * n)
+            if _lib.lib().osc_surface_x0x1x2(*args[1:], dptr(xyz), dptr(nrm), dptr(x12)) != 0:
+                raise ValueError(_lib.lib().osc_last_error(None).decode())
+            pos = xyz if dim == 3 else x12
+            if kind == "flux":
+                self._ctx.call("osc_flux", dptr(xyz), n, what, ctypes.byref(o), dptr(out), i32ptr(lv), ctypes.byref(nnc))
+            else:
+                self._ctx.call("osc_power_density", dptr(xyz), dptr(nrm), n, what, ctypes.byref(o), dptr(out), i32ptr(lv),
+                               ctypes.byref(nnc))
+        self.last_levels = lv
+        self._report(nnc)
+        return pos, out
 
     @staticmethod
     def _write_points(ofile, bofile, pos, out, dim):
@@ -614,22 +653,16 @@ class sr:
             raise ValueError("No particle beam defined")
         if dim not in (2, 3):
             raise ValueError("'dim' must be 2 or 3")
-        xyz, nrm, x12 = self._rectangle(npoints, plane, width, x0x1x2, rotations, translation, normal, False)
+        args = self._rectangle_args(npoints, plane, width, x0x1x2, rotations, translation, normal, False)
         if nparticles < 0:
             raise ValueError("'nparticles' must be >= 1 (sort of)")
         self._check_gpu(gpu, nthreads)
         q = _quantity(quantity)
         o = self._opts(polarization, angle, horizontal_direction, propogation_direction, precision, max_level,
                        max_level_extended, nparticles, q, compute, shard)
-        n = xyz.size // 3
-        out = np.zeros(n)
-        lv = np.zeros(n, dtype=np.int32)
-        nnc = ctypes.c_longlong()
-        self._ctx.call("osc_flux", dptr(xyz), n, float(energy_eV), ctypes.byref(o), dptr(out), i32ptr(lv), ctypes.byref(nnc))
-        self.last_levels = lv
-        self._report(nnc)
-        self._write_points(ofile, bofile, xyz if dim == 3 else x12, out, dim)
-        return self._points_result(xyz if dim == 3 else x12, out, return_numpy)
+        pos, out = self._rectangle_run(args, x0x1x2, dim, "flux", float(energy_eV), o)
+        self._write_points(ofile, bofile, pos, out, dim)
+        return self._points_result(pos, out, return_numpy)
 
     def calculate_power_density_rectangle(self, npoints=[51, 51], plane="XY", width=None, x0x1x2=None,
                                           rotations=None, translation=None, ofile="", bofile="", normal=0,
@@ -640,23 +673,16 @@ class sr:
             raise ValueError("No particle beam defined")
         if dim not in (2, 3):
             raise ValueError("'dim' must be 2 or 3")
-        xyz, nrm, x12 = self._rectangle(npoints, plane, width, x0x1x2, rotations, translation, normal, True)
+        args = self._rectangle_args(npoints, plane, width, x0x1x2, rotations, translation, normal, True)
         if nparticles < 0:
             raise ValueError("'nparticles' must be >= 1 (sort of)")
         self._check_gpu(gpu, nthreads)
         q = _quantity(quantity, pd=True)
         o = self._opts("", _ANGLE_UNSET, None, None, precision, max_level, max_level_extended, nparticles, q, compute,
                        shard)
-        n = xyz.size // 3
-        out = np.zeros(n)
-        lv = np.zeros(n, dtype=np.int32)
-        nnc = ctypes.c_longlong()
-        self._ctx.call("osc_power_density", dptr(xyz), dptr(nrm), n, int(normal != 0), ctypes.byref(o), dptr(out),
-                       i32ptr(lv), ctypes.byref(nnc))
-        self.last_levels = lv
-        self._report(nnc)
-        self._write_points(ofile, bofile, xyz if dim == 3 else x12, out, dim)
-        return self._points_result(xyz if dim == 3 else x12, out, return_numpy)
+        pos, out = self._rectangle_run(args, x0x1x2, dim, "power_density", int(normal != 0), o)
+        self._write_points(ofile, bofile, pos, out, dim)
+        return self._points_result(pos, out, return_numpy)
 
     # ---- STL surfaces (src/OSCARSSR_Python.cc:6852-7280, 9262-9276) ----------------------------------
     def add_stl(self, ifile, rotations=None, translation=None, scale=1, name=""):

@@ -67,3 +67,29 @@ def test_fp64_power_density_tiles_and_levels(nx, ny, normal, plane, level):
     kw = dict(npoints=[nx, ny], plane=plane, width=[0.02, 0.03], normal=normal, translation=[0, 0.01, 20], max_level=level)
     got, want = _both("calculate_power_density_rectangle", kw)
     assert np.max(np.abs(got - want)) <= 1e-12 * max(np.max(np.abs(want)), 1e-300)
+
+
+# A rectangle formed on the device against the same points uploaded: small (staged inputs, results stored by the
+# report kernel up to 8192 entries) and larger ones (downloads through page-locked memory).  Same bits.
+@pytest.mark.parametrize("nx, ny", [(1, 1), (7, 5), (64, 128), (91, 91)])
+@pytest.mark.parametrize("power", [False, True])
+def test_rectangle_formed_on_device_matches_uploaded_points(nx, ny, power):
+    import ctypes
+    from oscars_b200._lib import dptr, i32ptr
+    s = sr(gpu=1)
+    run_case(s, UND_SHORT_SETUP)
+    geo = dict(npoints=[nx, ny], plane="ZY", width=[0.02, 0.03], rotations=[0.1, 1.4, -0.2], translation=[0.001, 0, 20])
+    common = dict(geo, dim=3, max_level=9, normal=1, return_numpy=True)
+    if power:
+        pos, got = s.calculate_power_density_rectangle(**common)
+    else:
+        pos, got = s.calculate_flux_rectangle(energy_eV=E1_U, **common)
+    levels = s.last_levels
+    xyz, nrm, _ = s._rectangle(geo["npoints"], geo["plane"], geo["width"], None, geo["rotations"], geo["translation"], 1, power)
+    want, lv, nnc = np.zeros(nx * ny), np.zeros(nx * ny, np.int32), ctypes.c_longlong()
+    o = s._opts("", 112188979912321.0, None, None, 0.01, 9, 0, 0, 0, "fp64")
+    if power:
+        s._ctx.call("osc_power_density", dptr(xyz), dptr(nrm), nx * ny, 1, ctypes.byref(o), dptr(want), i32ptr(lv), ctypes.byref(nnc))
+    else:
+        s._ctx.call("osc_flux", dptr(xyz), nx * ny, E1_U, ctypes.byref(o), dptr(want), i32ptr(lv), ctypes.byref(nnc))
+    assert np.array_equal(pos.ravel(), xyz) and np.array_equal(got, want) and np.array_equal(levels, lv)
