@@ -117,7 +117,7 @@ Engine::~Engine() {
                     &b_knots_, &b_work_, &b_rec_, &b_rec_ext_, &b_state_, &b_out_, &b_lvl_, &b_act_[0], &b_act_[1],
                     &b_part_, &b_plan_, &b_cnt_, &adj_, &adj_s_, &adj_r_, &adj_sums_, &adj_z_, &fused_, &stl_geo_,
                     &stl_cen_, &stl_nrm_,
-                    &stl_state_, &stl_flags_})
+                    &stl_state_})
     b->release();
   if (stream) cudaStreamDestroy(stream);
   if (aux_) cudaStreamDestroy(aux_);
@@ -409,6 +409,7 @@ int Engine::wave_grid(int kind, int variant) {
     check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "attr");
     const int per = kind == 2   ? mixed_blocks_per_sm(variant)
                     : kind == 4 ? pd_mixed_blocks_per_sm()
+                    : kind == 7 ? stl_blocks_per_sm()
                     : kind >= 5 ? lines_blocks_per_sm(kind == 6)
                                 : fp64_blocks_per_sm(kind == 1, variant);
     wave_grid_[kind][variant] = sms * per;
@@ -794,7 +795,12 @@ bool Engine::reserve_bounce(const void* p, size_t bytes) {
     cudaGetLastError();
     return false;
   }
-  if (at.type != cudaMemoryTypeUnregistered || bytes > kBounceBytes) return false;
+  return at.type == cudaMemoryTypeUnregistered && bounce_for(bytes) != nullptr;
+}
+
+// bounce_ with at least `bytes` (nothing may be in flight in it), NULL beyond kBounceBytes.
+unsigned char* Engine::bounce_for(size_t bytes) {
+  if (bytes > kBounceBytes) return nullptr;
   if (bounce_bytes_ < bytes) {
     if (bounce_) cudaFreeHost(bounce_);
     bounce_ = nullptr;
@@ -803,11 +809,11 @@ bool Engine::reserve_bounce(const void* p, size_t bytes) {
     if (cudaHostAlloc(reinterpret_cast<void**>(&bounce_), want, cudaHostAllocDefault) != cudaSuccess) {
       cudaGetLastError();
       bounce_ = nullptr;
-      return false;
+      return nullptr;
     }
     bounce_bytes_ = want;
   }
-  return true;
+  return bounce_;
 }
 
 // Adds the statistics in ring slot `slot` to the request's; returns its error word.

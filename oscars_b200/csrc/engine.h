@@ -193,7 +193,7 @@ class Engine {
   std::vector<int> pending_;
   // kernel variants: kind 0 = FP64 flux, 1 = FP64 power density, 2 = mixed flux, 3 = batched mixed,
   // 4 = mixed power density
-  int wave_grid_[7][16] = {};  // kinds: 0 fp64, 1 power density, 2 mixed, 4 mixed power density, 5 / 6 fp64 / mixed lines
+  int wave_grid_[8][16] = {};  // kinds: 0 fp64, 1 power density, 2 mixed, 4 mixed power density, 5 / 6 fp64 / mixed lines, 7 STL
   int wave_grid(int kind, int variant);
   std::map<std::tuple<int, int, int, int>, int> tuned_;   // (kind, log2 entries, first level, last level) -> variant
   // (kind, entries, energies, last level, precision) -> highest level the last such request needed
@@ -266,8 +266,9 @@ class Engine {
   void prefill(bool mixed, int Lhead, int Lpre, bool bd_zeroed = false);
   void join_prefill();
   std::vector<PinnedStage> pin_pool_;  // trajectory staging of multi-particle requests
-  // STL request buffers: facet geometry (A, B - A, C - A), centres, normals, per-facet state and flags
-  DevBuf stl_geo_, stl_cen_, stl_nrm_, stl_state_, stl_flags_;
+  // STL request buffers: facet geometry (A, B - A, C - A), facets and centres, normals and box, per-facet
+  // state, flags and level counters
+  DevBuf stl_geo_, stl_cen_, stl_nrm_, stl_state_;
   // side stream of the prefill (levels above the first wave's) and its fork / join events
   cudaStream_t aux_ = nullptr;
   cudaEvent_t fork_ev_ = nullptr, join_ev_ = nullptr;
@@ -302,6 +303,7 @@ class Engine {
   int claim_stat_slot();
   void finish_request(int slot, cudaStream_t st);
   bool reserve_bounce(const void* p, size_t bytes);
+  unsigned char* bounce_for(size_t bytes);
   unsigned take_stats(int slot);
   unsigned early_err_ = 0;  // error words of statistics taken without their event
   void run_single(const RadRequest& rq, int64_t n_items, double weight, double* d_out, int32_t* d_lvl,

@@ -113,6 +113,22 @@ __device__ __forceinline__ double one_minus_b2(double bx, double by, double bz) 
   return __dsub_rn(1.0, __dadd_rn(__dadd_rn(__dmul_rn(bx, bx), __dmul_rn(by, by)), __dmul_rn(bz, bz)));
 }
 
+// Power-density term without N1 . normal, for N1 = n and y = 1 / |O - X|.  1 - b.N1 rounds as the
+// reference's operations do (the difference is ill-conditioned); the well-conditioned rest is
+// |u (n.a) - a (n.u)|^2, u = n - b, the squared norm of the numerator, which lies across N1 and so
+// equals the sum of its squared projections on N2 and N3, times (1 / (1 - b.N1))^5 and y^2.
+__device__ __forceinline__ double pd_term(double nx, double ny, double nz, double y, double bx, double by, double bz,
+                                          double ax, double ay, double az) {
+  const double om =
+      __dsub_rn(1.0, __dadd_rn(__dadd_rn(__dmul_rn(bx, nx), __dmul_rn(by, ny)), __dmul_rn(bz, nz)));
+  const double ux = __dsub_rn(nx, bx), uy = __dsub_rn(ny, by), uz = __dsub_rn(nz, bz);
+  const double na = fma(nx, ax, fma(ny, ay, nz * az));
+  const double nu = fma(nx, ux, fma(ny, uy, nz * uz));
+  const double mx = fma(ux, na, -(ax * nu)), my = fma(uy, na, -(ay * nu)), mz = fma(uz, na, -(az * nu));
+  const double io = rcp_near(om), io2 = io * io;
+  return fma(mx, mx, fma(my, my, mz * mz)) * (io2 * io2 * io) * (y * y);
+}
+
 // Bound of |w (t + D/c)| over a trajectory: it starts at A.x_start, lasts A.t_len and its times lie
 // within A.t_abs of zero, and the particle is slower than light.
 __device__ __forceinline__ double phase_reach(const FdWaveArgs& A, double Ox, double Oy, double Oz, double mw) {

@@ -164,22 +164,36 @@ struct PdWaveArgs {
   PdFinalArgs fin;
 };
 
-// One level of the STL power density (kernels_stl.cu): one CTA per facet not yet done.
-struct StlLevelArgs {
+// One wave of the STL power density (kernels_stl.cu): the first holds levels 0..level of every facet, a
+// later one level `level` of the facets not yet done, in spans.
+constexpr int kStlPartials = 9;  // sum, largest beta step, whether anything was visible, first and last visible beta
+struct StlWaveArgs {
   const double* lev;        // FP64 level cache (10 arrays of cap doubles)
   int64_t cap;
+  const double* box;        // n_box bounding boxes (x y z minima, maxima) that hold the wave's samples
+  int n_box;
   const double* geometry;   // n x 9: vertex A, B - A, C - A of each facet
   const double* centers;    // n x 3: facet centres (the observation points)
   const double* normals;    // n x 3: stored facet normals
   int64_t n;
-  int level;
-  double dt_level, precision, two_over_gamma;
+  int first, level;
+  double dt_prev, dt_level, precision, two_over_gamma;
   double* state;            // n x 4: running sum, last level value, result precision, last level
   int* done;                // n: stopped
-  int* level_out;           // n: level at which the facet stopped (-1 set by the host beforehand)
-  unsigned* n_active;       // facets not stopped after this level (zeroed by the host per level)
+  int* level_out;           // n: level at which the facet stopped (-1 before)
+  unsigned* n_active;       // per level, the facets not stopped after it
+  int* act;                 // later waves: the facets not yet done, and their number
+  int* n_act;
+  double* part;             // later waves: kStlPartials per (facet, span), fewer than max(n, 8 x grid) of them
+  unsigned* spans_done;     // n: spans finished (zero between waves)
 };
-cudaError_t launch_stl_level(const StlLevelArgs& a, cudaStream_t st);
+int stl_box_blocks(int64_t samples);
+int stl_blocks_per_sm();
+// Before a wave: a.n_box boxes of the samples [s_begin, s_end), the list of facets left; with a.first the start
+// of a request: geometry, normals, states, flags and counters from the facets `tri` (n x 12).
+cudaError_t launch_stl_prepare(const StlWaveArgs& a, int64_t s_begin, int64_t s_end, const double* tri, double* geo,
+                               double* nrm, double* box, cudaStream_t st);
+cudaError_t launch_stl_wave(const StlWaveArgs& a, int grid, cudaStream_t st);
 
 // Frame of the mixed-precision path: origin x0 (particle start), rows of rot = e1, e2, e3 with e3 the
 // initial direction; xperp_max / z_max bound the trajectory in that frame; t_ref = t0 / c;

@@ -359,11 +359,8 @@ __global__ void k_fd_finalize(FdFinalArgs A) {
 // ---------------------------------------------------------------------------------------------
 // Power density (src/OSCARSSR.cc:2869-2922):
 //   sum += [(N1 x ((N1 - b) x a/c)) . Nk]^2 / (1 - b.N1)^5 / |O - X|^2 * (N1 . normal),  k = 2, 3
-// N1, N1 . normal and 1 - b.N1 round as the reference's operations do (the difference is
-// ill-conditioned, and the directional cut is a sign); the well-conditioned rest is
-// |u (N1.a) - a (N1.u)|^2, u = N1 - b, the squared norm of the numerator, which lies across N1 and so
-// equals the sum of its squared projections on N2 and N3, times the fifth power of 1 / (1 - b.N1) and
-// 1 / |O - X|^2.
+// The term is pd_term (fd_common.cuh); N1 . normal, whose sign is the directional cut, rounds as the
+// reference's operations do.
 // Sample-split and fused like the flux waves; 67 FP64 instructions per (entry, sample) (with the
 // library's square root and four divisions: ~130, a separate finalize launch and 128 entries per CTA).
 // ---------------------------------------------------------------------------------------------
@@ -373,26 +370,17 @@ constexpr int kPdSub = 4;                       // groups of a CTA
 constexpr int kPdTile = kPdThreads / kPdSub;    // entries per CTA
 
 template <bool NORMAL, bool DIRECTIONAL>
-__device__ __forceinline__ double pd_term(double X, double Y, double Z, double bx, double by, double bz, double ax,
-                                          double ay, double az, double Ox, double Oy, double Oz, double Nx, double Ny,
-                                          double Nz) {
+__device__ __forceinline__ double pd_sample(double X, double Y, double Z, double bx, double by, double bz, double ax,
+                                            double ay, double az, double Ox, double Oy, double Oz, double Nx, double Ny,
+                                            double Nz) {
   const double Rx = __dsub_rn(Ox, X), Ry = __dsub_rn(Oy, Y), Rz = __dsub_rn(Oz, Z);
   const double s = __dadd_rn(__dadd_rn(__dmul_rn(Rx, Rx), __dmul_rn(Ry, Ry)), __dmul_rn(Rz, Rz));
   const double y = rsqrt_near(s), D = sqrt_by(s, y);
   const double nx = quot_by(Rx, D, y), ny = quot_by(Ry, D, y), nz = quot_by(Rz, D, y);
-  const double om =
-      __dsub_rn(1.0, __dadd_rn(__dadd_rn(__dmul_rn(bx, nx), __dmul_rn(by, ny)), __dmul_rn(bz, nz)));
-  const double ux = __dsub_rn(nx, bx), uy = __dsub_rn(ny, by), uz = __dsub_rn(nz, bz);
-  const double na = fma(nx, ax, fma(ny, ay, nz * az));
-  const double nu = fma(nx, ux, fma(ny, uy, nz * uz));
-  const double mx = fma(ux, na, -(ax * nu)), my = fma(uy, na, -(ay * nu)), mz = fma(uz, na, -(az * nu));
-  const double io = rcp_near(om), io2 = io * io;
-  double t = fma(mx, mx, fma(my, my, mz * mz)) * (io2 * io2 * io) * (y * y);
-  if (NORMAL) {
-    const double n1dn = __dadd_rn(__dadd_rn(__dmul_rn(nx, Nx), __dmul_rn(ny, Ny)), __dmul_rn(nz, Nz));
-    t = DIRECTIONAL && n1dn <= 0 ? 0.0 : t * n1dn;
-  }
-  return t;
+  const double t = pd_term(nx, ny, nz, y, bx, by, bz, ax, ay, az);
+  if (!NORMAL) return t;
+  const double n1dn = __dadd_rn(__dadd_rn(__dmul_rn(nx, Nx), __dmul_rn(ny, Ny)), __dmul_rn(nz, Nz));
+  return DIRECTIONAL && n1dn <= 0 ? 0.0 : t * n1dn;
 }
 
 __global__ void __launch_bounds__(kPdThreads, 5) k_pd_wave_fp64(PdWaveArgs A) {
@@ -479,7 +467,7 @@ __global__ void __launch_bounds__(kPdThreads, 5) k_pd_wave_fp64(PdWaveArgs A) {
       auto add = [&](auto normal, auto directional) {
 #pragma unroll 2
         for (int j = j0; j < j1; ++j)
-          sum += pd_term<normal.value, directional.value>(
+          sum += pd_sample<normal.value, directional.value>(
               st.v[buf][0][j], st.v[buf][1][j], st.v[buf][2][j], st.v[buf][3][j], st.v[buf][4][j], st.v[buf][5][j],
               st.v[buf][6][j], st.v[buf][7][j], st.v[buf][8][j], Ox, Oy, Oz, Nx, Ny, Nz);
       };

@@ -1,5 +1,5 @@
 // stl.cu -- host side of the power density on STL facets (src/OSCARSSR.cc:3154-3521): the particle
-// loop, the per-level launches of k_stl_level (kernels_stl.cu) on the FP64 level cache, and the
+// loop, the launches of k_stl_wave (kernels_stl.cu) on the FP64 level cache, and the
 // per-facet results with the reference's bookkeeping.
 #include <cmath>
 #include <cstring>
@@ -26,36 +26,30 @@ void Engine::power_density_stl(const double* tri, const double* centers, int64_t
   if (n <= 0) return;
   set_level_grid(ext_from);
   for (int64_t i = 0; i < n; ++i) out[i] = 0;
-  // facet geometry as RayIntersectionDistance forms it: A, B - A, C - A (src/TTriangle3D.cc)
-  std::vector<double> geo(9 * n), nrm(3 * n);
-  for (int64_t i = 0; i < n; ++i) {
-    const double* t = tri + 12 * i;
-    for (int c = 0; c < 3; ++c) {
-      geo[9 * i + c] = t[c];
-      geo[9 * i + 3 + c] = t[3 + c] - t[c];
-      geo[9 * i + 6 + c] = t[6 + c] - t[c];
-      nrm[3 * i + c] = t[9 + c];
-    }
-  }
+  // facets and centres up in one copy from page-locked memory; states, flags and counters down in one
+  const size_t up = sizeof(double) * 15 * n, back = sizeof(double) * 4 * n + sizeof(int) * 2 * n + sizeof(unsigned) * 32;
   stl_geo_.reserve(sizeof(double) * 9 * n);
-  stl_cen_.reserve(sizeof(double) * 3 * n);
-  stl_nrm_.reserve(sizeof(double) * 3 * n);
-  stl_state_.reserve(sizeof(double) * 4 * n);
-  stl_flags_.reserve(sizeof(int) * 2 * n);
-  check(cudaMemcpyAsync(stl_geo_.p, geo.data(), sizeof(double) * 9 * n, cudaMemcpyHostToDevice, st), "facets");
-  check(cudaMemcpyAsync(stl_cen_.p, centers, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st), "facets");
-  check(cudaMemcpyAsync(stl_nrm_.p, nrm.data(), sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st), "facets");
-  unsigned* n_active = cnt_.as<unsigned>();  // word 0 of the request counters
-  std::vector<double> init(4 * n), state(4 * n);
-  for (int64_t i = 0; i < n; ++i) {  // sum 0, last level value -1, result precision -1, level 0
-    init[4 * i] = 0;
-    init[4 * i + 1] = -1;
-    init[4 * i + 2] = -1;
-    init[4 * i + 3] = 0;
+  stl_cen_.reserve(up);  // facets n x 12, then centres n x 3
+  const int grid = wave_grid(7, 0);
+  const int64_t n_part = std::max<int64_t>(n, 8 * (int64_t)grid) * kStlPartials;
+  // normals, boxes, span partials; list, its count, finished spans
+  stl_nrm_.reserve(sizeof(double) * (3 * n + 6 * 148 + n_part) + sizeof(int) * (2 * n + 1));
+  stl_state_.reserve(back);
+  std::vector<unsigned char> pageable;
+  unsigned char* host = bounce_for(std::max(up, back));
+  if (!host) {
+    pageable.resize(std::max(up, back));
+    host = pageable.data();
   }
-  std::vector<int32_t> flags(2 * n);
+  std::memcpy(host, tri, sizeof(double) * 12 * n);
+  std::memcpy(host + sizeof(double) * 12 * n, centers, sizeof(double) * 3 * n);
+  check(cudaMemcpyAsync(stl_cen_.p, host, up, cudaMemcpyHostToDevice, st), "facets");
+  double* d_state = stl_state_.as<double>();
+  int* d_flags = reinterpret_cast<int*>(d_state + 4 * n);
+  unsigned* d_active = reinterpret_cast<unsigned*>(d_flags + 2 * n);
   const int np = o.nparticles;
   const double weight = np > 0 ? 1.0 / (double)np : 1.0;
+  const int L1 = std::min(9, lstop);  // facets can stop from level 9 on
   for (int ip = 0; ip < (np > 0 ? np : 1); ++ip) {
     if (np > 0) {  // src/OSCARSSR.cc:3234-3240: a new random particle and its trajectory
       model.random_particle();
@@ -66,42 +60,56 @@ void Engine::power_density_stl(const double* tri, const double* centers, int64_t
     check(cudaStreamSynchronize(st), "particle");  // the previous particle's launches read the caches
     upload_trajectory();
     const Particle& P = model.particle;
-    check(cudaMemcpyAsync(stl_state_.p, init.data(), sizeof(double) * 4 * n, cudaMemcpyHostToDevice, st), "state");
-    check(cudaMemsetAsync(stl_flags_.p, 0, sizeof(int) * n, st), "memset");
-    check(cudaMemsetAsync(stl_flags_.as<int>() + n, 0xff, sizeof(int) * n, st), "memset");  // levels -1
-    StlLevelArgs a{};
+    StlWaveArgs a{};
     a.geometry = stl_geo_.as<double>();
-    a.centers = stl_cen_.as<double>();
+    a.centers = stl_cen_.as<double>() + 12 * n;
     a.normals = stl_nrm_.as<double>();
+    double* d_box = stl_nrm_.as<double>() + 3 * n;
+    a.box = d_box;
+    a.part = d_box + 6 * 148;
+    a.act = reinterpret_cast<int*>(a.part + n_part);
+    a.spans_done = reinterpret_cast<unsigned*>(a.act + n);
+    a.n_act = a.act + 2 * n;
     a.n = n;
     a.precision = o.precision;
     a.two_over_gamma = 2. / P.gamma;
-    a.state = stl_state_.as<double>();
-    a.done = stl_flags_.as<int>();
-    a.level_out = stl_flags_.as<int>() + n;
-    a.n_active = n_active;
-    int last_level = 0;
-    for (int L = 0; L <= lstop; ++L) {
-      ensure_levels(L);
+    a.state = d_state;
+    a.done = d_flags;
+    a.level_out = d_flags + n;
+    a.n_active = d_active;
+    // the first waves go out three at a time, deep ones (which need their level's samples filled) one by one,
+    // then the host looks at the counters
+    for (int L = L1; L <= lstop;) {
+      const int end = std::min(lstop, L + (L <= 12 ? 2 : 0));
+      ensure_levels(end);
       a.lev = lev_.as<double>();
       a.cap = lev_cap_;
-      a.level = L;
-      a.dt_level = dt_inclusive(tstart_, tstop_, L);
-      check(cudaMemsetAsync(n_active, 0, sizeof(unsigned), st), "memset");
-      check(launch_stl_level(a, st), "stl level");
-      last_launches += 2;
-      last_samples += ((int64_t)1 << L) * n;
-      last_level = L;
-      if (L > 8) {  // facets can stop from level 9 on
-        check(cudaMemcpyAsync(ctl_host_ + 9, n_active, sizeof(unsigned), cudaMemcpyDeviceToHost, st), "count");
-        check(cudaStreamSynchronize(st), "count");
-        if (ctl_host_[9] == 0) break;
+      for (int l = L; l <= end; ++l) {
+        a.first = l == L1;
+        a.level = l;
+        a.dt_prev = l >= 1 ? dt_inclusive(tstart_, tstop_, l - 1) : 0;
+        a.dt_level = dt_inclusive(tstart_, tstop_, l);
+        const int64_t s0 = a.first ? 1 : (int64_t)1 << l, s1 = (int64_t)2 << l;
+        a.n_box = stl_box_blocks(s1 - s0);
+        check(launch_stl_prepare(a, s0, s1, stl_cen_.as<double>(), stl_geo_.as<double>(), stl_nrm_.as<double>(), d_box, st),
+              "stl prepare");
+        const int64_t units = a.first ? n : n * std::max<int64_t>(1, (s1 - s0) / 512);
+        check(launch_stl_wave(a, (int)std::min<int64_t>(units, a.first ? n : (int64_t)grid), st), "stl wave");
+        last_launches += 2;
       }
+      check(cudaMemcpyAsync(host, d_state, back, cudaMemcpyDeviceToHost, st), "state");
+      check(cudaStreamSynchronize(st), "state");
+      L = end + 1;
+      const unsigned* active = reinterpret_cast<const unsigned*>(host + sizeof(double) * 4 * n + sizeof(int) * 2 * n);
+      if (end > 8 && active[end] == 0) break;
     }
-    (void)last_level;
-    check(cudaMemcpyAsync(state.data(), stl_state_.p, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, st), "state");
-    check(cudaMemcpyAsync(flags.data(), stl_flags_.p, sizeof(int) * 2 * n, cudaMemcpyDeviceToHost, st), "state");
-    check(cudaStreamSynchronize(st), "state");
+    const double* state = reinterpret_cast<const double*>(host);
+    const int* flags = reinterpret_cast<const int*>(state + 4 * n);
+    const unsigned* active = reinterpret_cast<const unsigned*>(flags + 2 * n);
+    for (int l = 0; l <= lstop; ++l) {  // levels some facet still needed
+      last_samples += ((int64_t)1 << l) * n;
+      if (l > 8 && active[l] == 0) break;
+    }
     // src/OSCARSSR.cc:3503-3521.  Result_Level lives outside the loop over facets: a facet that does
     // not stop reports the level of the last facet that did (-1 before any).
     const double scale = std::fabs(P.q * P.current) / (16 * (kPi * kPi) * kEps0 * kC);

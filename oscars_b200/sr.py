@@ -729,8 +729,7 @@ class sr:
         self.last_levels = lv
         if stlofile:
             self._stl.write_stl(stlofile)
-        return [[[facets[i, 0:3].tolist(), facets[i, 3:6].tolist(), facets[i, 6:9].tolist()], float(out[i])]
-                for i in range(n)]
+        return [list(f) for f in zip(facets[:, :9].reshape(n, 3, 3).tolist(), out.tolist())]
 
     def last_stats(self):
         """(samples integrated, kernel launches) of the last radiation call."""
