@@ -5,7 +5,7 @@
 // observers and energies and whose results are averaged (src/OSCARSSR.cc:4026-4062); a set of
 // uneven undulator jobs is a batch of unrelated jobs.  Per chunk of jobs every stage runs once over
 // all of them:
-//   k_batch_rk4       FP64 RK4, one thread per (job, direction)           src/OSCARSSR.cc:910-1009
+//   k_batch_rk4       FP64 RK4, one lane pair per (job, direction)        src/OSCARSSR.cc:910-1009
 //   k_batch_extent    trajectory extent in the job frame (validity bound of the mixed phase form)
 //   k_batch_spline    clamped cubic spline, one thread per (job, component) include/TOMATH.h:141-203
 //   k_batch_fill      level samples written straight as mixed pair records, one thread per sample
@@ -153,96 +153,169 @@ __device__ void field_sum_d(const DevField* __restrict__ fs, int nf, const doubl
   }
 }
 
-struct Rk4Ctx {
-  const DevField* fs;
-  int nf;
-  const double* vals;
-  double qomg;
-  bool superluminal;
+// An ideal undulator without half-period factors or time dependence, its constants in registers: the
+// operations of field_sum_d and pole_block_d, with the pole limits formed once.
+struct IdealField {
+  double hi, lo, hi1, lo1, hi2, lo2;  // ends of the field, of its 3/4 poles, of its 1/4 poles
+  double cx, cy, cz, ux, uy, uz, k_arg, shift, taper, ax, ay, az;
 };
+__device__ __forceinline__ bool ideal_field(const DevField& f) { return f.kind == 0 && f.n_half == 0 && f.frequency == 0; }
+__device__ __forceinline__ IdealField load_ideal(const DevField& f) {
+  IdealField q;
+  const double L = f.length, lam = f.period_length, shift = f.shift[0];
+  q.hi = L / 2. + shift;
+  q.lo = -L / 2. + shift;
+  q.hi1 = L / 2. + shift - lam;
+  q.lo1 = -L / 2. + shift + lam;
+  q.hi2 = L / 2. + shift - lam / 2.;
+  q.lo2 = -L / 2. + shift + lam / 2.;
+  q.cx = f.center[0]; q.cy = f.center[1]; q.cz = f.center[2];
+  q.ux = f.period_unit[0]; q.uy = f.period_unit[1]; q.uz = f.period_unit[2];
+  q.k_arg = f.k_arg;
+  q.shift = shift;
+  q.taper = f.taper;
+  q.ax = f.a[0]; q.ay = f.a[1]; q.az = f.a[2];
+  return q;
+}
+__device__ __forceinline__ void add_ideal(const IdealField& f, double x, double y, double z, double* B) {
+  const double d = (x - f.cx) * f.ux + (y - f.cy) * f.uy + (z - f.cz) * f.uz;
+  const double tc = 1 + d * f.taper;
+  if (d > f.hi || d < f.lo) return;
+  const double s = sin(f.k_arg * (d - f.shift));
+  const double k = (d < f.lo1 || d > f.hi1) ? ((d < f.lo2 || d > f.hi2) ? 0.25 : 0.75) : 1.0;
+  B[0] = __dadd_rn(B[0], __dmul_rn(__dmul_rn(__dmul_rn(f.ax, k), s), tc));
+  B[1] = __dadd_rn(B[1], __dmul_rn(__dmul_rn(__dmul_rn(f.ay, k), s), tc));
+  B[2] = __dadd_rn(B[2], __dmul_rn(__dmul_rn(__dmul_rn(f.az, k), s), tc));
+}
 
-__device__ __forceinline__ void derivs_d(Rk4Ctx& c, double t, const double* x, double* dxdt) {
+// dv/dt of a state with velocity v in field B; false at or above the speed of light (reported to the host).
+__device__ __forceinline__ bool accel_d(double qomg, const double* v, const double* B, double* a) {
   constexpr double kInvC2 = 1.0 / (kCLight * kCLight);
-  const double one_minus = 1. - (x[1] * x[1] + x[3] * x[3] + x[5] * x[5]) * kInvC2;
-  if (one_minus <= 0) {  // a state at or above c: reported to the host, dxdt left as it was
-    c.superluminal = true;
-    return;
-  }
-  double B[3];
-  field_sum_d(c.fs, c.nf, c.vals, x[0], x[2], x[4], t, B);
-  dxdt[0] = x[1];
-  dxdt[1] = c.qomg * (-x[5] * B[1] + x[3] * B[2]);
-  dxdt[2] = x[3];
-  dxdt[3] = c.qomg * (x[5] * B[0] - x[1] * B[2]);
-  dxdt[4] = x[5];
-  dxdt[5] = c.qomg * (x[1] * B[1] - x[3] * B[0]);
+  a[0] = __dmul_rn(qomg, __fma_rn(v[1], B[2], -__dmul_rn(v[2], B[1])));
+  a[1] = __dmul_rn(qomg, __fma_rn(v[2], B[0], -__dmul_rn(v[0], B[2])));
+  a[2] = __dmul_rn(qomg, __fma_rn(v[0], B[1], -__dmul_rn(v[1], B[0])));
+  return !(1. - (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]) * kInvC2 <= 0);
 }
 
-__device__ __forceinline__ void rk4_step_d(Rk4Ctx& c, double* y, const double* dydx, double x, double h) {
-  double dym[6], dyt[6], yt[6];
-  const double hh = h * 0.5, h6 = h / 6.0, xh = x + hh;
-  for (int i = 0; i < 6; ++i) yt[i] = y[i] + hh * dydx[i];
-  derivs_d(c, xh, yt, dyt);
-  for (int i = 0; i < 6; ++i) yt[i] = y[i] + hh * dyt[i];
-  derivs_d(c, xh, yt, dym);
-  for (int i = 0; i < 6; ++i) {
-    yt[i] = y[i] + h * dym[i];
-    dym[i] += dyt[i];
+// RK4 of one trajectory per lane pair.  What bounds it is the latency of one step's chain, and most of
+// that is the four field evaluations.  The position of a stage needs the velocity of the stage before,
+// not its acceleration, so stages 1 and 2 evaluate the field at positions both known at the start of the
+// step, and stages 3 and 4 at positions both known once those two are: the pair's lanes evaluate two
+// stages' fields side by side, exchange them and carry the same state (one thread for all four:
+// 2.05 us per undulator step with its field's constants re-read, 2.7 us with two fields; a pair with the
+// constants in registers: 0.36 and 0.49 us).  Every operation is spelled out with its rounding: a trajectory's
+// last bits move the phases far along it, and left to the compiler the fusing differs with the code around it.
+// NF: ideal undulators held in registers (0: any fields).
+template <int NF>
+__device__ __forceinline__ void rk4_pair(const DevJob& J, bool fwd, int role, const DevField* __restrict__ fields,
+                                         const double* __restrict__ vals, double* __restrict__ K, unsigned pair,
+                                         bool* superluminal) {
+  const DevField* fs = fields + J.field_begin;
+  IdealField q[NF > 0 ? NF : 1];
+#pragma unroll
+  for (int f = 0; f < NF; ++f) q[f] = load_ideal(fs[f]);
+  auto field = [&](const double* x, double t, double* B) {
+    if (NF > 0) {
+      B[0] = B[1] = B[2] = 0;
+#pragma unroll
+      for (int f = 0; f < NF; ++f) add_ideal(q[f], x[0], x[1], x[2], B);
+    } else {
+      field_sum_d(fs, J.field_count, vals, x[0], x[1], x[2], t, B);
+    }
+  };
+  // the field at two stages' positions: this lane's, then both
+  auto both = [&](const double* xa, double ta, const double* xb, double tb, double* Ba, double* Bb) {
+    double x[3], B[3], o[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) x[c] = role ? xb[c] : xa[c];
+    field(x, role ? tb : ta, B);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      o[c] = __shfl_xor_sync(pair, B[c], 1);
+      Ba[c] = role ? o[c] : B[c];
+      Bb[c] = role ? B[c] : o[c];
+    }
+  };
+  const int64_t n = (int64_t)J.nf + J.nb;
+  const double* x0 = J.frame.x0;
+  double x[3] = {x0[0], x0[1], x0[2]}, v[3] = {J.b0[0] * kCLight, J.b0[1] * kCLight, J.b0[2] * kCLight};
+  double a1[3], a_prev[3] = {0, 0, 0};
+  const double t0 = J.frame.t_ref, h = fwd ? J.dt : -J.dt;
+  const double hh = h * 0.5, h6 = h / 6.0, qomg = J.qomg;
+  // beta and a/c by one product with 1/c (within an ulp of the host's division); each lane stores five of
+  // a point's ten values
+  constexpr double kInvC = 1.0 / kCLight;
+  auto store = [&](int64_t i, double tt, const double* a) {
+    double* p = K + (role ? 5 * n : 0) + i;
+    p[0] = role ? v[1] * kInvC : tt;
+    p[n] = role ? v[2] * kInvC : x[0];
+    p[2 * n] = role ? a[0] * kInvC : x[1];
+    p[3 * n] = role ? a[1] * kInvC : x[2];
+    p[4 * n] = role ? a[2] * kInvC : v[0] * kInvC;
+  };
+  bool ok = true;
+  const int steps = fwd ? J.nf : J.nb;
+  for (int i = 0; i < steps; ++i) {
+    const double tt = t0 + h * i, th = tt + hh;
+    double y[3], w2[3], w3[3], w4[3], z3[3], z4[3], a2[3], a3[3], a4[3], Ba[3], Bb[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) y[c] = __fma_rn(hh, v[c], x[c]);
+    both(x, tt, y, th, Ba, Bb);
+    ok &= accel_d(qomg, v, Ba, a1);
+    if (fwd) {
+      store(J.nb + i, tt, i == 0 ? a1 : a_prev);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) a_prev[c] = a1[c];
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) w2[c] = __fma_rn(hh, a1[c], v[c]);
+    ok &= accel_d(qomg, w2, Bb, a2);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      z3[c] = __fma_rn(hh, w2[c], x[c]);
+      w3[c] = __fma_rn(hh, a2[c], v[c]);
+      z4[c] = __fma_rn(h, w3[c], x[c]);
+    }
+    both(z3, th, z4, tt + h, Ba, Bb);
+    ok &= accel_d(qomg, w3, Ba, a3);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) w4[c] = __fma_rn(h, a3[c], v[c]);
+    ok &= accel_d(qomg, w4, Bb, a4);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double dx = __dadd_rn(w3[c], w2[c]), dv = __dadd_rn(a3[c], a2[c]);
+      x[c] = __fma_rn(h6, __fma_rn(2.0, dx, __dadd_rn(v[c], w4[c])), x[c]);
+      v[c] = __fma_rn(h6, __fma_rn(2.0, dv, __dadd_rn(a1[c], a4[c])), v[c]);
+    }
+    if (!fwd) store(J.nb - 1 - i, t0 + h * (i + 1), a1);
   }
-  derivs_d(c, x + h, yt, dyt);
-  for (int i = 0; i < 6; ++i) y[i] = y[i] + h6 * (dydx[i] + dyt[i] + 2.0 * dym[i]);
+  if (!ok) *superluminal = true;
 }
 
-// One thread per (job, direction).  Forward points land at [nb, nb + nf), backward points at
-// [0, nb) in time order; each point carries the acceleration of the state before it, as the
-// reference's integrator stores it (src/OSCARSSR.cc:930-1004).
-__global__ void k_batch_rk4(const DevJob* __restrict__ jobs, int njobs, const DevField* __restrict__ fields,
-                            const double* __restrict__ field_vals, double* __restrict__ arena,
-                            unsigned* __restrict__ err) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 2 * njobs) return;
+// Forward points land at [nb, nb + nf), backward points at [0, nb) in time order; each point carries the
+// acceleration of the state before it, as the reference's integrator stores it
+// (src/OSCARSSR.cc:930-1004).  per_warp (1 to 16) trajectories share a warp: one each while there are
+// warps to spare, since trajectories that sit in different poles run one after another.
+__global__ void __launch_bounds__(32) k_batch_rk4(const DevJob* __restrict__ jobs, int njobs, int per_warp,
+                                                  const DevField* __restrict__ fields,
+                                                  const double* __restrict__ field_vals, double* __restrict__ arena,
+                                                  unsigned* __restrict__ err) {
+  const int slot = threadIdx.x >> 1;
+  const int t = blockIdx.x * per_warp + slot;
+  if (slot >= per_warp || t >= 2 * njobs) return;
   const DevJob& J = jobs[t >> 1];
   const bool fwd = (t & 1) == 0;
-  const int64_t n = (int64_t)J.nf + J.nb;
+  const unsigned pair = 3u << (threadIdx.x & 30);
   double* K = arena + J.knots;
-  Rk4Ctx c{fields + J.field_begin, J.field_count, field_vals, J.qomg, false};
-  const double* x0 = J.frame.x0;
-  double x[6] = {x0[0], J.b0[0] * kCLight, x0[1], J.b0[1] * kCLight, x0[2], J.b0[2] * kCLight};
-  double dxdt[6] = {0, 0, 0, 0, 0, 0};
-  const double t0 = J.frame.t_ref;
-  // beta and a/c by one product with 1/c (within an ulp of the host's division): divisions here would
-  // sit in the in-order instruction stream of the serial chain
-  constexpr double kInvC = 1.0 / kCLight;
-  auto store = [&](int64_t i, double tt) {
-    K[i] = tt;
-    K[n + i] = x[0];
-    K[2 * n + i] = x[2];
-    K[3 * n + i] = x[4];
-    K[4 * n + i] = x[1] * kInvC;
-    K[5 * n + i] = x[3] * kInvC;
-    K[6 * n + i] = x[5] * kInvC;
-    K[7 * n + i] = dxdt[1] * kInvC;
-    K[8 * n + i] = dxdt[3] * kInvC;
-    K[9 * n + i] = dxdt[5] * kInvC;
-  };
-  if (fwd) {
-    derivs_d(c, t0, x, dxdt);
-    for (int i = 0; i < J.nf; ++i) {
-      const double tt = t0 + J.dt * i;
-      store(J.nb + i, tt);
-      derivs_d(c, tt, x, dxdt);
-      rk4_step_d(c, x, dxdt, tt, J.dt);
-    }
-  } else {
-    const double dtr = -J.dt;
-    for (int i = 0; i < J.nb; ++i) {
-      const double t1 = t0 + dtr * i;
-      derivs_d(c, t1, x, dxdt);
-      rk4_step_d(c, x, dxdt, t1, dtr);
-      store(J.nb - 1 - i, t0 + dtr * (i + 1));
-    }
-  }
-  if (c.superluminal) atomicOr(err, kErrSuperluminal);
+  bool superluminal = false;
+  const DevField* fs = fields + J.field_begin;
+  if (J.field_count == 1 && ideal_field(fs[0]))
+    rk4_pair<1>(J, fwd, threadIdx.x & 1, fields, field_vals, K, pair, &superluminal);
+  else if (J.field_count == 2 && ideal_field(fs[0]) && ideal_field(fs[1]))
+    rk4_pair<2>(J, fwd, threadIdx.x & 1, fields, field_vals, K, pair, &superluminal);
+  else
+    rk4_pair<0>(J, fwd, threadIdx.x & 1, fields, field_vals, K, pair, &superluminal);
+  if (superluminal) atomicOr(err, kErrSuperluminal);
 }
 
 // The same clamped spline with each sweep split across the threads of a block (one block per job
@@ -947,6 +1020,9 @@ static cudaError_t launch_batch_wave(const BatchWaveArgs& a, int grid, int varia
 // Host orchestration
 // ---------------------------------------------------------------------------------------------
 namespace {
+// trajectories per warp of k_batch_rk4: as few as keep one warp per sub-partition (592 on B200)
+int rk4_per_warp(int nj) { return std::min(16, std::max(1, (2 * nj + 591) / 592)); }
+int rk4_blocks(int nj) { return (2 * nj + rk4_per_warp(nj) - 1) / rk4_per_warp(nj); }
 constexpr int kBatchPrefill = 13;        // levels enqueued without the host (records kept resident)
 constexpr int kBatchMinSpan = 128;
 constexpr int kBatchMaxJobsPerChunk = 8192;
@@ -1234,7 +1310,7 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
     // trajectories, splines, the resident levels' records and the waves up to Lpre: no host sync
     auto front = [&](int v, bool tune) {
       check(cudaMemsetAsync(misc, 0, 64, st), "memset");
-      dev::k_batch_rk4<<<(2 * nj + 63) / 64, 64, 0, st>>>(d_jobs, nj, b_fields_.as<DevField>(),
+      dev::k_batch_rk4<<<rk4_blocks(nj), 32, 0, st>>>(d_jobs, nj, rk4_per_warp(nj), b_fields_.as<DevField>(),
                                                           b_fvals_.as<double>(), b_knots_.as<double>(), misc);
       dev::k_batch_extent<<<nj, 256, 0, st>>>(d_jobs, b_knots_.as<double>());
       dev::launch_batch_splines(d_jobs, nj, n_max, n_total, b_knots_.as<double>(), b_work_.as<double>(), spline_kernel,
@@ -1395,7 +1471,7 @@ void Engine::batch_trajectories(const std::vector<FieldSpec>& fields, const std:
   check(cudaMemcpyAsync(b_jobs_.p, dj.data(), sizeof(DevJob) * nj, cudaMemcpyHostToDevice, st), "jobs");
   unsigned* err = b_cnt_.as<unsigned>();
   check(cudaMemsetAsync(err, 0, sizeof(unsigned), st), "memset");
-  dev::k_batch_rk4<<<(2 * nj + 63) / 64, 64, 0, st>>>(b_jobs_.as<DevJob>(), nj, b_fields_.as<DevField>(),
+  dev::k_batch_rk4<<<rk4_blocks(nj), 32, 0, st>>>(b_jobs_.as<DevJob>(), nj, rk4_per_warp(nj), b_fields_.as<DevField>(),
                                                       b_fvals_.as<double>(), b_knots_.as<double>(), err);
   dev::launch_batch_splines(b_jobs_.as<DevJob>(), nj, n_max, n_total, b_knots_.as<double>(), b_work_.as<double>(),
                             spline_kernel, st);

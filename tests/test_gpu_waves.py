@@ -123,3 +123,24 @@ def test_stl_shadowing_matches_oracle(tmp_path, shields, spread, level, seed):
     _write_stl(path, tris)
     got, want = _stl_both(path, dict(max_level=level))
     assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))
+
+
+# Device trajectories: one or two ideal undulators in registers, other fields through the general evaluation, one to
+# several trajectories a warp.  Every path rounds alike: a job's trajectory does not depend on its company, and an
+# undulator given as two halves of its amplitude in one job (registers) or with an idle grid beside them (general
+# evaluation) moves the particle the same way.
+@pytest.mark.parametrize("npoints", [3, 4, 33, 1000])
+def test_device_trajectory_paths_agree_bit_for_bit(npoints):
+    from oscars_b200.batch import BatchRunner, Job, grid, undulator
+    a = undulator([0, 0.5, 0], [0, 0, 0.05], 5, phase=-0.7, taper=0.01)
+    b = undulator([0.25, 0, 0.01], [0, 0, 0.04], 6)
+    idle = grid(np.zeros((8, 3)), [2, 2, 2], [5, 5, 5], [1, 1, 1])
+
+    def job(*fields):
+        return Job(fields=list(fields), energy_GeV=3.0, ctstartstop=(-0.4, 0.5), npoints=npoints, obs=[[0, 0, 20]], energies_eV=[400.0])
+    r = BatchRunner(gpu=0)
+    alone = [r.trajectories([job(*f)])[0] for f in ([a], [a, idle], [a, b], [a, b, idle])]
+    assert np.array_equal(alone[0], alone[1]) and np.array_equal(alone[2], alone[3])
+    many = r.trajectories([job(a), job(a, b), job(a, idle)] * 200)  # 1200 trajectories: three a warp
+    for k in range(0, 600, 3):
+        assert np.array_equal(many[k], alone[0]) and np.array_equal(many[k + 1], alone[2]) and np.array_equal(many[k + 2], alone[0])
