@@ -129,7 +129,7 @@ def test_stl_shadowing_matches_oracle(tmp_path, shields, spread, level, seed):
 # several trajectories a warp.  Every path rounds alike: a job's trajectory does not depend on its company, and an
 # undulator given as two halves of its amplitude in one job (registers) or with an idle grid beside them (general
 # evaluation) moves the particle the same way.
-@pytest.mark.parametrize("npoints", [3, 4, 33, 1000])
+@pytest.mark.parametrize("npoints", [7, 8, 33, 1000])
 def test_device_trajectory_paths_agree_bit_for_bit(npoints):
     from oscars_b200.batch import BatchRunner, Job, grid, undulator
     a = undulator([0, 0.5, 0], [0, 0, 0.05], 5, phase=-0.7, taper=0.01)
@@ -137,7 +137,8 @@ def test_device_trajectory_paths_agree_bit_for_bit(npoints):
     idle = grid(np.zeros((8, 3)), [2, 2, 2], [5, 5, 5], [1, 1, 1])
 
     def job(*fields):
-        return Job(fields=list(fields), energy_GeV=3.0, ctstartstop=(-0.4, 0.5), npoints=npoints, obs=[[0, 0, 20]], energies_eV=[400.0])
+        return Job(fields=list(fields), energy_GeV=3.0, ctstartstop=(-4e-4 * npoints, 5e-4 * npoints), npoints=npoints,
+                   obs=[[0, 0, 20]], energies_eV=[400.0])
     r = BatchRunner(gpu=0)
     alone = [r.trajectories([job(*f)])[0] for f in ([a], [a, idle], [a, b], [a, b, idle])]
     assert np.array_equal(alone[0], alone[1]) and np.array_equal(alone[2], alone[3])
