@@ -30,7 +30,7 @@ NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr
 
 CU_SOURCES = ["kernels_fp64.cu", "kernels_mixed.cu", "kernels_lines.cu", "kernels_stl.cu", "engine.cu", "stl.cu", "noalloc.cu", "batch.cu", "adjoint.cu"]
 CC_SOURCES = ["host_core.cc", "capi.cc"]
-HEADERS = ["host_core.h", "engine.h", "kernels.h", "batch.h", "device_common.cuh", "fd_common.cuh"]
+HEADERS = ["host_core.h", "engine.h", "kernels.h", "batch.h", "device_common.cuh", "fd_common.cuh", "lines.cuh"]
 
 
 def _newer(src_list, target):

@@ -39,7 +39,7 @@ namespace dev {
 
 // ---- 1. entry sums and weights ------------------------------------------------------------
 // part: partials of a one-span first wave at level L (two segments: levels 0..L-1 and level L),
-// entry-major [entry][segment][kFdPartials] (the FP64 wave, unfused) when tile_entries == 0, else
+// entry-major [entry][segment][kFdPartials] (the FP64 and line waves, unfused) when tile_entries == 0, else
 // tile-major [tile][segment][kFdPartials][entry in tile] (the mixed wave).  S: the 6 sums of every
 // entry; flux: F = C2 |C0 dT S|^2.
 __global__ void k_adj_sums(const double* __restrict__ part, int64_t n, int tile_entries, double c0dt, double c2,
@@ -954,7 +954,17 @@ void Engine::flux_vjp(const double* obs, int64_t n_obs, const std::vector<double
     w.n_e = n_e; w.n_items = N; w.act = nullptr; w.n_act = nullptr; w.first = 1; w.level = level;
     w.min_span = 32; w.target_units = 1; w.err = cnt + kCntErr; w.work = work; w.fused = 0;
     int te = 0;
-    if (mixed) {
+    // enough energies an observer: the line kernels, which form each sample's term once for all of them
+    if (n_e >= kLineMinEnergies && forced_variant[mixed ? 2 : 0] < 0) {
+      part_.reserve(sizeof(double) * 2 * kFdPartials * N);
+      w.lev = mixed ? reinterpret_cast<const double*>(mrec_.p) : lev_.as<double>();
+      w.cap = lev_cap_; w.tile_entries = lines_entries_per_cta(); w.part = part_.as<double>();
+      w.e_tiles = (n_e + w.tile_entries - 1) / w.tile_entries;
+      set_phase_reach(w);
+      check(launch_fd_lines(w, mixed ? &frame_ : nullptr,
+                            (int)std::min<int64_t>(2 * n_obs * w.e_tiles, wave_grid(mixed ? 6 : 5, 0)), st),
+            "adjoint forward (lines)");
+    } else if (mixed) {
       const int v = variant_in_use(2);
       te = mixed_entries_per_cta(v);
       part_.reserve(sizeof(double) * 2 * kFdPartials * te * ((N + te - 1) / te));

@@ -26,6 +26,7 @@
 #include "engine.h"
 #include "fd_common.cuh"
 #include "kernels.h"
+#include "lines.cuh"
 
 namespace osc {
 namespace dev {
@@ -577,14 +578,15 @@ void launch_batch_splines(const DevJob* d_jobs, int nj, int64_t n_max, int64_t n
 }
 
 
-// Level samples [s_begin, s_end) of every job whose active count is non-zero (all jobs when `cnt` is
+// Level samples [s_begin, s_end) of every job with active entries or tiles (all jobs when `cnt` is
 // NULL), evaluated from its spline and written as pair records (fd_common.cuh): job j's records
 // start at float kPairFloats / 2 * j * stride of `rec`, sample s at local index s - s_off (s_off
 // even); sample 0 is the zero-amplitude record; levels above ext_from are extended levels
 // (level_time).  One thread per (job, sample).
 __global__ void k_batch_fill(const DevJob* __restrict__ jobs, int njobs, const double* __restrict__ arena,
-                             const unsigned* __restrict__ cnt, float* __restrict__ rec, int64_t stride,
-                             int64_t s_off, int64_t s_begin, int64_t s_end, int ext_from) {
+                             const unsigned* __restrict__ cnt, const unsigned* __restrict__ n_tiles,
+                             float* __restrict__ rec, int64_t stride, int64_t s_off, int64_t s_begin, int64_t s_end,
+                             int ext_from) {
   // The two samples of a pair sit in adjacent lanes (per = s_end - s_begin, s_begin and the block
   // size are even) and exchange their FP64 values for the pair's step: every lane reaches the
   // shuffles, lanes past the grid's end or of a finished job on a valid sample, writing nothing.
@@ -592,7 +594,7 @@ __global__ void k_batch_fill(const DevJob* __restrict__ jobs, int njobs, const d
   const int64_t g_raw = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t g = g_raw < per * njobs ? g_raw : per * njobs - 2 + (g_raw & 1);
   const int j = (int)(g / per);
-  const bool active = g_raw < per * njobs && !(cnt && cnt[j] == 0);
+  const bool active = g_raw < per * njobs && !(cnt && cnt[j] == 0 && n_tiles[j] == 0);
   const DevJob& J = jobs[j];
   const int64_t s = s_begin + g % per;
   const int64_t n = (int64_t)J.nf + J.nb;
@@ -620,13 +622,24 @@ __global__ void k_batch_fill(const DevJob* __restrict__ jobs, int njobs, const d
                       qy, qz, xo, yo, zo, to);
 }
 
+// Energies of a line job's widest block: the stride of its partials.
+__host__ __device__ inline int line_width(const DevJob& J) { return J.n_e < kLnTile ? (int)J.n_e : kLnTile; }
+
 // Offsets of one wave over the chunk (one block of 1024 threads): per job the active count n_j (all
 // entries on the first wave), units = ceil(n_j / tile) x spans, partial doubles
 // n_j x nseg x spans x kFdPartials, and exclusive prefix sums of the three.  `spans` is common to
 // the wave: the smallest power of two giving at least target_units units in total (wave_spans).
+// With LINES the line jobs' plan instead, its entries being their tiles (tile = 1) and cnt their active tile
+// counts: units include the segments, partials the energies of a block.
+template <bool LINES>
 __global__ void __launch_bounds__(1024) k_batch_plan(const DevJob* __restrict__ jobs, int njobs,
                                                      const unsigned* __restrict__ cnt, int first, int L, int tile,
                                                      int64_t target, int min_span, BatchPlan P) {
+  auto active = [&](int j) -> int64_t {
+    const DevJob& J = jobs[j];
+    if (!first) return (int64_t)cnt[j];
+    return (J.e_tiles > 0) != LINES ? 0 : J.n_obs * (LINES ? (int64_t)J.e_tiles : J.n_e);
+  };
   constexpr int T = 1024;
   __shared__ int64_t red[3][T];
   __shared__ int64_t carry[3];
@@ -634,8 +647,7 @@ __global__ void __launch_bounds__(1024) k_batch_plan(const DevJob* __restrict__ 
   const int tid = threadIdx.x;
   int64_t tiles = 0;
   for (int j = tid; j < njobs; j += T) {
-    const int64_t na = first ? jobs[j].n_obs * jobs[j].n_e : (int64_t)cnt[j];
-    tiles += (na + tile - 1) / tile;
+    tiles += (active(j) + tile - 1) / tile;
   }
   red[0][tid] = tiles;
   __syncthreads();
@@ -655,9 +667,9 @@ __global__ void __launch_bounds__(1024) k_batch_plan(const DevJob* __restrict__ 
     const int j = base + tid;
     int64_t v[3] = {0, 0, 0};
     if (j < njobs) {
-      const int64_t na = first ? jobs[j].n_obs * jobs[j].n_e : (int64_t)cnt[j];
-      v[0] = (na + tile - 1) / tile * spans;
-      v[1] = na * nseg * spans * kFdPartials;
+      const int64_t na = active(j);
+      v[0] = (na + tile - 1) / tile * spans * (LINES ? nseg : 1);
+      v[1] = na * nseg * spans * kFdPartials * (LINES ? line_width(jobs[j]) : 1);
       v[2] = na;
     }
     for (int q = 0; q < 3; ++q) red[q][tid] = v[q];
@@ -861,6 +873,40 @@ __device__ __forceinline__ double lanes_max(double v) {
   return v;
 }
 
+// One entry of a batch after its sum S up to level L: finish it (converged or last level) or keep its state.
+template <class A_t>
+__device__ __forceinline__ void batch_entry_decide(const A_t& A, int L, const DevJob& J, int64_t e, const C3& S,
+                                                   double last_mag, double dmax, bool& finished, bool& unconverged,
+                                                   bool& survive) {
+  auto mag = [&](C3 v, double scale) {
+    C3 t = c3_scale(v, scale);
+    if (A.project) t = c3_project(t, J.pol);
+    return c3_mag2(t);
+  };
+  const double T = J.tstop - J.tstart;
+  const double dtl = T / (ldexp(1.0, L + 1) - 1);  // DeltaT inclusive to level L
+  const double this_mag = mag(S, dtl);
+  const double prec = fabs(this_mag - last_mag) / last_mag;
+  const bool stop = (L > 8 && prec < A.precision && dmax < kPiD) || (L > 8 && dmax < kPiD && this_mag == last_mag);
+  if (stop || L >= A.max_level) {
+    const int result_level = stop ? L : -1;
+    double v;
+    if (A.quantity == 1) v = prec;
+    else if (A.quantity == 2) v = (double)result_level;
+    else v = J.c2 * mag(S, J.c0 * dtl);
+    A.out[e] = v;
+    if (A.level_out) A.level_out[e] = result_level;
+    finished = true;
+    unconverged = !stop;
+  } else {
+    const int64_t N = A.n_entries;
+    A.state[e] = S.xr; A.state[N + e] = S.xi; A.state[2 * N + e] = S.yr;
+    A.state[3 * N + e] = S.yi; A.state[4 * N + e] = S.zr; A.state[5 * N + e] = S.zi;
+    A.state[6 * N + e] = this_mag;
+    survive = true;
+  }
+}
+
 // Span reduction and stop rule of every active entry of the chunk.  LANES threads per entry; with one
 // (the launch below) a warp's 32 entries read their adjacent partial records together, which the
 // waves with one span per entry -- the large ones -- make contiguous.
@@ -923,29 +969,7 @@ __global__ void __launch_bounds__(256) k_batch_finalize(BatchFinalArgs A) {
       seg_sum(0, S, dmax);
     }
     bool finished = false, unconverged = false, survive = false;
-    if (live && lane == 0) {
-      const double dtl = T / (ldexp(1.0, L + 1) - 1);  // DeltaT inclusive to level L
-      const double this_mag = mag(S, dtl);
-      const double prec = fabs(this_mag - last_mag) / last_mag;
-      const bool stop = (L > 8 && prec < A.precision && dmax < kPiD) || (L > 8 && dmax < kPiD && this_mag == last_mag);
-      if (stop || L >= A.max_level) {
-        const int result_level = stop ? L : -1;
-        double v;
-        if (A.quantity == 1) v = prec;
-        else if (A.quantity == 2) v = (double)result_level;
-        else v = J.c2 * mag(S, J.c0 * dtl);
-        A.out[e] = v;
-        if (A.level_out) A.level_out[e] = result_level;
-        finished = true;
-        unconverged = !stop;
-      } else {
-        const int64_t N = A.n_entries;
-        A.state[e] = S.xr; A.state[N + e] = S.xi; A.state[2 * N + e] = S.yr;
-        A.state[3 * N + e] = S.yi; A.state[4 * N + e] = S.zr; A.state[5 * N + e] = S.zi;
-        A.state[6 * N + e] = this_mag;
-        survive = true;
-      }
-    }
+    if (live && lane == 0) batch_entry_decide(A, L, J, e, S, last_mag, dmax, finished, unconverged, survive);
     const unsigned fin = __ballot_sync(full, finished), unc = __ballot_sync(full, unconverged);
     if (lane32 == 0) {
       if (fin) atomicAdd(A.samples, (unsigned long long)__popc(fin) * (unsigned long long)((2ll << L) - 1));
@@ -959,6 +983,170 @@ __global__ void __launch_bounds__(256) k_batch_finalize(BatchFinalArgs A) {
     if (survive && lane32 == leader) pos = atomicAdd(&A.cnt_next[j], (unsigned)__popc(peers));
     pos = __shfl_sync(full, pos, leader);
     if (survive) A.act_next[J.entry_begin + pos + __popc(peers & ((1u << lane32) - 1u))] = (int)item;
+  }
+}
+
+// ---- line jobs: many energies at each observer ----------------------------------------------------
+// The terms of a sample are formed once for a tile of up to 64 energies of one observer (lines.cuh), as in the
+// spectra's kernels: an (energy, pair) costs ~33 instructions in the place of 113.  Later waves go over the
+// tiles that still hold active energies, each tile's energies packed.
+__global__ void __launch_bounds__(kLnThreads, 4) k_batch_lines(BatchLineArgs A) {
+  __shared__ __align__(16) LineStage st;
+  __shared__ double red[(kLnWarps - 1) * 7 * kLnTile];
+  __shared__ WavePlan P;
+  __shared__ int64_t next_unit;
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) P = wave_plan_spans(A.first, A.level, *A.plan.spans);
+  __syncthreads();
+  const int64_t units = A.plan.unit_start[A.njobs];
+  unsigned chunk = 0;
+  int64_t u = blockIdx.x;
+  while (u < units) {
+    int64_t after = 0;
+    if (tid == 0) after = (int64_t)gridDim.x + (int64_t)atomicAdd(A.work, 1ull);
+    const int j = find_job(A.plan.unit_start, A.njobs, u);
+    const DevJob& J = A.jobs[j];
+    const int64_t local = u - A.plan.unit_start[j];
+    const int span = (int)local & (P.spans - 1);
+    const int g = P.nseg == 2 ? (int)(local >> P.log2_spans) & 1 : 0;
+    const int64_t pos = local >> (P.log2_spans + P.nseg - 1);  // of the tile in the job's list
+    const int64_t tile = A.first ? pos : (int64_t)A.tiles[J.tile_begin + pos];
+    const int64_t io = tile / J.e_tiles;
+    const int e0 = (int)(tile - io * J.e_tiles) * kLnTile;
+    const int n_act = A.first ? min(kLnTile, (int)J.n_e - e0) : A.tile_cnt[J.tile_begin + tile];
+    const int64_t entry0 = J.entry_begin + io * J.n_e + e0;
+    const int64_t b0 = seg_begin(P, g) + (int64_t)span * seg_span(P, g);
+    const int64_t b1 = min(seg_end(P, g), b0 + seg_span(P, g));
+    const int64_t p0 = b0 >> 1, p1 = b1 > b0 ? b1 >> 1 : p0;  // spans are whole pairs
+    const double* ob = A.obs + 3 * (J.obs_begin + io);
+    const double* R = J.frame.rot;
+    const double ox = ob[0] - J.frame.x0[0], oy = ob[1] - J.frame.x0[1], oz = ob[2] - J.frame.x0[2];
+    const double fx = R[0] * ox + R[1] * oy + R[2] * oz;
+    const double fy = R[3] * ox + R[4] * oy + R[5] * oz;
+    const double fz = R[6] * ox + R[7] * oy + R[8] * oz;
+    LineSums sum;
+#pragma unroll
+    for (int k = 0; k < kLnPer; ++k) {
+      const int q = lane + 32 * k;
+      const bool live = q < n_act;
+      const int ie = !live ? 0 : A.first ? e0 + q : A.act[entry0 + q];
+      const double om = A.omega[J.omega_begin + ie];
+      line_energy(sum, k, om);
+      if (live && tid < 32 && span == 0 && !mixed_geometry_ok(fx, fy, fz, om, J.frame)) atomicOr(A.err, kErrBadArgs);
+    }
+    // pair records of job j: absolute pair p at rec_j[kPairF4 * (p - s_off / 2)]
+    const float4* rec_j = A.rec + kPairF4 * ((int64_t)j * (A.stride >> 1)) - kPairF4 * (A.s_off >> 1);
+    line_sum(st, chunk, rec_j, p0, p1, span > 0, make_pair_obs(fx, fy, fz, 0.0), n_act > 32 ? kLnPer : 1, sum);
+    double dm[kLnPer];
+#pragma unroll
+    for (int k = 0; k < kLnPer; ++k) dm[k] = p1 > p0 ? (double)sum.dmax[k] : -1.0;  // -1 marks an empty span
+    if (tid == 0) next_unit = after;
+    line_combine(sum.S, dm, red);
+    if (tid < 32) {
+      const int W = line_width(J);
+      double* p = A.part + A.plan.part_start[j] + ((pos * P.nseg + g) * P.spans + span) * (int64_t)(kFdPartials * W);
+#pragma unroll
+      for (int k = 0; k < kLnPer; ++k) {
+        if (lane + 32 * k >= n_act) continue;
+#pragma unroll
+        for (int c = 0; c < 6; ++c) p[c * W + lane + 32 * k] = sum.S[k][c];
+        p[8 * W + lane + 32 * k] = dm[k];
+      }
+    }
+    __syncthreads();
+    u = next_unit;
+  }
+}
+
+// Span reduction and stop rule of the active tiles, 64 threads (two warps) a tile.  The tile's survivors are packed
+// in its block's place of the next list and the tile joins its job's next tiles; fewer than kLineMinEnergies, which
+// would leave most of a warp idle, go on as single entries.
+constexpr int kLnFinTiles = 4;  // tiles per block
+__global__ void __launch_bounds__(kLnFinTiles* kLnTile) k_batch_line_finalize(BatchLineFinalArgs A) {
+  __shared__ int sur[kLnFinTiles][2], base_entry[kLnFinTiles];
+  const BatchLineArgs& W = A.w;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *W.work = 0;
+  const int64_t total = W.plan.act_start[W.njobs];
+  const int spans = *W.plan.spans;
+  const int L = W.level;
+  const int nseg = (W.first && L >= 1) ? 2 : 1;
+  const int sub = threadIdx.x / kLnTile, q = threadIdx.x % kLnTile, half = q >> 5, lane = threadIdx.x & 31;
+  for (int64_t base = (int64_t)blockIdx.x * kLnFinTiles; base < total; base += (int64_t)gridDim.x * kLnFinTiles) {
+    const int64_t gidx = base + sub;
+    const bool on = gidx < total;
+    const int j = on ? find_job(W.plan.act_start, W.njobs, gidx) : 0;
+    const DevJob& J = W.jobs[j];
+    const int64_t pos = on ? gidx - W.plan.act_start[j] : 0;
+    int64_t tile = 0, entry0 = 0;
+    int n_act = 0, e0 = 0, ie = 0;
+    if (on) {
+      tile = W.first ? pos : (int64_t)W.tiles[J.tile_begin + pos];
+      const int64_t io = tile / J.e_tiles;
+      e0 = (int)(tile - io * J.e_tiles) * kLnTile;
+      n_act = W.first ? min(kLnTile, (int)J.n_e - e0) : W.tile_cnt[J.tile_begin + tile];
+      entry0 = J.entry_begin + io * J.n_e + e0;
+    }
+    const bool live = q < n_act;
+    if (live) ie = W.first ? e0 + q : W.act[entry0 + q];
+    const int64_t e = entry0 + (ie - e0);
+    bool finished = false, unconverged = false, survive = false;
+    if (live) {
+      const int wd = line_width(J);
+      const double* pbase = W.part + W.plan.part_start[j] + pos * nseg * spans * (int64_t)(kFdPartials * wd) + q;
+      auto seg_sum = [&](int g, C3& s, double& dmax) {
+        C3 t = {0, 0, 0, 0, 0, 0};
+#pragma unroll 4
+        for (int sp = 0; sp < spans; ++sp) {
+          const double* p = pbase + (int64_t)(g * spans + sp) * (kFdPartials * wd);
+          t.xr += p[0]; t.xi += p[wd]; t.yr += p[2 * wd]; t.yi += p[3 * wd]; t.zr += p[4 * wd]; t.zi += p[5 * wd];
+          dmax = fmax(dmax, p[8 * wd]);  // the span maxima include the step into each span (-1: empty)
+        }
+        s.xr += t.xr; s.xi += t.xi; s.yr += t.yr; s.yi += t.yi; s.zr += t.zr; s.zi += t.zi;
+      };
+      C3 S = {0, 0, 0, 0, 0, 0};
+      double last_mag = -1, dmax = 0;
+      if (W.first) {
+        double unused = 0;
+        if (nseg == 2) {
+          seg_sum(0, S, unused);
+          C3 t = c3_scale(S, (J.tstop - J.tstart) / (ldexp(1.0, L) - 1));  // DeltaT inclusive to level L-1
+          if (A.project) t = c3_project(t, J.pol);
+          last_mag = c3_mag2(t);
+        }
+        seg_sum(nseg - 1, S, dmax);
+      } else {
+        const int64_t N = A.n_entries;
+        S = {A.state[e], A.state[N + e], A.state[2 * N + e], A.state[3 * N + e], A.state[4 * N + e], A.state[5 * N + e]};
+        last_mag = A.state[6 * N + e];
+        seg_sum(0, S, dmax);
+      }
+      batch_entry_decide(A, L, J, e, S, last_mag, dmax, finished, unconverged, survive);
+    }
+    const unsigned full = 0xffffffffu;
+    const unsigned fin = __ballot_sync(full, finished), unc = __ballot_sync(full, unconverged);
+    const unsigned su = __ballot_sync(full, survive);
+    if (lane == 0) {
+      if (fin) atomicAdd(A.samples, (unsigned long long)__popc(fin) * (unsigned long long)((2ll << L) - 1));
+      if (unc) atomicAdd(A.not_converged, (unsigned long long)__popc(unc));
+      sur[sub][half] = __popc(su);
+    }
+    __syncthreads();
+    const int left = sur[sub][0] + sur[sub][1];
+    if (on && q == 0 && left > 0) {
+      if (left >= kLineMinEnergies) {
+        A.tile_cnt_next[J.tile_begin + tile] = left;
+        A.tiles_next[J.tile_begin + atomicAdd(&A.n_tiles_next[j], 1u)] = (int)tile;
+      } else {
+        base_entry[sub] = (int)atomicAdd(&A.cnt_next[j], (unsigned)left);
+      }
+    }
+    __syncthreads();
+    if (survive) {
+      const int at = (half ? sur[sub][0] : 0) + __popc(su & ((1u << lane) - 1u));
+      if (left >= kLineMinEnergies) A.act_next[entry0 + at] = ie;
+      else A.entries_next[J.entry_begin + base_entry[sub] + at] = (int)(e - J.entry_begin);
+    }
+    __syncthreads();
   }
 }
 
@@ -1001,6 +1189,12 @@ static int batch_blocks_per_sm(int variant) {
     case 2: return batch_occ<2, 4>();
     default: return batch_occ<1, 4>();
   }
+}
+
+int batch_lines_blocks_per_sm() {
+  int n = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dev::k_batch_lines, dev::kLnThreads, 0);
+  return n > 0 ? n : 1;
 }
 
 static int batch_tile(int variant) { return dev::kBThreads / kBatchSub[variant]; }
@@ -1214,7 +1408,9 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
   const int64_t rec_per_job = (int64_t)2 << Lpre;  // levels 0..Lpre, sample s at index s
   auto job_bytes = [&](const DevJob& d) {
     return sizeof(double) * 28 * ((size_t)d.nf + d.nb) + kMixedRecordBytesPerSample * (size_t)rec_per_job +
-           (size_t)(d.n_obs * d.n_e) * (56 + 8 + 4 + 8 + 16 * kFdPartials);
+           (size_t)(d.n_obs * d.n_e) * (56 + 8 + 4 + 8) +
+           (size_t)16 * kFdPartials *  // partials of one span: entries, or blocks of energies (twice as many at most)
+               std::max(d.n_obs * d.n_e, d.n_obs * ((d.n_e + dev::kLnTile - 1) / dev::kLnTile) * dev::line_width(d));
   };
   // Chunks: the jobs that fit the budget from the start, then, when more than one chunk is needed,
   // the same number of chunks with the jobs spread evenly (each chunk runs its serial RK4 once, so
@@ -1243,8 +1439,16 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
     }
     const int nj = (int)(j1 - j0);
     int64_t knots = 0, work = 0, N = 0, n_max = 0, n_total = 0;
+    int64_t n_tiles = 0, line_part = 0, n_entry_jobs = 0;  // line tiles, their partials of one span, entries of the others
     for (int k = 0; k < nj; ++k) {
       DevJob& d = dj[j0 + k];
+      // a block of energies shares each sample's term from kLineMinEnergies on (and level 9: every span is then
+      // whole folds); a pinned variant keeps the general kernel
+      d.e_tiles = forced_variant[3] < 0 && Lfirst == 9 && d.n_e >= kLineMinEnergies ? (int)((d.n_e + dev::kLnTile - 1) / dev::kLnTile) : 0;
+      d.tile_begin = n_tiles;
+      n_tiles += d.n_obs * d.e_tiles;
+      line_part += 2 * d.n_obs * d.e_tiles * dev::line_width(d) * kFdPartials;
+      if (d.e_tiles == 0) n_entry_jobs += d.n_obs * d.n_e;
       const int64_t n = (int64_t)d.nf + d.nb;
       n_max = std::max(n_max, n);
       n_total += n;
@@ -1257,7 +1461,11 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
     }
     // partial sums: spans = 1 gives 2 segments x N entries; a wave split into more spans has fewer
     // than 2 x target units of at most max_tile entries each (wave_spans)
-    const size_t part_doubles = (size_t)std::max<int64_t>(2 * N, 4 * target * max_tile) * kFdPartials;
+    const bool any_lines = n_tiles > 0, any_entries = n_entry_jobs > 0;
+    const int line_grid = any_lines ? wave_grid(8, 0) : 0;
+    const size_t part_doubles = std::max<size_t>(
+        (size_t)std::max<int64_t>(std::max(2 * n_entry_jobs, N), 4 * target * max_tile) * kFdPartials,
+        any_lines ? std::max<size_t>(line_part, (size_t)16 * line_grid * dev::kLnTile * kFdPartials) : 0);
     b_jobs_.reserve(sizeof(DevJob) * nj);
     b_knots_.reserve(sizeof(double) * knots);
     b_work_.reserve(sizeof(double) * work);
@@ -1270,6 +1478,18 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
     b_part_.reserve(sizeof(double) * part_doubles);
     b_plan_.reserve(sizeof(int64_t) * 3 * (nj + 1) + 64);
     b_cnt_.reserve(sizeof(unsigned) * 2 * nj + 256);
+    // line jobs: plan, unit counter, lists of tiles and their counts, per-job tile counts
+    b_line_.reserve(sizeof(int64_t) * (3 * (nj + 1) + 8) + sizeof(int) * (4 * n_tiles + 2 * nj + (n_tiles > 0 ? 2 * N : 0)));
+    BatchPlan ln_plan;
+    ln_plan.unit_start = b_line_.as<int64_t>();
+    ln_plan.part_start = ln_plan.unit_start + (nj + 1);
+    ln_plan.act_start = ln_plan.part_start + (nj + 1);
+    ln_plan.spans = reinterpret_cast<int*>(ln_plan.act_start + (nj + 1));
+    unsigned long long* ln_work = reinterpret_cast<unsigned long long*>(ln_plan.act_start + (nj + 1) + 1);
+    int* ln_tiles[2] = {reinterpret_cast<int*>(ln_work + 7), reinterpret_cast<int*>(ln_work + 7) + n_tiles};
+    int* ln_cnt[2] = {ln_tiles[1] + n_tiles, ln_tiles[1] + 2 * n_tiles};
+    unsigned* ln_n[2] = {reinterpret_cast<unsigned*>(ln_cnt[1] + n_tiles), reinterpret_cast<unsigned*>(ln_cnt[1] + n_tiles) + nj};
+    int* ln_act[2] = {reinterpret_cast<int*>(ln_n[1] + nj), reinterpret_cast<int*>(ln_n[1] + nj) + N};
     check(cudaMemcpyAsync(b_jobs_.p, dj.data() + j0, sizeof(DevJob) * nj, cudaMemcpyHostToDevice, st), "jobs");
     DevJob* d_jobs = b_jobs_.as<DevJob>();
     unsigned* cnt0 = b_cnt_.as<unsigned>();
@@ -1284,13 +1504,40 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
     plan.spans = reinterpret_cast<int*>(plan.act_start + (nj + 1));
 
     int cur = 0;  // active list / count array of the next wave
+    // The line jobs of a wave: their own plan, lists and counters (lists of wave `cur`, survivors to the others).
+    auto line_wave = [&](int L, bool first, unsigned* cin, unsigned* cout, int64_t stride, int64_t s_off, const float4* rec) {
+      check(cudaMemsetAsync(ln_n[cur ^ 1], 0, sizeof(unsigned) * nj, st), "memset");
+      dev::k_batch_plan<true><<<1, 1024, 0, st>>>(d_jobs, nj, ln_n[cur], first, L, 1, 4 * (int64_t)line_grid, kBatchMinSpan,
+                                                  ln_plan);
+      BatchLineArgs w{};
+      w.jobs = d_jobs; w.njobs = nj; w.rec = rec; w.stride = stride; w.s_off = s_off;
+      w.obs = b_obs_.as<double>(); w.omega = b_omega_.as<double>(); w.act = ln_act[cur];
+      w.tiles = ln_tiles[cur]; w.tile_cnt = ln_cnt[cur]; w.plan = ln_plan; w.first = first; w.level = L;
+      w.part = b_part_.as<double>(); w.err = misc; w.work = ln_work;
+      dev::k_batch_lines<<<line_grid, dev::kLnThreads, 0, st>>>(w);
+      BatchLineFinalArgs f{};
+      f.w = w; f.max_level = lstop; f.quantity = o.quantity; f.project = project; f.precision = o.precision;
+      f.n_entries = N; f.state = b_state_.as<double>(); f.act_next = ln_act[cur ^ 1];
+      f.entries_next = b_act_[cur ^ 1].as<int>();
+      f.tiles_next = ln_tiles[cur ^ 1]; f.tile_cnt_next = ln_cnt[cur ^ 1]; f.n_tiles_next = ln_n[cur ^ 1];
+      f.cnt_next = cout; f.out = b_out_.as<double>(); f.level_out = b_lvl_.as<int32_t>();
+      f.not_converged = m64; f.samples = m64 + 1;
+      dev::k_batch_line_finalize<<<sms * 8, dev::kLnFinTiles * dev::kLnTile, 0, st>>>(f);
+      check(cudaGetLastError(), "batch lines");
+      last_launches += 3;
+    };
     auto wave = [&](int L, int v, int64_t stride, int64_t s_off, const float4* rec) {
       const bool first = L == Lfirst;
       unsigned* cin = cnts[cur];
       unsigned* cout = cnts[cur ^ 1];
       check(cudaMemsetAsync(cout, 0, sizeof(unsigned) * nj, st), "memset");
       const int tile = batch_tile(v);
-      dev::k_batch_plan<<<1, 1024, 0, st>>>(d_jobs, nj, cin, first, L, tile, target, kBatchMinSpan, plan);
+      if (any_lines) line_wave(L, first, cin, cout, stride, s_off, rec);
+      if (first && !any_entries) {  // (later waves may have line jobs' last entries)
+        cur ^= 1;
+        return;
+      }
+      dev::k_batch_plan<false><<<1, 1024, 0, st>>>(d_jobs, nj, cin, first, L, tile, target, kBatchMinSpan, plan);
       BatchWaveArgs w{};
       w.jobs = d_jobs; w.njobs = nj; w.rec = rec; w.stride = stride; w.s_off = s_off;
       w.obs = b_obs_.as<double>(); w.omega = b_omega_.as<double>(); w.act = b_act_[cur].as<int>(); w.cnt = cin;
@@ -1310,6 +1557,8 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
     // trajectories, splines, the resident levels' records and the waves up to Lpre: no host sync
     auto front = [&](int v, bool tune) {
       check(cudaMemsetAsync(misc, 0, 64, st), "memset");
+      check(cudaMemsetAsync(ln_work, 0, sizeof(unsigned long long), st), "memset");
+      if (!any_lines) check(cudaMemsetAsync(ln_n[0], 0, sizeof(unsigned) * 2 * nj, st), "memset");
       dev::k_batch_rk4<<<rk4_blocks(nj), 32, 0, st>>>(d_jobs, nj, rk4_per_warp(nj), b_fields_.as<DevField>(),
                                                           b_fvals_.as<double>(), b_knots_.as<double>(), misc);
       dev::k_batch_extent<<<nj, 256, 0, st>>>(d_jobs, b_knots_.as<double>());
@@ -1317,10 +1566,11 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
                                 st);
       const int64_t fill_n = rec_per_job * nj;  // samples 0 .. 2^(Lpre+1) - 1 of every job
       dev::k_batch_fill<<<(unsigned)((fill_n + 255) / 256), 256, 0, st>>>(
-          d_jobs, nj, b_knots_.as<double>(), nullptr, b_rec_.as<float>(), rec_per_job, 0, 0, rec_per_job, ext_from);
+          d_jobs, nj, b_knots_.as<double>(), nullptr, nullptr, b_rec_.as<float>(), rec_per_job, 0, 0, rec_per_job,
+          ext_from);
       check(cudaGetLastError(), "batch trajectories");
       last_launches += 4;
-      if (tune) v = tune_batch(nj, Lfirst, target, d_jobs, plan, misc, m64, rec_per_job);
+      if (tune && any_entries) v = tune_batch(nj, Lfirst, target, d_jobs, plan, misc, m64, rec_per_job);
       for (int L = Lfirst; L <= Lpre; ++L) wave(L, v, rec_per_job, 0, b_rec_.as<float4>());
       return v;
     };
@@ -1372,8 +1622,9 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
     }
     // levels beyond the resident ones: records of one level at a time, for the jobs still active
     for (int L = Lpre + 1; L <= lstop; ++L) {
-      std::vector<unsigned> c(nj);
+      std::vector<unsigned> c(2 * nj);
       check(cudaMemcpyAsync(c.data(), cnts[cur], sizeof(unsigned) * nj, cudaMemcpyDeviceToHost, st), "counts");
+      check(cudaMemcpyAsync(c.data() + nj, ln_n[cur], sizeof(unsigned) * nj, cudaMemcpyDeviceToHost, st), "counts");
       check(cudaStreamSynchronize(st), "counts");
       bool any = false;
       for (unsigned x : c) any = any || x > 0;
@@ -1382,7 +1633,7 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
       b_rec_ext_.reserve((size_t)kMixedRecordBytesPerSample * len * nj);
       const int64_t fill_n = len * nj;
       dev::k_batch_fill<<<(unsigned)((fill_n + 255) / 256), 256, 0, st>>>(
-          d_jobs, nj, b_knots_.as<double>(), cnts[cur], b_rec_ext_.as<float>(), len, len, len, 2 * len, ext_from);
+          d_jobs, nj, b_knots_.as<double>(), cnts[cur], ln_n[cur], b_rec_ext_.as<float>(), len, len, len, 2 * len, ext_from);
       check(cudaGetLastError(), "batch fill");
       ++last_launches;
       wave(L, v, len, len, b_rec_ext_.as<float4>());
@@ -1496,7 +1747,7 @@ int Engine::tune_batch(int nj, int Lfirst, int64_t target, const DevJob* d_jobs,
   float best_ms = 1e30f;
   for (int v = 0; v < kBatchVariants; ++v) {
     const int tile = batch_tile(v);
-    dev::k_batch_plan<<<1, 1024, 0, st>>>(d_jobs, nj, nullptr, 1, Lfirst, tile, target, kBatchMinSpan, plan);
+    dev::k_batch_plan<false><<<1, 1024, 0, st>>>(d_jobs, nj, nullptr, 1, Lfirst, tile, target, kBatchMinSpan, plan);
     BatchWaveArgs w{};
     w.jobs = d_jobs; w.njobs = nj; w.rec = b_rec_.as<float4>(); w.stride = rec_stride; w.s_off = 0;
     w.obs = b_obs_.as<double>(); w.omega = b_omega_.as<double>(); w.act = nullptr; w.cnt = nullptr;

@@ -47,6 +47,8 @@ struct DevJob {
   int64_t u_off;            // offset of the job's 9 x n spline work block
   int64_t obs_begin, omega_begin, n_obs, n_e;
   int64_t entry_begin;      // first entry of the job in its chunk (job-major; obs-major, energy fastest)
+  int64_t tile_begin;       // line jobs: first (observer, energy block) tile of the job in its chunk
+  int e_tiles;              // line jobs: energy blocks per observer; 0: the job's entries go one by one
 };
 
 // Offsets of one wave, written by k_batch_plan: prefix sums over the jobs of the chunk.
@@ -93,9 +95,48 @@ struct BatchFinalArgs {
   unsigned long long* work_reset;
 };
 
+// A wave of the chunk's line jobs: units are (job, tile, segment, span), a tile the active ones of a block of
+// energies at one observer.  act holds each tile's energies from its block's place in the entry order.
+struct BatchLineArgs {
+  const DevJob* jobs;
+  int njobs;
+  const float4* rec;
+  int64_t stride, s_off;
+  const double* obs;
+  const double* omega;
+  const int* act;           // energies of the active tiles (unused on the first wave, like the next two)
+  const int* tiles;         // per job, its active tiles from tile_begin
+  const int* tile_cnt;      // per tile, its active energies
+  BatchPlan plan;           // act_start: active tiles
+  int first, level;
+  double* part;             // per job from part_start: [tile][segment][span][kFdPartials][energy of the block]
+  unsigned* err;
+  unsigned long long* work;
+};
+
+struct BatchLineFinalArgs {
+  BatchLineArgs w;          // (the wave's lists, plan and partials)
+  int max_level, quantity, project;
+  double precision;
+  int64_t n_entries;
+  double* state;
+  int* act_next;
+  int* entries_next;        // per job from entry_begin: survivors that go on as single entries
+  int* tiles_next;
+  int* tile_cnt_next;
+  unsigned* n_tiles_next;   // per job
+  unsigned* cnt_next;       // per job, single entries
+  double* out;
+  int* level_out;
+  unsigned long long* not_converged;
+  unsigned long long* samples;
+};
+
 struct FieldSpec;
 // Device form of a field; grid values and half-period factors are appended to `vals`.
 DevField to_dev_field(FieldSpec f, std::vector<double>& vals);
+
+int batch_lines_blocks_per_sm();
 
 // Compiled variants of the batched wave kernel (groups per CTA, minimum CTAs per SM).
 constexpr int kBatchVariants = 4;

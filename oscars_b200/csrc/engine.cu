@@ -115,7 +115,7 @@ Engine::~Engine() {
   for (DevBuf* b : {&knots_, &lev_, &bd_bits_, &mrec_bd_, &obs_, &nrm_, &omega_, &out_, &lvl_, &state_, &part_, &act_[0],
                     &act_[1], &cnt_, &acc_, &acc_comp_, &mrec_, &b_fields_, &b_fvals_, &b_obs_, &b_omega_, &b_acc_, &b_jobs_,
                     &b_knots_, &b_work_, &b_rec_, &b_rec_ext_, &b_state_, &b_out_, &b_lvl_, &b_act_[0], &b_act_[1],
-                    &b_part_, &b_plan_, &b_cnt_, &adj_, &adj_s_, &adj_r_, &adj_sums_, &adj_z_, &fused_, &stl_geo_,
+                    &b_part_, &b_plan_, &b_cnt_, &b_line_, &adj_, &adj_s_, &adj_r_, &adj_sums_, &adj_z_, &fused_, &stl_geo_,
                     &stl_cen_, &stl_nrm_,
                     &stl_state_})
     b->release();
@@ -409,6 +409,7 @@ int Engine::wave_grid(int kind, int variant) {
     check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "attr");
     const int per = kind == 2   ? mixed_blocks_per_sm(variant)
                     : kind == 4 ? pd_mixed_blocks_per_sm()
+                    : kind == 8 ? batch_lines_blocks_per_sm()
                     : kind == 7 ? stl_blocks_per_sm()
                     : kind >= 5 ? lines_blocks_per_sm(kind == 6)
                                 : fp64_blocks_per_sm(kind == 1, variant);

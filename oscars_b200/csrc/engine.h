@@ -193,7 +193,7 @@ class Engine {
   std::vector<int> pending_;
   // kernel variants: kind 0 = FP64 flux, 1 = FP64 power density, 2 = mixed flux, 3 = batched mixed,
   // 4 = mixed power density
-  int wave_grid_[8][16] = {};  // kinds: 0 fp64, 1 power density, 2 mixed, 4 mixed power density, 5 / 6 fp64 / mixed lines, 7 STL
+  int wave_grid_[9][16] = {};  // kinds: 0 fp64, 1 power density, 2 mixed, 4 mixed power density, 5 / 6 fp64 / mixed lines, 7 STL, 8 batched lines
   int wave_grid(int kind, int variant);
   std::map<std::tuple<int, int, int, int>, int> tuned_;   // (kind, log2 entries, first level, last level) -> variant
   // (kind, entries, energies, last level, precision) -> highest level the last such request needed
@@ -226,7 +226,7 @@ class Engine {
 
   // batched path
   DevBuf b_fields_, b_fvals_, b_obs_, b_omega_, b_acc_, b_jobs_, b_knots_, b_work_, b_rec_, b_rec_ext_, b_state_, b_out_,
-      b_lvl_, b_act_[2], b_part_, b_plan_, b_cnt_;
+      b_lvl_, b_act_[2], b_part_, b_plan_, b_cnt_, b_line_;
   DevBuf adj_, adj_s_, adj_r_;      // adjoint scratch
   // forward sums S (6 per entry) and flux of the last osc_flux_vjp, kept for a following call with
   // the same key (trajectory version, observers, energies, level, arithmetic, normalisation)

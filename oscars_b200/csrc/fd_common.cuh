@@ -302,6 +302,14 @@ __device__ __forceinline__ double nonneg_float_to_double(float x) {
   return __hiloint2double((int)((u >> 3) + 0x38000000u), (int)(u << 29));
 }
 
+// Exact float -> double of any finite normal float or zero on the integer pipe (denormals, which the
+// flushed FP32 arithmetic does not produce, would come out as ~6e-39).
+__device__ __forceinline__ double float_to_double_bits(float x) {
+  const unsigned u = __float_as_uint(x);
+  const unsigned hi = (u & 0x7FFFFFFFu) ? ((((u & 0x7FFFFFFFu) >> 3) + 0x38000000u) | (u & 0x80000000u)) : u;
+  return __hiloint2double((int)hi, (int)(u << 29));
+}
+
 // FP64 retarded phase of one sample as a fraction of a turn in [-1/2, 1/2) (see the section
 // comment), shifted by half a turn: a constant phase shared by every sample, which drops out of
 // |E|^2.  corr_f and half_iD = 1 / (2 D) are the sample's FP32 values.  v = 1.5 * 2^22 + turns lies

@@ -240,6 +240,9 @@ int fp64_blocks_per_sm(bool power_density, int variant);
 int fp64_entries_per_cta(int variant);
 const char* fp64_variant_name(int variant);
 
+// Energies of an observer from which its entries go in line tiles: with n of 32 lanes in use the mixed line kernel
+// takes 33 x 32 / n instructions an (energy, pair), the general one 113.
+constexpr int kLineMinEnergies = 10;
 // Many energies of one observer (kernels_lines.cu): a.lev = the FP64 level cache (F = NULL) or the
 // mixed records in frame *F; tile_entries = lines_entries_per_cta().
 int lines_entries_per_cta();

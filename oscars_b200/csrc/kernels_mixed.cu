@@ -260,14 +260,6 @@ struct PdObsMx {
   float2 nx, ny, nz;  // surface normal in the particle frame (both lanes)
 };
 
-// Exact float -> double of any finite normal float or zero on the integer pipe (denormals, which the
-// flushed FP32 arithmetic does not produce, would come out as ~6e-39).
-__device__ __forceinline__ double float_to_double_bits(float x) {
-  const unsigned u = __float_as_uint(x);
-  const unsigned hi = (u & 0x7FFFFFFFu) ? ((((u & 0x7FFFFFFFu) >> 3) + 0x38000000u) | (u & 0x80000000u)) : u;
-  return __hiloint2double((int)hi, (int)(u << 29));
-}
-
 template <bool NORMAL, bool DIRECTIONAL>
 __device__ __forceinline__ double pd_pair(const float4* __restrict__ q, const PdObsMx& o) {
   const float4 q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4], q5 = q[5];

@@ -145,3 +145,40 @@ def test_device_trajectory_paths_agree_bit_for_bit(npoints):
     many = r.trajectories([job(a), job(a, b), job(a, idle)] * 200)  # 1200 trajectories: three a warp
     for k in range(0, 600, 3):
         assert np.array_equal(many[k], alone[0]) and np.array_equal(many[k + 1], alone[2]) and np.array_equal(many[k + 2], alone[0])
+
+
+# Batched line tiles (10 energies and more) against the general kernel pinned: same terms, steps and FP32 sums, so the
+# same levels and, but for the order of FP64 additions, the same values (1e-10 of the peak, as above).  Tiles that run
+# low on active energies hand them on as single entries; jobs below 10 energies sit in the same batch.
+@pytest.mark.parametrize("sizes, kw", [([(1, 9), (1, 10), (3, 64), (2, 65)], {}), ([(5, 130), (7, 33), (40, 1), (1, 700)], {}),
+                                       ([(4, 40), (1, 12)], dict(max_level=10)), ([(3, 20), (6, 70)], dict(precision=1e-4)),
+                                       ([(2, 30), (9, 11)], dict(max_level=6))])
+def test_batch_lines_match_general_kernel(sizes, kw):
+    from oscars_b200.batch import BatchRunner, Job, undulator
+    jobs = [Job(fields=[undulator([0, 0.5, 0], [0, 0, 0.05], 11, phase=-np.pi / 2)], energy_GeV=3.0, ctstartstop=(-0.5, 0.5),
+                npoints=5001, obs=[[1e-4 * k, 5e-5 * k, 20.0 + 0.1 * i] for k in range(m)], energies_eV=np.linspace(300, 1500, n))
+            for i, (m, n) in enumerate(sizes)]
+    got = []
+    for variant in (0, -1):
+        r = BatchRunner(gpu=0)
+        r.set_variant(variant)
+        for _ in range(2):  # the second call replays the captured graph
+            f = r.flux(jobs, **kw)
+        got.append((f, [x.copy() for x in r.last_levels]))
+    for a, b, la, lb in zip(got[0][0], got[1][0], got[0][1], got[1][1]):
+        assert np.array_equal(la, lb)
+        assert np.max(np.abs(a - b)) <= 1e-10 * np.max(np.abs(a))
+
+
+# The adjoint's forward sums by line tiles against the general kernels pinned (same bounds).
+@pytest.mark.parametrize("compute", ["fp64", "mixed"])
+@pytest.mark.parametrize("n_obs, n, level", [(1, 10, 9), (3, 65, 10), (5, 33, 7)])
+def test_tuning_forward_lines_match_general_kernel(compute, n_obs, n, level):
+    from oscars_b200.tuning import TuningProblem
+    out = []
+    for variant in (0, -1):
+        p = TuningProblem(bfield=[0, 0.5, 0], period=[0, 0, 0.05], nperiods=11, obs=[[1e-4 * k, 0, 20.0] for k in range(n_obs)],
+                          energies_eV=np.linspace(400, 500, n), level=level, ctstartstop=(-0.5, 0.5), npoints=5001, compute=compute)
+        p.sr._ctx.call("osc_set_variant", 2 if compute == "mixed" else 0, variant)
+        out.append(p.flux(1 + 0.01 * np.cos(np.arange(22))))
+    assert np.max(np.abs(out[0] - out[1])) <= (1e-10 if compute == "mixed" else 1e-12) * np.max(np.abs(out[0]))
