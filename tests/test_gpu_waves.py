@@ -182,3 +182,22 @@ def test_tuning_forward_lines_match_general_kernel(compute, n_obs, n, level):
         p.sr._ctx.call("osc_set_variant", 2 if compute == "mixed" else 0, variant)
         out.append(p.flux(1 + 0.01 * np.cos(np.arange(22))))
     assert np.max(np.abs(out[0] - out[1])) <= (1e-10 if compute == "mixed" else 1e-12) * np.max(np.abs(out[0]))
+
+
+# The adjoint's samples take an observer's energies together: observers that change inside, at and across a staged
+# chunk (64 or 128 entries).  The gradient is linear in the entries, so it is the sum of the single observers'
+# gradients: FP64 to the roundings of 2^10 samples' sums (1e-11), mixed to its FP32 sums over other chunks (1e-5).
+@pytest.mark.parametrize("compute, tol", [("fp64", 1e-11), ("mixed", 1e-5)])
+@pytest.mark.parametrize("n_obs, n", [(2, 1), (3, 65), (5, 64), (2, 130)])
+def test_gradient_is_the_sum_over_observers(compute, tol, n_obs, n):
+    from oscars_b200.tuning import TuningProblem
+    obs = [[3e-4 * k, 1e-4, 20.0] for k in range(n_obs)]
+    s, weight = 1 + 0.01 * np.cos(np.arange(22)), np.cos(np.arange(n_obs * n)).reshape(n_obs, n) + 1.5
+
+    def gradient(o, w):
+        p = TuningProblem(bfield=[0, 0.5, 0], period=[0, 0, 0.05], nperiods=11, obs=o, energies_eV=np.linspace(400, 500, n),
+                          level=9, ctstartstop=(-0.5, 0.5), npoints=5001, compute=compute)
+        return p.vjp(s, w)[1]
+    whole = gradient(obs, weight)
+    parts = sum(gradient([obs[k]], weight[k:k + 1]) for k in range(n_obs))
+    assert np.max(np.abs(whole - parts)) <= tol * np.max(np.abs(whole))
