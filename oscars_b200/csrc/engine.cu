@@ -104,7 +104,7 @@ Engine::~Engine() {
   if (last_stream_valid_ && last_stream_ != stream) cudaStreamSynchronize(last_stream_);
   if (mapped_) cudaFreeHost(mapped_);
   if (bounce_) cudaFreeHost(bounce_);
-  for (PinnedStage& p : pin_pool_) {
+  for (TrajectoryBuffers& p : traj_pool_) {
     if (p.copied) {
       cudaEventSynchronize(p.copied);
       cudaEventDestroy(p.copied);
@@ -871,28 +871,34 @@ void Engine::use_stream(cudaStream_t s) {
 }
 
 // Trajectories of a list of particles integrated on host worker threads ahead of their use: worker
-// threads claim particles in order and fill a ring of slots; the consumer takes particle k's slot
-// when it is ready and releases it for particle k + slots.  A worker's exception is rethrown to
-// the consumer at that particle.
+// threads claim the particles' forward and backward sweeps in order and fill a ring of slots; the
+// consumer takes particle k's slot when it is ready and releases it for particle k + slots.  A worker's
+// exception is rethrown to the consumer at that particle.
+// What bounds a beam request is these integrations: 10 ms of one core for a particle of 60000 points and two
+// undulators (serial Runge-Kutta steps, half of it their sines), 3.5 ms for its spline and staging, 0.45 ms
+// on the device.  Half trajectories keep the cores evenly loaded and bring the first particle sooner, and
+// the buffers (20 MB a particle) stay with the engine between requests, as mapping them anew cost ~8 ms a
+// particle in page faults: 16 particles on 16 cores take 23 ms, 36 ms with whole trajectories on 15 threads
+// and fresh buffers (26 ms with half trajectories and fresh buffers).
 class TrajectoryPipeline {
  public:
   // `device`: the workers also lay each trajectory out in pinned host memory in the device knot
   // layout (t | y[9] | ypp[9] | diag), so that its upload is one asynchronous copy.
-  // `pool`: pinned staging buffers and their copy events, kept by the engine between requests (pinned
-  // allocations are slow); grown here to the slots this pipeline uses.
-  TrajectoryPipeline(const Model& m, const std::vector<Particle>& parts, int device, std::vector<PinnedStage>& pool)
-      : m_(m), parts_(parts), device_(device) {
-    const unsigned hw = std::max(2u, std::thread::hardware_concurrency());
-    const int nthreads = (int)std::min<size_t>(std::min(hw - 1u, 32u), std::max<size_t>(1, parts.size()));
-    const size_t nslots = std::min<size_t>(2 * nthreads, std::max<size_t>(1, parts.size()));
+  // `pool`: the slots' buffers, kept by the engine between requests; grown here to the slots this pipeline
+  // uses.
+  TrajectoryPipeline(const Model& m, const std::vector<Particle>& parts, int device, std::vector<TrajectoryBuffers>& pool)
+      : m_(m), parts_(parts), device_(device), pool_(pool) {
+    const size_t hw = std::max(2u, std::thread::hardware_concurrency());
+    const size_t nthreads = std::min(std::min<size_t>(hw, 32), std::max<size_t>(1, 2 * parts.size()));
+    const size_t nslots = std::min<size_t>(nthreads + 4, std::max<size_t>(1, parts.size()));
     while (pool.size() < nslots) {
       pool.emplace_back();
       const cudaError_t e = cudaEventCreateWithFlags(&pool.back().copied, cudaEventDisableTiming);
       if (e != cudaSuccess) throw Error{OSC_ERR_CUDA, std::string("event: ") + cudaGetErrorString(e)};
     }
     slots_.resize(nslots);
-    for (size_t i = 0; i < nslots; ++i) slots_[i].stage = &pool[i];
-    for (int i = 0; i < nthreads; ++i) workers_.emplace_back([this] { work(); });
+    for (size_t i = 0; i < nslots; ++i) slots_[i].buf = &pool[i];
+    for (size_t i = 0; i < nthreads; ++i) workers_.emplace_back([this] { work(); });
   }
   ~TrajectoryPipeline() {
     {
@@ -901,11 +907,17 @@ class TrajectoryPipeline {
     }
     cv_.notify_all();
     for (auto& t : workers_) t.join();
+    // the kept buffers are bounded: beyond kKeep bytes of pageable memory they are given back
+    constexpr size_t kKeep = (size_t)768 << 20;
+    size_t bytes = 0;
+    for (TrajectoryBuffers& b : pool_) bytes += b.pageable_bytes();
+    if (bytes > kKeep)
+      for (TrajectoryBuffers& b : pool_) b.drop_pageable();
   }
   // The upload of particle k's pinned copy was enqueued on `st`: the slot's next trajectory is staged
   // only after that copy has run (the request need not have waited for the device by then).
   void uploaded(size_t k, cudaStream_t st) {
-    const cudaError_t e = cudaEventRecord(slots_[k % slots_.size()].stage->copied, st);
+    const cudaError_t e = cudaEventRecord(slots_[k % slots_.size()].buf->copied, st);
     if (e != cudaSuccess) throw Error{OSC_ERR_CUDA, std::string("event: ") + cudaGetErrorString(e)};
   }
   // Particle k's trajectory: its knots and their pinned copy in the device layout.  The slot stays
@@ -913,10 +925,10 @@ class TrajectoryPipeline {
   Knots& wait(size_t k, const double** pinned) {
     Slot& s = slots_[k % slots_.size()];
     std::unique_lock<std::mutex> g(mu_);
-    cv_.wait(g, [&] { return s.ready && s.particle == (int64_t)k; });
+    ready_.wait(g, [&] { return s.ready && s.particle == (int64_t)k; });
     if (s.err) std::rethrow_exception(s.err);
-    *pinned = s.stage->pinned;
-    return s.knots;
+    *pinned = s.buf->pinned;
+    return s.buf->knots;
   }
   void release(size_t k) {
     {
@@ -929,16 +941,14 @@ class TrajectoryPipeline {
 
  private:
   struct Slot {
-    Knots knots;
-    std::vector<double> sweep[2];
-    PinnedStage* stage = nullptr;
+    TrajectoryBuffers* buf = nullptr;
     int64_t particle = -1;
+    int sweeps = 0;  // of `particle`, finished
     bool ready = false;
     std::exception_ptr err;
   };
-  static void stage(Slot& s, int device) {  // knots -> pinned t | y | ypp | diag
-    const Knots& k = s.knots;
-    PinnedStage& p = *s.stage;
+  static void stage(TrajectoryBuffers& p, int device) {  // knots -> pinned t | y | ypp | diag
+    const Knots& k = p.knots;
     const size_t n = (size_t)k.n, need = 20 * n;
     cudaError_t ev = cudaEventSynchronize(p.copied);  // the previous copy out of this buffer has run
     if (ev != cudaSuccess) throw Error{OSC_ERR_CUDA, std::string("event: ") + cudaGetErrorString(ev)};
@@ -961,37 +971,60 @@ class TrajectoryPipeline {
   void work() {
     for (;;) {
       size_t k;
+      int dir;
       {
         std::unique_lock<std::mutex> g(mu_);
-        cv_.wait(g, [&] { return stop_ || next_ >= parts_.size() || next_ < consumed_ + slots_.size(); });
-        if (stop_ || next_ >= parts_.size()) return;
-        k = next_++;
+        cv_.wait(g, [&] { return stop_ || next_ >= 2 * parts_.size() || next_ / 2 < consumed_ + slots_.size(); });
+        if (stop_ || next_ >= 2 * parts_.size()) return;
+        k = next_ / 2;
+        dir = (int)(next_ % 2);
+        ++next_;
+        if (dir == 0) {  // the slot's new particle
+          Slot& s = slots_[k % slots_.size()];
+          s.particle = (int64_t)k;
+          s.sweeps = 0;
+          s.err = nullptr;
+        }
       }
       Slot& s = slots_[k % slots_.size()];
       std::exception_ptr err;
       try {
-        m_.integrate(parts_[k], s.knots, s.sweep, false);
-        stage(s, device_);
+        m_.integrate_sweep(parts_[k], dir, s.buf->sweep[dir]);
       } catch (...) {
         err = std::current_exception();
       }
       {
         std::lock_guard<std::mutex> g(mu_);
+        if (err && !s.err) s.err = err;
+        if (++s.sweeps < 2) continue;
+        err = s.err;
+      }
+      if (!err) {  // this thread finished the second sweep: knots, spline, staging
+        try {
+          s.buf->knots.clear();
+          m_.join_sweeps(s.buf->sweep, s.buf->knots);
+          stage(*s.buf, device_);
+        } catch (...) {
+          err = std::current_exception();
+        }
+      }
+      {
+        std::lock_guard<std::mutex> g(mu_);
         s.err = err;
-        s.particle = (int64_t)k;
         s.ready = true;
       }
-      cv_.notify_all();
+      ready_.notify_all();
     }
   }
   const Model& m_;
   const std::vector<Particle>& parts_;
   const int device_;
+  std::vector<TrajectoryBuffers>& pool_;
   std::vector<Slot> slots_;
   std::vector<std::thread> workers_;
   std::mutex mu_;
-  std::condition_variable cv_;
-  size_t next_ = 0, consumed_ = 0;
+  std::condition_variable cv_, ready_;
+  size_t next_ = 0, consumed_ = 0;  // sweeps claimed, particles consumed
   bool stop_ = false;
 };
 
@@ -1183,7 +1216,7 @@ void Engine::radiation(RadRequest& rq) {
       // their trajectories are integrated on host worker threads while the GPU sums earlier ones;
       // the model holds the particle in use and its trajectory (the last ones when done, as the
       // reference leaves them)
-      TrajectoryPipeline pipe(model, mine, device, pin_pool_);
+      TrajectoryPipeline pipe(model, mine, device, traj_pool_);
       for (size_t k = 0; k < mine.size(); ++k) {
         const double* pinned = nullptr;
         Knots& kn = pipe.wait(k, &pinned);

@@ -67,12 +67,23 @@ struct BatchJob {
 double dt_inclusive(double tstart, double tstop, int L);
 void polarization_vector(const osc_rad_opts& o, double P[6], bool& project);
 
-// A pinned host buffer for staging one trajectory's upload, with the event recorded after its copy
-// to the device was enqueued (kept by the engine across multi-particle requests).
-struct PinnedStage {
+// Host buffers of one trajectory under way (kept by the engine across multi-particle requests): its sweeps, knots
+// and spline scratch, and the pinned copy its upload reads, with the event recorded after that copy was
+// enqueued.
+struct TrajectoryBuffers {
+  std::vector<double> sweep[2];
+  Knots knots;
   double* pinned = nullptr;
   size_t doubles = 0;
   cudaEvent_t copied = nullptr;
+  size_t pageable_bytes() const {
+    return sizeof(double) * (sweep[0].capacity() + sweep[1].capacity() + knots.t.capacity() + knots.y.capacity() +
+                             knots.ypp.capacity() + knots.diag.capacity() + knots.work.capacity());
+  }
+  void drop_pageable() {
+    for (std::vector<double>& v : sweep) std::vector<double>().swap(v);
+    knots = Knots();
+  }
 };
 
 class Engine {
@@ -265,7 +276,7 @@ class Engine {
   // bd_zeroed: the request prologue has zeroed the beta-step words of the levels to fill
   void prefill(bool mixed, int Lhead, int Lpre, bool bd_zeroed = false);
   void join_prefill();
-  std::vector<PinnedStage> pin_pool_;  // trajectory staging of multi-particle requests
+  std::vector<TrajectoryBuffers> traj_pool_;  // trajectories of multi-particle requests
   // STL request buffers: facet geometry (A, B - A, C - A), facets and centres, normals and box, per-facet
   // state, flags and level counters
   DevBuf stl_geo_, stl_cen_, stl_nrm_, stl_state_;

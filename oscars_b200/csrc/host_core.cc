@@ -805,121 +805,64 @@ void Model::compute_trajectory() {
   integrate(particle, knots, sweep, true);
 }
 
-void Model::integrate(const Particle& P, Knots& knots, std::vector<double>* sweep, bool threads) const {
+void Model::check_times(const Particle& P) const {
   if (!P.set) throw Error{OSC_ERR_RANGE, "particle not initialized.  make sure you have a particle or beam defined"};
   if (ctstart > P.t0 || ctstop < P.t0)
     throw Error{OSC_ERR_RANGE, "start time is greater than T0 or stop time is less than T0"};
   if (ctstart >= ctstop)
     throw Error{OSC_ERR_RANGE, "start time is greater than stop time.  check that set_ctstartstop is set"};
+}
+
+void Model::integrate(const Particle& P, Knots& knots, std::vector<double>* sweep, bool threads) const {
+  check_times(P);
   knots.clear();
+  // The forward and backward sweeps are independent integrations from the same initial state; they
+  // run on two host threads and are stitched together afterwards.
+  if (threads && (traj_method == kRKAS || npoints > 4096)) {
+    parallel_tasks(2, [&](int dir) { integrate_sweep(P, dir, sweep[dir]); });
+  } else {
+    integrate_sweep(P, 0, sweep[0]);
+    integrate_sweep(P, 1, sweep[1]);
+  }
+  join_sweeps(sweep, knots);
+}
+
+void Model::integrate_sweep(const Particle& P, int dir, std::vector<double>& buf) const {
+  check_times(P);
+  buf.clear();
   const double dt = ((ctstop - ctstart) / kC / (npoints - 1));
+  Integrator I{fields, P.qomg};
+  double x[6] = {P.x0.x, P.b0.x * kC, P.x0.y, P.b0.y * kC, P.x0.z, P.b0.z * kC};
+  double dxdt[6] = {0, 0, 0, 0, 0, 0};
   if (traj_method == kRKAS) {  // src/OSCARSSR.cc:1015-1072
-    std::vector<double>& fwd = sweep[0];
-    std::vector<double>& bwd = sweep[1];
-    fwd.clear();
-    bwd.clear();
-    auto run = [&](int dir) {
-      Integrator I{fields, P.qomg};
-      Rkas R{I, dt, traj_precision};
-      double x[6] = {P.x0.x, P.b0.x * kC, P.x0.y, P.b0.y * kC, P.x0.z, P.b0.z * kC};
-      double dxdt[6] = {0, 0, 0, 0, 0, 0};
-      I.derivs(P.t0 / kC, x, dxdt);  // the reference evaluates it first (its value is not used)
-      R.propagate(x, P.t0 / kC, (dir == 0 ? ctstop : ctstart) / kC, dir == 0 ? fwd : bwd);
-    };
-    if (threads) {
-      parallel_tasks(2, run);
-    } else {
-      run(0);
-      run(1);
-    }
-    // forward reversed, backward appended, all reversed: the backward points earliest first, then the
-    // forward ones; both start at t0, so t0 appears twice (as in the reference)
-    const int64_t nf = (int64_t)fwd.size() / 10, nb = (int64_t)bwd.size() / 10, n = nf + nb;
-    if (n < 3)
-      throw Error{OSC_ERR_LENGTH, "TSpline1D3 does not see enough points for interpolation.  Please use >= 3 points"};
-    knots.n = n;
-    knots.t.resize(n);
-    knots.y.resize(9 * n);
-    for (int64_t j = 0; j < nb; ++j) {
-      const double* r = &bwd[10 * (nb - 1 - j)];
-      knots.t[j] = r[0];
-      for (int c = 0; c < 9; ++c) knots.y[c * n + j] = r[1 + c];
-    }
-    for (int64_t j = 0; j < nf; ++j) {
-      const double* r = &fwd[10 * j];
-      knots.t[nb + j] = r[0];
-      for (int c = 0; c < 9; ++c) knots.y[c * n + nb + j] = r[1 + c];
-    }
-    knots.tstart = knots.t.front();
-    knots.tstop = knots.t.back();
-    spline_second_derivatives(knots, threads);
+    Rkas R{I, dt, traj_precision};
+    I.derivs(P.t0 / kC, x, dxdt);  // the reference evaluates it first (its value is not used)
+    R.propagate(x, P.t0 / kC, (dir == 0 ? ctstop : ctstart) / kC, buf);
     return;
   }
-  const size_t nf = (size_t)(1 + (ctstop - P.t0) / kC / dt);
-  const size_t nb = (size_t)((P.t0 - ctstart) / kC / dt);
-
-  // The forward and backward sweeps are independent integrations from the same initial state; they
-  // run on two host threads and are stitched together afterwards (backward reversed, then forward).
-  std::vector<double>& fwd = sweep[0];
-  std::vector<double>& bwd = sweep[1];
-  fwd.clear();
-  bwd.clear();
-  fwd.reserve(10 * nf);
-  bwd.reserve(10 * nb);
-  auto forward = [&]() {
-    Integrator I{fields, P.qomg};
-    double x[6] = {P.x0.x, P.b0.x * kC, P.x0.y, P.b0.y * kC, P.x0.z, P.b0.z * kC};
-    double dxdt[6] = {0, 0, 0, 0, 0, 0};
+  if (dir == 0) {
+    const size_t nf = (size_t)(1 + (ctstop - P.t0) / kC / dt);
+    buf.reserve(10 * nf);
     I.derivs(P.t0 / kC, x, dxdt);
     for (size_t i = 0; i != nf; ++i) {
       const double t = P.t0 / kC + dt * i;
       if (i == 0) I.derivs(t, x, dxdt);
-      push_point(fwd, x, dxdt, t);
+      push_point(buf, x, dxdt, t);
       I.derivs(t, x, dxdt);
       I.step(x, dxdt, t, dt, x);
     }
-  };
-  auto backward = [&]() {
-    Integrator I{fields, P.qomg};
-    double x[6] = {P.x0.x, P.b0.x * kC, P.x0.y, P.b0.y * kC, P.x0.z, P.b0.z * kC};
-    double dxdt[6] = {0, 0, 0, 0, 0, 0};
+  } else {
+    const size_t nb = (size_t)((P.t0 - ctstart) / kC / dt);
+    buf.reserve(10 * nb);
     const double dtr = -dt;
     for (size_t i = 0; i != nb; ++i) {
       const double t1 = P.t0 / kC + dtr * (i);
       const double t2 = P.t0 / kC + dtr * (i + 1);
       I.derivs(t1, x, dxdt);
       I.step(x, dxdt, t1, dtr, x);
-      push_point(bwd, x, dxdt, t2);
+      push_point(buf, x, dxdt, t2);
     }
-  };
-  if (threads && nf + nb > 4096) {
-    parallel_tasks(2, [&](int i) {
-      if (i == 0) forward();
-      else backward();
-    });
-  } else {
-    forward();
-    backward();
   }
-  const int64_t n = (int64_t)(nf + nb);
-  if (n < 2) throw Error{OSC_ERR_LENGTH, "Not enough points in this trajectory"};
-  if (n < 3) throw Error{OSC_ERR_LENGTH, "TSpline1D3 does not see enough points for interpolation.  Please use >= 3 points"};
-  knots.n = n;
-  knots.t.resize(n);
-  knots.y.resize(9 * n);
-  for (int64_t j = 0; j < (int64_t)nb; ++j) {  // backward points, earliest first
-    const double* r = &bwd[10 * (nb - 1 - j)];
-    knots.t[j] = r[0];
-    for (int c = 0; c < 9; ++c) knots.y[c * n + j] = r[1 + c];
-  }
-  for (int64_t j = 0; j < (int64_t)nf; ++j) {
-    const double* r = &fwd[10 * j];
-    knots.t[nb + j] = r[0];
-    for (int c = 0; c < 9; ++c) knots.y[c * n + nb + j] = r[1 + c];
-  }
-  knots.tstart = knots.t.front();
-  knots.tstop = knots.t.back();
-  spline_second_derivatives(knots, threads);
 }
 
 void Model::set_trajectory(const double* traj, int64_t n) {
@@ -948,47 +891,84 @@ void Model::ensure_trajectory() {
 
 // ---------------------------------------------------------------------------------------------
 // Spline (include/TOMATH.h:141-203): the diagonal recurrence depends only on the knot times, so it
-// is shared by the 9 components; each component's right-hand side sweep runs on its own.
+// is shared by the 9 components.  Each component is two serial recurrences (a divide in each step of
+// the first), so the 9 go along one sweep as independent chains, in pairs of one SSE vector, and each
+// step's slope serves the next one too.  Every quotient is the one of a component alone.
+// get(i, y): knot i's time, and its 9 values in y; called once per knot, in order.
 // ---------------------------------------------------------------------------------------------
-void spline_second_derivatives(Knots& k, bool threads) {
+template <class Get>
+static void spline_pass(Knots& k, Get&& get) {
+  constexpr int W = 10;  // 9 components and one of zeros
   const int64_t N = k.n;
-  const double* X = k.t.data();
-  k.ypp.assign(9 * N, 0.0);
-  std::vector<double>& diag = k.diag;
-  diag.assign(N, 0.0);
-  if (k.work.size() < (size_t)(11 * N)) k.work.resize(11 * N);
-  double* sigv = k.work.data();
-  double* pv = sigv + N;
+  k.ypp.resize(9 * N);
+  k.diag.resize(N);
+  if (k.work.size() < (size_t)(W * N)) k.work.resize(W * N);
+  double *diag = k.diag.data(), *u = k.work.data(), *ypp = k.ypp.data();
+  double slope[W] = {}, uc[W] = {}, y[W] = {}, yn[W] = {};
+  double x_1 = get(0, y), x0 = get(1, yn);  // times of knots i - 1 and i
+  double dx = x0 - x_1;
+  for (int c = 0; c < W; ++c) {
+    slope[c] = (yn[c] - y[c]) / dx;
+    u[c] = uc[c] = (3. / dx) * (slope[c] - slope[c]);
+    y[c] = yn[c];
+  }
   diag[0] = -0.5;
   for (int64_t i = 1; i < N - 1; ++i) {
-    const double sig = (X[i] - X[i - 1]) / (X[i + 1] - X[i - 1]);
+    const double x1 = get(i + 1, yn);
+    const double span = x1 - x_1;
+    const double sig = dx / span;
     const double p = sig * diag[i - 1] + 2;
     diag[i] = (sig - 1.) / p;
-    sigv[i] = sig;
-    pv[i] = p;
-  }
-  auto component = [&](int c) {
-    const double* Y = k.y.data() + c * N;
-    double* ypp = k.ypp.data() + c * N;
-    double* u = k.work.data() + (2 + c) * N;
-    const double dydx0 = (Y[1] - Y[0]) / (X[1] - X[0]);
-    u[0] = (3. / (X[1] - X[0])) * ((Y[1] - Y[0]) / (X[1] - X[0]) - dydx0);
-    for (int64_t i = 1; i < N - 1; ++i) {
-      double ui = (Y[i + 1] - Y[i]) / (X[i + 1] - X[i]) - (Y[i] - Y[i - 1]) / (X[i] - X[i - 1]);
-      u[i] = (6. * ui / (X[i + 1] - X[i - 1]) - sigv[i] * u[i - 1]) / pv[i];
+    dx = x1 - x0;
+    x_1 = x0;
+    x0 = x1;
+    for (int c = 0; c < W; ++c) {
+      const double next = (yn[c] - y[c]) / dx;
+      const double ui = next - slope[c];
+      slope[c] = next;
+      y[c] = yn[c];
+      uc[c] = (6. * ui / span - sig * uc[c]) / p;
+      u[W * i + c] = uc[c];
     }
-    const double qn = 0.5;
-    const double dydxN = (Y[N - 1] - Y[N - 2]) / (X[N - 1] - X[N - 2]);
-    const double un = (3. / (X[N - 1] - X[N - 2])) * (dydxN - (Y[N - 1] - Y[N - 2]) / (X[N - 1] - X[N - 2]));
-    for (int64_t i = 0; i < N - 1; ++i) ypp[i] = diag[i];
-    ypp[N - 1] = (un - qn * u[N - 2]) / (qn * diag[N - 2] + 1.);
-    for (int64_t j = N - 2; j >= 0; --j) ypp[j] = ypp[j] * ypp[j + 1] + u[j];
-  };
-  if (threads && N > 4096) {
-    parallel_tasks(9, component);
-  } else {
-    for (int c = 0; c < 9; ++c) component(c);
   }
+  const double qn = 0.5;
+  for (int c = 0; c < W; ++c) {
+    const double un = (3. / dx) * (slope[c] - slope[c]);
+    uc[c] = (un - qn * uc[c]) / (qn * diag[N - 2] + 1.);
+  }
+  for (int c = 0; c < 9; ++c) ypp[c * N + N - 1] = uc[c];
+  diag[N - 1] = 0.0;
+  for (int64_t j = N - 2; j >= 0; --j) {
+    for (int c = 0; c < W; ++c) uc[c] = diag[j] * uc[c] + u[W * j + c];
+    for (int c = 0; c < 9; ++c) ypp[c * N + j] = uc[c];
+  }
+}
+
+void spline_second_derivatives(Knots& k) {
+  spline_pass(k, [&](int64_t i, double* y) {
+    for (int c = 0; c < 9; ++c) y[c] = k.y[c * k.n + i];
+    return k.t[i];
+  });
+}
+
+// Backward points earliest first, then the forward ones.  (RKAS sweeps both start at t0, so t0 appears twice, as
+// in the reference.)
+void Model::join_sweeps(const std::vector<double>* sweep, Knots& knots) const {
+  const std::vector<double>&fwd = sweep[0], &bwd = sweep[1];
+  const int64_t nf = (int64_t)fwd.size() / 10, nb = (int64_t)bwd.size() / 10, n = nf + nb;
+  if (n < 2 && traj_method == kRK4) throw Error{OSC_ERR_LENGTH, "Not enough points in this trajectory"};
+  if (n < 3) throw Error{OSC_ERR_LENGTH, "TSpline1D3 does not see enough points for interpolation.  Please use >= 3 points"};
+  knots.n = n;
+  knots.t.resize(n);
+  knots.y.resize(9 * n);
+  spline_pass(knots, [&](int64_t j, double* y) {
+    const double* r = j < nb ? &bwd[10 * (nb - 1 - j)] : &fwd[10 * (j - nb)];
+    knots.t[j] = r[0];
+    for (int c = 0; c < 9; ++c) y[c] = knots.y[c * n + j] = r[1 + c];
+    return r[0];
+  });
+  knots.tstart = knots.t.front();
+  knots.tstop = knots.t.back();
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -183,6 +183,10 @@ class Model {
   // several threads may integrate different particles at once (threads = false: no use of the host
   // task pool inside).
   void integrate(const Particle& P, Knots& out, std::vector<double>* sweep, bool threads) const;
+  // Its parts: one sweep (0 forward, 1 backward) of points into `buf`, and both sweeps' knots and spline.
+  void check_times(const Particle& P) const;
+  void integrate_sweep(const Particle& P, int dir, std::vector<double>& buf) const;
+  void join_sweeps(const std::vector<double>* sweep, Knots& out) const;
   // Select the method: "RK4" (precision must be -1, the binding's "not given") or "RKAS".
   void set_trajectory_calculation(const std::string& method, double precision);
   // Use a trajectory computed elsewhere (10 x n SoA: t, x y z, beta, a/c) with its spline.
@@ -190,9 +194,7 @@ class Model {
 };
 
 // Spline second derivatives of the 9 components (TSpline1D3::Derivatives, include/TOMATH.h:141-203).
-// `threads`: the 9 components on the host task pool (callers that are themselves worker threads pass
-// false).
-void spline_second_derivatives(Knots& k, bool threads = true);
+void spline_second_derivatives(Knots& k);
 
 // Runs fn(0) .. fn(n - 1) on a process-wide set of persistent host threads (the caller works too)
 // and returns when all have finished; the first exception a task throws is rethrown here.  Calls

@@ -201,3 +201,29 @@ def test_gradient_is_the_sum_over_observers(compute, tol, n_obs, n):
     whole = gradient(obs, weight)
     parts = sum(gradient([obs[k]], weight[k:k + 1]) for k in range(n_obs))
     assert np.max(np.abs(whole - parts)) <= tol * np.max(np.abs(whole))
+
+
+# A beam's trajectories come from host threads that share half trajectories and kept buffers: one particle, more
+# particles than slots, and the buffers again at other lengths, against one request per particle of the same
+# draw (weights and sums round to 1e-15 a particle).
+@pytest.mark.parametrize("method", ["RK4", "RKAS"])
+def test_beam_is_the_mean_of_its_particles(method):
+    kw = dict(energy_eV=E1_U, npoints=[3, 2], width=[0.004, 0.006], translation=[0, 0, 20], max_level=7, return_numpy=True)
+    o = sr(gpu=1)
+    o.add_bfield_undulator(bfield=[0, 0.5, 0], period=[0, 0, 0.05], nperiods=5)
+    o.set_particle_beam(type="electron", energy_GeV=3, x0=[0, 0, 0], d0=[0, 0, 1], current=0.5, sigma_energy_GeV=0.003,
+                        beta=[1.5, 0.8], alpha=[0, 0], emittance=[0.9e-9, 8e-12])
+    o.set_ctstartstop(-0.4, 0.4)
+    o.set_trajectory_calculation(method, **({} if method == "RK4" else {"precision": 1e-7}))
+    for n, points in ((1, 801), (44, 1201), (3, 401)):
+        o.set_npoints_trajectory(points)
+        o.set_seed(7)
+        whole = o.calculate_flux_rectangle(nparticles=n, **kw)[1]
+        o.set_seed(7)
+        mean = 0
+        for _ in range(n):
+            o.set_new_particle()
+            mean = mean + o.calculate_flux_rectangle(**kw)[1] / n
+        # (an RKAS trajectory holds its start time twice: its spline and results are NaN, on both sides)
+        assert np.isnan(mean).all() == (method == "RKAS")
+        np.testing.assert_allclose(whole, mean, rtol=0, atol=1e-13 * np.max(np.abs(np.nan_to_num(mean))))
