@@ -4,7 +4,7 @@
 // observer list at its own energies.  A multi-particle beam is a batch of jobs that share fields,
 // observers and energies and whose results are averaged (src/OSCARSSR.cc:4026-4062); a set of
 // uneven undulator jobs is a batch of unrelated jobs.  Per chunk of jobs every stage runs once over
-// all of them:
+// all of them, or, up to the prefilled level, once over each group of similar trajectory length:
 //   k_batch_rk4       FP64 RK4, one lane pair per (job, direction)        src/OSCARSSR.cc:910-1009
 //   k_batch_extent    trajectory extent in the job frame (validity bound of the mixed phase form)
 //   k_batch_spline    clamped cubic spline, one thread per (job, component) include/TOMATH.h:141-203
@@ -568,6 +568,7 @@ __global__ void k_batch_spline(const DevJob* __restrict__ jobs, int njobs, doubl
 // take the latency of the longest trajectory's recurrences (~1.6 us per point for both sweeps on
 // B200), the block-parallel ones the chunk's total work (~1.3 ns per point, all 9 components).  mode
 // 0 takes whichever the chunk's shape makes shorter, 1 the serial and 2 the block-parallel kernel.
+// n_max, n_total: of the whole chunk, also where only some of its jobs are solved here.
 void launch_batch_splines(const DevJob* d_jobs, int nj, int64_t n_max, int64_t n_total, double* knots, double* work,
                           int mode, cudaStream_t st) {
   const double serial_ms = 1.6e-3 * (double)n_max, parallel_ms = 1.3e-6 * (double)n_total;
@@ -1220,6 +1221,42 @@ int rk4_blocks(int nj) { return (2 * nj + rk4_per_warp(nj) - 1) / rk4_per_warp(n
 constexpr int kBatchPrefill = 13;        // levels enqueued without the host (records kept resident)
 constexpr int kBatchMinSpan = 128;
 constexpr int kBatchMaxJobsPerChunk = 8192;
+
+// A chunk's jobs in up to kBatchGroups groups of increasing trajectory length: a group's waves run while the longer
+// trajectories of the later ones are still being integrated (a serial chain that leaves the chip idle).
+// Sorts dj by chain length when there is more than one group; returns the groups' ends.
+// A further group costs ~0.1 ms a level of smaller launches and tails, 0.5 ms in all, so one is split off where its
+// first wave is at least as long (kGroupEntries x 1024 samples at 0.85e12 a second) and its chain at least
+// kGroupSteps shorter than the next group's (0.65 us a step).  32 jobs of 6000 to 51000 points and 3.4 million
+// entries: integration 17.8 ms, splines and records 4.5, waves 32; 54 ms one after another, 43 ms in four groups.
+constexpr int64_t kGroupEntries = 1 << 19;
+constexpr int kGroupSteps = 2000;
+std::vector<int> batch_groups(DevJob* dj, int nj) {
+  auto chain = [](const DevJob& d) { return std::max(d.nf, d.nb); };
+  std::vector<int> order(nj);
+  for (int k = 0; k < nj; ++k) order[k] = k;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return chain(dj[a]) < chain(dj[b]); });
+  int64_t N = 0, done = 0, in_group = 0;
+  for (int k = 0; k < nj; ++k) N += dj[k].n_obs * dj[k].n_e;
+  const int64_t share = std::max(kGroupEntries, (N + kBatchGroups - 1) / kBatchGroups);
+  std::vector<int> ends;
+  for (int k = 0; k + 1 < nj; ++k) {
+    const DevJob& d = dj[order[k]];
+    in_group += d.n_obs * d.n_e;
+    done += d.n_obs * d.n_e;
+    if (in_group < share || N - done < kGroupEntries) continue;
+    if (chain(dj[order[nj - 1]]) - chain(d) < kGroupSteps) break;
+    ends.push_back(k + 1);
+    in_group = 0;
+  }
+  ends.push_back(nj);
+  if (ends.size() > 1) {
+    std::vector<DevJob> sorted(nj);
+    for (int k = 0; k < nj; ++k) sorted[k] = dj[order[k]];
+    std::copy(sorted.begin(), sorted.end(), dj);
+  }
+  return ends;
+}
 }  // namespace
 
 DevField to_dev_field(FieldSpec f, std::vector<double>& vals) {
@@ -1338,6 +1375,19 @@ static std::vector<DevJob> build_dev_jobs(size_t n_fields, const std::vector<Bat
   }
 
   return dj;
+}
+
+// Streams and events of the trajectory groups of a batch, at the highest priority: the few warps of an integration
+// start before the waves that would fill the chip.
+void Engine::batch_streams() {
+  if (batch_fork_ev_) return;
+  int lo = 0, hi = 0;
+  check(cudaDeviceGetStreamPriorityRange(&lo, &hi), "priorities");
+  for (int g = 0; g < kBatchGroups; ++g) {
+    if (!batch_stream_[g]) check(cudaStreamCreateWithPriority(&batch_stream_[g], cudaStreamNonBlocking, hi), "cudaStreamCreate");
+    if (!batch_ev_[g]) check(cudaEventCreateWithFlags(&batch_ev_[g], cudaEventDisableTiming), "event");
+  }
+  check(cudaEventCreateWithFlags(&batch_fork_ev_, cudaEventDisableTiming), "event");
 }
 
 int Engine::batch_resident(int v) {
@@ -1459,6 +1509,9 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
       d.entry_begin = N;
       N += d.n_obs * d.n_e;
     }
+    const int64_t last_entry = dj[j1 - 1].entry_begin;
+    // (an average adds its jobs in their order)
+    const std::vector<int> groups = average ? std::vector<int>{nj} : batch_groups(dj.data() + j0, nj);
     // partial sums: spans = 1 gives 2 segments x N entries; a wave split into more spans has fewer
     // than 2 x target units of at most max_tile entries each (wave_spans)
     const bool any_lines = n_tiles > 0, any_entries = n_entry_jobs > 0;
@@ -1504,13 +1557,14 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
     plan.spans = reinterpret_cast<int*>(plan.act_start + (nj + 1));
 
     int cur = 0;  // active list / count array of the next wave
+    int g0 = 0, gn = nj;  // the jobs that the next wave goes over: [g0, g0 + gn)
     // The line jobs of a wave: their own plan, lists and counters (lists of wave `cur`, survivors to the others).
     auto line_wave = [&](int L, bool first, unsigned* cin, unsigned* cout, int64_t stride, int64_t s_off, const float4* rec) {
-      check(cudaMemsetAsync(ln_n[cur ^ 1], 0, sizeof(unsigned) * nj, st), "memset");
-      dev::k_batch_plan<true><<<1, 1024, 0, st>>>(d_jobs, nj, ln_n[cur], first, L, 1, 4 * (int64_t)line_grid, kBatchMinSpan,
-                                                  ln_plan);
+      check(cudaMemsetAsync(ln_n[cur ^ 1] + g0, 0, sizeof(unsigned) * gn, st), "memset");
+      dev::k_batch_plan<true><<<1, 1024, 0, st>>>(d_jobs + g0, gn, ln_n[cur] + g0, first, L, 1, 4 * (int64_t)line_grid,
+                                                  kBatchMinSpan, ln_plan);
       BatchLineArgs w{};
-      w.jobs = d_jobs; w.njobs = nj; w.rec = rec; w.stride = stride; w.s_off = s_off;
+      w.jobs = d_jobs + g0; w.njobs = gn; w.rec = rec; w.stride = stride; w.s_off = s_off;
       w.obs = b_obs_.as<double>(); w.omega = b_omega_.as<double>(); w.act = ln_act[cur];
       w.tiles = ln_tiles[cur]; w.tile_cnt = ln_cnt[cur]; w.plan = ln_plan; w.first = first; w.level = L;
       w.part = b_part_.as<double>(); w.err = misc; w.work = ln_work;
@@ -1519,7 +1573,7 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
       f.w = w; f.max_level = lstop; f.quantity = o.quantity; f.project = project; f.precision = o.precision;
       f.n_entries = N; f.state = b_state_.as<double>(); f.act_next = ln_act[cur ^ 1];
       f.entries_next = b_act_[cur ^ 1].as<int>();
-      f.tiles_next = ln_tiles[cur ^ 1]; f.tile_cnt_next = ln_cnt[cur ^ 1]; f.n_tiles_next = ln_n[cur ^ 1];
+      f.tiles_next = ln_tiles[cur ^ 1]; f.tile_cnt_next = ln_cnt[cur ^ 1]; f.n_tiles_next = ln_n[cur ^ 1] + g0;
       f.cnt_next = cout; f.out = b_out_.as<double>(); f.level_out = b_lvl_.as<int32_t>();
       f.not_converged = m64; f.samples = m64 + 1;
       dev::k_batch_line_finalize<<<sms * 8, dev::kLnFinTiles * dev::kLnTile, 0, st>>>(f);
@@ -1528,23 +1582,24 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
     };
     auto wave = [&](int L, int v, int64_t stride, int64_t s_off, const float4* rec) {
       const bool first = L == Lfirst;
-      unsigned* cin = cnts[cur];
-      unsigned* cout = cnts[cur ^ 1];
-      check(cudaMemsetAsync(cout, 0, sizeof(unsigned) * nj, st), "memset");
+      unsigned* cin = cnts[cur] + g0;
+      unsigned* cout = cnts[cur ^ 1] + g0;
+      rec += (int64_t)dev::kPairF4 * g0 * (stride >> 1);
+      check(cudaMemsetAsync(cout, 0, sizeof(unsigned) * gn, st), "memset");
       const int tile = batch_tile(v);
       if (any_lines) line_wave(L, first, cin, cout, stride, s_off, rec);
       if (first && !any_entries) {  // (later waves may have line jobs' last entries)
         cur ^= 1;
         return;
       }
-      dev::k_batch_plan<false><<<1, 1024, 0, st>>>(d_jobs, nj, cin, first, L, tile, target, kBatchMinSpan, plan);
+      dev::k_batch_plan<false><<<1, 1024, 0, st>>>(d_jobs + g0, gn, cin, first, L, tile, target, kBatchMinSpan, plan);
       BatchWaveArgs w{};
-      w.jobs = d_jobs; w.njobs = nj; w.rec = rec; w.stride = stride; w.s_off = s_off;
+      w.jobs = d_jobs + g0; w.njobs = gn; w.rec = rec; w.stride = stride; w.s_off = s_off;
       w.obs = b_obs_.as<double>(); w.omega = b_omega_.as<double>(); w.act = b_act_[cur].as<int>(); w.cnt = cin;
       w.plan = plan; w.first = first; w.level = L; w.part = b_part_.as<double>(); w.err = misc; w.work = m64 + 2;
       check(launch_batch_wave(w, batch_resident(v), v, st), "batch wave");
       BatchFinalArgs f{};
-      f.jobs = d_jobs; f.njobs = nj; f.act = w.act; f.cnt = cin; f.plan = plan; f.part = w.part;
+      f.jobs = d_jobs + g0; f.njobs = gn; f.act = w.act; f.cnt = cin; f.plan = plan; f.part = w.part;
       f.first = first; f.level = L; f.max_level = lstop; f.quantity = o.quantity; f.project = project;
       f.precision = o.precision; f.n_entries = N; f.state = b_state_.as<double>();
       f.act_next = b_act_[cur ^ 1].as<int>(); f.cnt_next = cout; f.out = b_out_.as<double>();
@@ -1554,24 +1609,51 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
       last_launches += 3;
       cur ^= 1;
     };
-    // trajectories, splines, the resident levels' records and the waves up to Lpre: no host sync
+    // trajectories, splines, the resident levels' records and the waves up to Lpre: no host sync.  With more than
+    // one group the trajectories go on streams of their own, all integrations from the start.
+    const int n_groups = (int)groups.size();
+    if (n_groups > 1) batch_streams();
     auto front = [&](int v, bool tune) {
       check(cudaMemsetAsync(misc, 0, 64, st), "memset");
       check(cudaMemsetAsync(ln_work, 0, sizeof(unsigned long long), st), "memset");
       if (!any_lines) check(cudaMemsetAsync(ln_n[0], 0, sizeof(unsigned) * 2 * nj, st), "memset");
-      dev::k_batch_rk4<<<rk4_blocks(nj), 32, 0, st>>>(d_jobs, nj, rk4_per_warp(nj), b_fields_.as<DevField>(),
-                                                          b_fvals_.as<double>(), b_knots_.as<double>(), misc);
-      dev::k_batch_extent<<<nj, 256, 0, st>>>(d_jobs, b_knots_.as<double>());
-      dev::launch_batch_splines(d_jobs, nj, n_max, n_total, b_knots_.as<double>(), b_work_.as<double>(), spline_kernel,
-                                st);
-      const int64_t fill_n = rec_per_job * nj;  // samples 0 .. 2^(Lpre+1) - 1 of every job
-      dev::k_batch_fill<<<(unsigned)((fill_n + 255) / 256), 256, 0, st>>>(
-          d_jobs, nj, b_knots_.as<double>(), nullptr, nullptr, b_rec_.as<float>(), rec_per_job, 0, 0, rec_per_job,
-          ext_from);
-      check(cudaGetLastError(), "batch trajectories");
-      last_launches += 4;
-      if (tune && any_entries) v = tune_batch(nj, Lfirst, target, d_jobs, plan, misc, m64, rec_per_job);
-      for (int L = Lfirst; L <= Lpre; ++L) wave(L, v, rec_per_job, 0, b_rec_.as<float4>());
+      if (n_groups > 1) check(cudaEventRecord(batch_fork_ev_, st), "record");
+      const int per_warp = rk4_per_warp(nj);
+      auto begin = [&](int g) { return g > 0 ? groups[g - 1] : 0; };
+      for (int g = 0; g < n_groups; ++g) {
+        const int b = begin(g), n = groups[g] - b;
+        cudaStream_t ts = n_groups > 1 ? batch_stream_[g] : st;
+        if (n_groups > 1) check(cudaStreamWaitEvent(ts, batch_fork_ev_, 0), "wait");
+        dev::k_batch_rk4<<<(2 * n + per_warp - 1) / per_warp, 32, 0, ts>>>(d_jobs + b, n, per_warp, b_fields_.as<DevField>(),
+                                                                           b_fvals_.as<double>(), b_knots_.as<double>(), misc);
+      }
+      for (int g = 0; g < n_groups; ++g) {
+        const int b = begin(g), n = groups[g] - b;
+        cudaStream_t ts = n_groups > 1 ? batch_stream_[g] : st;
+        dev::k_batch_extent<<<n, 256, 0, ts>>>(d_jobs + b, b_knots_.as<double>());
+        dev::launch_batch_splines(d_jobs + b, n, n_max, n_total, b_knots_.as<double>(), b_work_.as<double>(), spline_kernel,
+                                  ts);
+        const int64_t fill_n = rec_per_job * n;  // samples 0 .. 2^(Lpre+1) - 1 of every job
+        dev::k_batch_fill<<<(unsigned)((fill_n + 255) / 256), 256, 0, ts>>>(
+            d_jobs + b, n, b_knots_.as<double>(), nullptr, nullptr,
+            b_rec_.as<float>() + (int64_t)dev::kPairFloats * b * (rec_per_job >> 1), rec_per_job, 0, 0, rec_per_job, ext_from);
+        check(cudaGetLastError(), "batch trajectories");
+        if (n_groups > 1) check(cudaEventRecord(batch_ev_[g], ts), "record");
+        last_launches += 4;
+      }
+      if (tune && any_entries) {
+        for (int g = 0; g < n_groups && n_groups > 1; ++g) check(cudaStreamWaitEvent(st, batch_ev_[g], 0), "wait");
+        v = tune_batch(nj, Lfirst, target, d_jobs, plan, misc, m64, rec_per_job);
+      }
+      for (int g = 0; g < n_groups; ++g) {
+        if (n_groups > 1) check(cudaStreamWaitEvent(st, batch_ev_[g], 0), "wait");
+        g0 = begin(g);
+        gn = groups[g] - g0;
+        cur = 0;
+        for (int L = Lfirst; L <= Lpre; ++L) wave(L, v, rec_per_job, 0, b_rec_.as<float4>());
+      }
+      g0 = 0;
+      gn = nj;
       return v;
     };
     // a new shape is tuned and run eagerly; a known shape is captured and replayed as a graph
@@ -1647,7 +1729,7 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
       check(cudaGetLastError(), "batch average");
       ++last_launches;
       if (level_out && j1 == dj.size())  // levels of the last particle, as the reference leaves them
-        check(cudaMemcpyAsync(level_out, b_lvl_.as<int32_t>() + dj[j1 - 1].entry_begin, sizeof(int32_t) * m_avg,
+        check(cudaMemcpyAsync(level_out, b_lvl_.as<int32_t>() + last_entry, sizeof(int32_t) * m_avg,
                               cudaMemcpyDeviceToHost, st), "levels");
     } else {
       check(cudaMemcpyAsync(out + done_entries, b_out_.p, sizeof(double) * N, cudaMemcpyDeviceToHost, st), "download");

@@ -141,4 +141,7 @@ int batch_lines_blocks_per_sm();
 // Compiled variants of the batched wave kernel (groups per CTA, minimum CTAs per SM).
 constexpr int kBatchVariants = 4;
 
+// Groups of a batch's jobs whose trajectories are integrated side by side with the waves of shorter ones.
+constexpr int kBatchGroups = 4;
+
 }  // namespace osc

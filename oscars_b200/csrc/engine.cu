@@ -122,6 +122,11 @@ Engine::~Engine() {
   if (stream) cudaStreamDestroy(stream);
   if (aux_) cudaStreamDestroy(aux_);
   if (copy_) cudaStreamDestroy(copy_);
+  if (batch_fork_ev_) cudaEventDestroy(batch_fork_ev_);
+  for (int g = 0; g < kBatchGroups; ++g) {
+    if (batch_ev_[g]) cudaEventDestroy(batch_ev_[g]);
+    if (batch_stream_[g]) cudaStreamDestroy(batch_stream_[g]);
+  }
 }
 
 void Engine::check(cudaError_t e, const char* what) {

@@ -288,6 +288,9 @@ class Engine {
   // counter resets, while the request stream fills the level samples; the first wave waits for
   // in_ev_ (wait_inputs).
   cudaStream_t copy_ = nullptr;
+  cudaStream_t batch_stream_[kBatchGroups] = {};
+  cudaEvent_t batch_ev_[kBatchGroups] = {}, batch_fork_ev_ = nullptr;
+  void batch_streams();
   cudaEvent_t in_fork_ev_ = nullptr, in_ev_ = nullptr;
   bool inputs_pending_ = false;
   // observers / normals the waves read: the caller's device buffers, or their uploads

@@ -227,3 +227,24 @@ def test_beam_is_the_mean_of_its_particles(method):
         # (an RKAS trajectory holds its start time twice: its spline and results are NaN, on both sides)
         assert np.isnan(mean).all() == (method == "RKAS")
         np.testing.assert_allclose(whole, mean, rtol=0, atol=1e-13 * np.max(np.abs(np.nan_to_num(mean))))
+
+
+# Jobs of uneven trajectory length go in groups, sorted by it, whose waves overlap the longer integrations: against
+# each job alone (levels equal; the spans of its sums round in FP64 only).
+def test_batch_groups_match_single_jobs():
+    from oscars_b200.batch import BatchRunner, Job, undulator
+    def job(points, side, n, ct):
+        xs = np.linspace(-0.002, 0.002, side)
+        return Job(fields=[undulator([0, 0.6, 0], [0, 0, 0.04], 8)], energy_GeV=3, ctstartstop=(-ct, ct), npoints=points,
+                   obs=[[x, y, 20.0] for x in xs for y in xs], energies_eV=np.linspace(300, 900, n), current=0.5)
+    jobs = [job(9001, 40, 340, 0.5), job(12001, 3, 20, 0.6), job(3001, 41, 330, 0.4), job(10001, 2, 5, 0.5)]
+    kw = dict(compute="mixed", max_level=11)
+    r = BatchRunner(gpu=0)
+    for _ in range(2):  # the second call replays the captured graph
+        whole = r.flux(jobs, **kw)
+        levels = [x.copy() for x in r.last_levels]
+        for k, j in enumerate(jobs):
+            one = BatchRunner(gpu=0)
+            alone = one.flux([j], **kw)[0]
+            assert np.array_equal(levels[k], one.last_levels[0])
+            assert np.max(np.abs(whole[k] - alone)) <= 1e-12 * np.max(np.abs(alone))
