@@ -17,8 +17,8 @@
 //   k_adj_spline_solve  second derivatives -> knot values (transpose of the tridiagonal sweeps)
 //   k_adj_rk4_recompute trajectory states recomputed from checkpoints every 256 steps
 //   k_adj_rk4_segments  knots -> RK4 states -> field amplitudes, parallel in time: every 64-step
-//                       segment of both integration chains runs its reverse pass at once (each
-//                       step's stages recomputed and differentiated), once with the knot adjoints and
+//                       segment of both integration chains runs its reverse pass at once (all its
+//                       steps' stages linearised side by side first), once with the knot adjoints and
 //                       once per unit adjoint entering it;
 //   k_adj_rk4_lam       a sequential sweep of the 6 x 6 segment Jacobians joins the segments
 //   k_adj_rk4_pgrad     the parameter gradients of the unit-adjoint passes, weighted by it.
@@ -65,16 +65,19 @@ __global__ void k_adj_weights(const double* __restrict__ S, int64_t n, const dou
                               double c0dt, double c2, double* __restrict__ W,
                               unsigned long long* __restrict__ wmax_bits) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  const double w = 2.0 * c2 * c0dt * c0dt * grad_flux[e];
   double mx = 0;
-  for (int k = 0; k < 3; ++k) {
-    const double re = w * S[6 * e + 2 * k], im = -w * S[6 * e + 2 * k + 1];  // conj(S)
-    W[6 * e + 2 * k] = re;
-    W[6 * e + 2 * k + 1] = im;
-    mx = fmax(mx, fmax(fabs(re), fabs(im)));
+  if (e < n) {
+    const double w = 2.0 * c2 * c0dt * c0dt * grad_flux[e];
+    for (int k = 0; k < 3; ++k) {
+      const double re = w * S[6 * e + 2 * k], im = -w * S[6 * e + 2 * k + 1];  // conj(S)
+      W[6 * e + 2 * k] = re;
+      W[6 * e + 2 * k + 1] = im;
+      mx = fmax(mx, fmax(fabs(re), fabs(im)));
+    }
   }
-  if (mx > 0) atomicMax(wmax_bits, (unsigned long long)__double_as_longlong(mx));
+  // one atomic per warp: 113000 entries' own ones on the one word took 77 us, 5 us this way
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0 && mx > 0) atomicMax(wmax_bits, (unsigned long long)__double_as_longlong(mx));
 }
 
 // ---- 2. per-sample gradients --------------------------------------------------------------
@@ -424,36 +427,50 @@ __device__ __forceinline__ Affine compose(Affine first, Affine then) {  // then(
 }
 
 // x_k = A(k) x_{k-1} + B(k) for k = 0 .. m-1 (x_{-1} = 0), in index order k or (reverse) m-1-k;
-// A(k), B(k) are callables of the recurrence index, `out(k, x)` receives every x_k.
+// A(k), B(k) are callables of the recurrence index, `out(k, x)` receives every x_k.  Tiles of 4 neighbouring elements a
+// thread, evaluated once and read in whole sectors, the value entering a tile carried (20001 points, both
+// recurrences and the gather: 178 us with one run of 20 elements a thread, evaluated twice, 92 us this way).
 template <class FA, class FB, class FO>
 __device__ void block_linear_scan(int64_t m, FA A, FB B, FO out) {
-  __shared__ double sa[kScanThreads], sb[kScanThreads];
-  const int t = threadIdx.x;
-  const int64_t chunk = (m + kScanThreads - 1) / kScanThreads;
-  const int64_t k0 = t * chunk, k1 = min(m, k0 + chunk);
-  Affine f{1.0, 0.0};
-  for (int64_t k = k0; k < k1; ++k) f = compose(f, Affine{A(k), B(k)});
-  sa[t] = f.a;
-  sb[t] = f.b;
-  __syncthreads();
-  for (int o = 1; o < kScanThreads; o <<= 1) {  // inclusive scan of the chunk maps
-    Affine prev{1.0, 0.0};
-    if (t >= o) prev = Affine{sa[t - o], sb[t - o]};
-    __syncthreads();
-    if (t >= o) {
-      const Affine cur = compose(prev, Affine{sa[t], sb[t]});
-      sa[t] = cur.a;
-      sb[t] = cur.b;
+  constexpr int E = 4;  // neighbouring elements of a thread
+  __shared__ Affine totals[kScanThreads / 32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const unsigned full = 0xffffffffu;
+  auto warp_scan = [&](Affine s) {  // inclusive
+    for (int o = 1; o < 32; o <<= 1) {
+      const Affine prev{__shfl_up_sync(full, s.a, o), __shfl_up_sync(full, s.b, o)};
+      if (lane >= o) s = compose(prev, s);
     }
+    return s;
+  };
+  double carry = 0;  // x entering the tile
+  for (int64_t base = 0; base < m; base += kScanThreads * E) {
+    const int64_t k0 = base + t * E;
+    Affine f[E], own{1.0, 0.0};
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      f[e] = k0 + e < m ? Affine{A(k0 + e), B(k0 + e)} : Affine{1.0, 0.0};
+      own = compose(own, f[e]);
+    }
+    const Affine in_warp = warp_scan(own);
+    if (lane == 31) totals[warp] = in_warp;
+    __syncthreads();
+    const Affine warps = warp_scan(totals[lane]);
+    const Affine all{__shfl_sync(full, warps.a, 31), __shfl_sync(full, warps.b, 31)};
+    const Affine before{__shfl_sync(full, warps.a, (warp + 31) & 31), __shfl_sync(full, warps.b, (warp + 31) & 31)};
+    const Affine lower{__shfl_up_sync(full, in_warp.a, 1), __shfl_up_sync(full, in_warp.b, 1)};
+    double x = warp > 0 ? before.a * carry + before.b : carry;
+    if (lane > 0) x = lower.a * x + lower.b;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      if (k0 + e < m) {
+        x = f[e].a * x + f[e].b;
+        out(k0 + e, x);
+      }
+    }
+    carry = all.a * carry + all.b;
     __syncthreads();
   }
-  double x = t > 0 ? sb[t - 1] : 0.0;  // value entering this chunk (x_{-1} = 0)
-  __syncthreads();
-  for (int64_t k = k0; k < k1; ++k) {
-    x = A(k) * x + B(k);
-    out(k, x);
-  }
-  __syncthreads();
 }
 
 // One block per component; pbar (adjoint of ypp) is overwritten, ybar accumulates; work: n doubles
@@ -510,11 +527,15 @@ struct AdjFields {
   double* pbar;      // gradient of the parameters (n_half of the parameter field)
 };
 
-// Field value at a point, and, when Bb != nullptr, the vector-Jacobian products of B with respect to
-// the position (added to posb) and to the parameter field's half-period factors (added to pbar).
-__device__ void field_vjp(const AdjFields& F, double x, double y, double z, double t, double* B, const double* Bb,
-                          double* posb) {
+// The fields at a point: B, and with LIN what a reverse step needs of them there, so that it evaluates none itself:
+// rec: B (3), dB_b/dx_c (9, row b), the velocity (3, the caller's), and for the pole blocks of the field with
+// half-period factors the factor's coefficient (2) and index (2 ints, -1: none).
+constexpr int kSegRec = 18;
+template <bool LIN>
+__device__ __forceinline__ void field_lin(const AdjFields& F, double x, double y, double z, double t, double* B, double* rec) {
   B[0] = B[1] = B[2] = 0;
+  double G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, co[2] = {0, 0};
+  int idx[2] = {-1, -1};
   for (int i = 0; i < F.nf; ++i) {
     const DevField& f = F.fs[i];
     const double d = (x - f.center[0]) * f.period_unit[0] + (y - f.center[1]) * f.period_unit[1] +
@@ -529,7 +550,7 @@ __device__ void field_vjp(const AdjFields& F, double x, double y, double z, doub
       const double L = f.length, lam = f.period_length;
       if (d > L / 2. + shift || d < -L / 2. + shift) continue;
       const double th = 2.0 * kPiD * (d - shift) / lam;
-      const double s = sin(th), c = cos(th);
+      const double s = sin(th);
       double kf = 1.0;
       int64_t hk = -1;
       if (d < -L / 2. + shift + lam || d > L / 2. + shift - lam) {
@@ -543,21 +564,40 @@ __device__ void field_vjp(const AdjFields& F, double x, double y, double z, doub
       B[0] += amp[0] * phi * w;
       B[1] += amp[1] * phi * w;
       B[2] += amp[2] * phi * w;
-      if (Bb) {
-        const double gA = (Bb[0] * amp[0] + Bb[1] * amp[1] + Bb[2] * amp[2]) * w;
-        const double dphi = kf * (c * (2.0 * kPiD / lam) * tc + s * f.taper);
-        posb[0] += gA * dphi * f.period_unit[0];
-        posb[1] += gA * dphi * f.period_unit[1];
-        posb[2] += gA * dphi * f.period_unit[2];
-        if (hk >= 0 && i == F.param_field) atomicAdd(&F.pbar[hk], gA * s * tc);
+      if (LIN) {
+        const double dphi = kf * (cos(th) * (2.0 * kPiD / lam) * tc + s * f.taper);
+#pragma unroll
+        for (int b = 0; b < 3; ++b)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) G[3 * b + c] += amp[b] * w * dphi * f.period_unit[c];
+        if (hk >= 0 && i == F.param_field) {
+          co[blk] = w * (s * tc);
+          idx[blk] = (int)hk;
+        }
       }
     }
   }
+  if (LIN) {
+#pragma unroll
+    for (int b = 0; b < 3; ++b) rec[b] = B[b];
+#pragma unroll
+    for (int c = 0; c < 9; ++c) rec[3 + c] = G[c];
+    rec[15] = co[0];
+    rec[16] = co[1];
+    reinterpret_cast<int*>(rec + 17)[0] = idx[0];
+    reinterpret_cast<int*>(rec + 17)[1] = idx[1];
+  }
 }
 
-__device__ void f_eval(const AdjFields& F, double t, const double* y, double* dy) {
+template <bool LIN>
+__device__ __forceinline__ void f_eval(const AdjFields& F, double t, const double* y, double* dy, double* rec) {
   double B[3];
-  field_vjp(F, y[0], y[2], y[4], t, B, nullptr, nullptr);
+  field_lin<LIN>(F, y[0], y[2], y[4], t, B, rec);
+  if (LIN) {
+    rec[12] = y[1];
+    rec[13] = y[3];
+    rec[14] = y[5];
+  }
   dy[0] = y[1];
   dy[1] = F.qomg * (-y[5] * B[1] + y[3] * B[2]);
   dy[2] = y[3];
@@ -566,59 +606,78 @@ __device__ void f_eval(const AdjFields& F, double t, const double* y, double* dy
   dy[5] = F.qomg * (y[1] * B[1] - y[3] * B[0]);
 }
 
-// yb += (df/dy)^T fb at (t, y); parameter gradient accumulated by field_vjp.
-__device__ void f_vjp(const AdjFields& F, double t, const double* y, const double* fb, double* yb) {
-  const double vx = y[1], vy = y[3], vz = y[5];
-  double B[3];
-  const double Bb[3] = {F.qomg * (fb[3] * vz - fb[5] * vy), F.qomg * (-fb[1] * vz + fb[5] * vx),
-                        F.qomg * (fb[1] * vy - fb[3] * vx)};
-  double posb[3] = {0, 0, 0};
-  field_vjp(F, y[0], y[2], y[4], t, B, Bb, posb);
-  yb[0] += posb[0];
-  yb[2] += posb[1];
-  yb[4] += posb[2];
-  yb[1] += fb[0] + F.qomg * (-fb[3] * B[2] + fb[5] * B[1]);
-  yb[3] += fb[2] + F.qomg * (fb[1] * B[2] - fb[5] * B[0]);
-  yb[5] += fb[4] + F.qomg * (-fb[1] * B[1] + fb[3] * B[0]);
+// The parameter gradient of one reverse pass: neighbouring steps share their half-period, whose sum goes out when
+// the index changes.
+struct ParamSum {
+  double* out;
+  double amp[2][3], sum[2];
+  int at[2];
+  __device__ __forceinline__ void flush(int b) {
+    if (at[b] >= 0) atomicAdd(&out[at[b]], sum[b]);
+  }
+  __device__ __forceinline__ void add(int b, int k, double v) {
+    if (k != at[b]) {
+      flush(b);
+      at[b] = k;
+      sum[b] = 0;
+    }
+    sum[b] += v;
+  }
+};
+
+// yb += (df/dy)^T fb at the point of record R; parameter gradient to P.
+__device__ __forceinline__ void f_vjp(double qomg, const double* R, const double* fb, double* yb, ParamSum& P) {
+  const double vx = R[12], vy = R[13], vz = R[14];
+  const double Bb[3] = {qomg * (fb[3] * vz - fb[5] * vy), qomg * (-fb[1] * vz + fb[5] * vx),
+                        qomg * (fb[1] * vy - fb[3] * vx)};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) yb[2 * c] += Bb[0] * R[3 + c] + Bb[1] * R[6 + c] + Bb[2] * R[9 + c];
+  yb[1] += fb[0] + qomg * (-fb[3] * R[2] + fb[5] * R[1]);
+  yb[3] += fb[2] + qomg * (fb[1] * R[2] - fb[5] * R[0]);
+  yb[5] += fb[4] + qomg * (-fb[1] * R[1] + fb[3] * R[0]);
+#pragma unroll
+  for (int b = 0; b < 2; ++b) {
+    const int k = reinterpret_cast<const int*>(R + 17)[b];
+    if (k >= 0) P.add(b, k, (Bb[0] * P.amp[b][0] + Bb[1] * P.amp[b][1] + Bb[2] * P.amp[b][2]) * R[15 + b]);
+  }
 }
 
 __device__ void rk4_step(const AdjFields& F, double* y, double t, double h) {
   double k1[6], k2[6], k3[6], k4[6], yt[6];
-  f_eval(F, t, y, k1);
+  f_eval<false>(F, t, y, k1, nullptr);
   for (int i = 0; i < 6; ++i) yt[i] = y[i] + h * 0.5 * k1[i];
-  f_eval(F, t + h * 0.5, yt, k2);
+  f_eval<false>(F, t + h * 0.5, yt, k2, nullptr);
   for (int i = 0; i < 6; ++i) yt[i] = y[i] + h * 0.5 * k2[i];
-  f_eval(F, t + h * 0.5, yt, k3);
+  f_eval<false>(F, t + h * 0.5, yt, k3, nullptr);
   for (int i = 0; i < 6; ++i) yt[i] = y[i] + h * k3[i];
-  f_eval(F, t + h, yt, k4);
+  f_eval<false>(F, t + h, yt, k4, nullptr);
   for (int i = 0; i < 6; ++i) y[i] = y[i] + h / 6.0 * (k1[i] + k4[i] + 2.0 * (k2[i] + k3[i]));
 }
 
-// lam (adjoint of the step's output) -> adjoint of its input y (returned in lam).
-__device__ void rk4_vjp(const AdjFields& F, const double* y, double t, double h, double* lam) {
-  double k1[6], k2[6], k3[6], y2[6], y3[6], y4[6];
-  f_eval(F, t, y, k1);
-  for (int i = 0; i < 6; ++i) y2[i] = y[i] + h * 0.5 * k1[i];
-  f_eval(F, t + h * 0.5, y2, k2);
-  for (int i = 0; i < 6; ++i) y3[i] = y[i] + h * 0.5 * k2[i];
-  f_eval(F, t + h * 0.5, y3, k3);
-  for (int i = 0; i < 6; ++i) y4[i] = y[i] + h * k3[i];
-  double yb[6], k1b[6], k2b[6], k3b[6], k4b[6], tmp[6];
-  for (int i = 0; i < 6; ++i) {
-    yb[i] = lam[i];
-    k1b[i] = h / 6.0 * lam[i];
-    k2b[i] = h / 3.0 * lam[i];
-    k3b[i] = h / 3.0 * lam[i];
-    k4b[i] = h / 6.0 * lam[i];
+// Records of the four stages of the step from y; only the first one's with `last` (the chain ends there).
+__device__ void rk4_records(const AdjFields& F, const double* y, double t, double h, bool last, double (*rec)[kSegRec]) {
+  double k[6], yt[6];
+#pragma unroll 1
+  for (int s = 0; s < 4; ++s) {
+    const double c = s == 0 ? 0.0 : (s == 3 ? h : h * 0.5);
+    for (int i = 0; i < 6; ++i) yt[i] = s == 0 ? y[i] : y[i] + c * k[i];
+    f_eval<true>(F, t + c, yt, k, rec[s]);
+    if (last) break;
   }
-  for (int i = 0; i < 6; ++i) tmp[i] = 0;
-  f_vjp(F, t + h, y4, k4b, tmp);
-  for (int i = 0; i < 6; ++i) { yb[i] += tmp[i]; k3b[i] += h * tmp[i]; tmp[i] = 0; }
-  f_vjp(F, t + h * 0.5, y3, k3b, tmp);
-  for (int i = 0; i < 6; ++i) { yb[i] += tmp[i]; k2b[i] += h * 0.5 * tmp[i]; tmp[i] = 0; }
-  f_vjp(F, t + h * 0.5, y2, k2b, tmp);
-  for (int i = 0; i < 6; ++i) { yb[i] += tmp[i]; k1b[i] += h * 0.5 * tmp[i]; tmp[i] = 0; }
-  f_vjp(F, t, y, k1b, tmp);
+}
+
+// lam (adjoint of a step's output) -> adjoint of its input (returned in lam).
+__device__ __forceinline__ void rk4_vjp(double qomg, const double (*rec)[kSegRec], double h, double* lam, ParamSum& P) {
+  const double h6 = h / 6.0, h3 = h / 3.0, hh = h * 0.5;
+  double yb[6], kb[6], tmp[6];
+  for (int i = 0; i < 6; ++i) { yb[i] = lam[i]; kb[i] = h6 * lam[i]; tmp[i] = 0; }
+  f_vjp(qomg, rec[3], kb, tmp, P);
+  for (int i = 0; i < 6; ++i) { yb[i] += tmp[i]; kb[i] = h3 * lam[i] + h * tmp[i]; tmp[i] = 0; }
+  f_vjp(qomg, rec[2], kb, tmp, P);
+  for (int i = 0; i < 6; ++i) { yb[i] += tmp[i]; kb[i] = h3 * lam[i] + hh * tmp[i]; tmp[i] = 0; }
+  f_vjp(qomg, rec[1], kb, tmp, P);
+  for (int i = 0; i < 6; ++i) { yb[i] += tmp[i]; kb[i] = h6 * lam[i] + hh * tmp[i]; tmp[i] = 0; }
+  f_vjp(qomg, rec[0], kb, tmp, P);
   for (int i = 0; i < 6; ++i) lam[i] = yb[i] + tmp[i];
 }
 
@@ -684,23 +743,17 @@ __global__ void k_adj_rk4_recompute(AdjFields F, AdjSegs S, double* __restrict__
   }
 }
 
-// Knot state / acceleration adjoints in the RK4 state layout.
-__device__ __forceinline__ void knot_state_adj(const double* kb, int64_t n, int64_t j, double* lam) {
-  lam[0] += kb[j]; lam[2] += kb[n + j]; lam[4] += kb[2 * n + j];
-  lam[1] += kb[3 * n + j] / kCLight; lam[3] += kb[4 * n + j] / kCLight; lam[5] += kb[5 * n + j] / kCLight;
-}
-__device__ __forceinline__ void knot_accel_adj(const double* kb, int64_t n, int64_t j, double* fb) {
-  fb[0] = 0; fb[2] = 0; fb[4] = 0;
-  fb[1] = kb[6 * n + j] / kCLight; fb[3] = kb[7 * n + j] / kCLight; fb[5] = kb[8 * n + j] / kCLight;
-}
-
-// One block per segment; thread 0 runs the segment's reverse pass with the knot adjoints and zero
-// adjoint entering (its parameter gradient goes straight to the result), threads 1..6 run it with the
-// unit adjoint e_{r-1} entering and no knot adjoints (the columns of the segment's transposed
-// Jacobian and parameter sensitivities, combined by k_adj_rk4_lam and k_adj_rk4_pgrad).
-__global__ void __launch_bounds__(32) k_adj_rk4_segments(AdjFields F, AdjSegs S) {
-  const int r = threadIdx.x;
-  if (r > 6) return;
+// One block per segment.  Its states are known, so a thread per state first forms its stages' records and fetches its
+// knots' adjoints; the reverse passes then are a chain of ~40 FP64 operations a step without a field evaluation
+// (they made seven each, 17000 cycles a step).  Warp 1's first thread runs the pass with the knot adjoints and zero
+// adjoint entering (its parameter gradient goes straight to the result), warp 0's first six run it with the
+// unit adjoints entering and no knot adjoints (the columns of the segment's transposed Jacobian and
+// parameter sensitivities, combined by k_adj_rk4_lam and k_adj_rk4_pgrad).
+// 20001 points: 568 -> 73 us.
+constexpr int kSegThreads = 96;  // a state each, 0 .. kSegSteps
+__global__ void __launch_bounds__(kSegThreads) k_adj_rk4_segments(AdjFields F, AdjSegs S) {
+  __shared__ double rec[kSegSteps + 1][4][kSegRec];
+  __shared__ double knot[kSegSteps + 1][9];  // per state: adjoints of x, beta (RK4 order) and of the acceleration
   const int64_t g = blockIdx.x;
   const int dir = g < S.base[1] ? 0 : 1;
   const int64_t m = g - S.base[dir];
@@ -709,33 +762,48 @@ __global__ void __launch_bounds__(32) k_adj_rk4_segments(AdjFields F, AdjSegs S)
   const int64_t M = dir == 0 ? (int64_t)S.nf - 1 : (int64_t)S.nb;
   const int64_t s0 = m * kSegSteps, s1 = min(M, s0 + kSegSteps);
   const int64_t lo = m == 0 ? 0 : s0 + 1;
-  AdjFields Fr = F;
-  if (r > 0) Fr.pbar = S.pseg + (g * 6 + (r - 1)) * S.n_params;
-  double lam[6] = {0, 0, 0, 0, 0, 0};
-  if (r > 0) lam[r - 1] = 1.0;
-  double zi[6], zp[6];
-  for (int64_t i = s1; i >= lo; --i) {
-    seg_state(S, dir, i, zi);
-    if (r == 0) {
-      const int64_t sk = dir == 0 ? S.nb + i : (i >= 1 ? S.nb - i : -1);
-      if (sk >= 0) knot_state_adj(S.kb, n, sk, lam);
-      const int64_t ak = dir == 0 ? (i + 1 <= (int64_t)S.nf - 1 ? S.nb + i + 1 : -1)
-                                  : (i <= (int64_t)S.nb - 1 ? S.nb - 1 - i : -1);
-      double fb[6];
-      if (ak >= 0) {
-        knot_accel_adj(S.kb, n, ak, fb);
-        f_vjp(Fr, S.t0 + h * (double)i, zi, fb, lam);
-      }
-      if (dir == 0 && i == 0) {  // knot nb also holds f(t_0, z_0)
-        knot_accel_adj(S.kb, n, S.nb, fb);
-        f_vjp(Fr, S.t0, zi, fb, lam);
-      }
-    }
-    if (i > 0) {
-      seg_state(S, dir, i - 1, zp);
-      rk4_vjp(Fr, zp, S.t0 + h * (double)(i - 1), h, lam);
+  if (threadIdx.x <= s1 - s0) {
+    const int k = threadIdx.x;
+    const int64_t i = s0 + k;
+    double z[6];
+    seg_state(S, dir, i, z);
+    rk4_records(F, z, S.t0 + h * (double)i, h, i == s1, rec[k]);
+    const int64_t sk = dir == 0 ? S.nb + i : (i >= 1 ? S.nb - i : -1);  // the knot of state i
+    const int64_t ak = dir == 0 ? (i + 1 <= (int64_t)S.nf - 1 ? S.nb + i + 1 : -1)
+                                : (i <= (int64_t)S.nb - 1 ? S.nb - 1 - i : -1);  // the knot that holds f(t_i, z_i)
+    for (int c = 0; c < 3; ++c) {
+      knot[k][2 * c] = sk >= 0 ? S.kb[c * n + sk] : 0.0;
+      knot[k][2 * c + 1] = sk >= 0 ? S.kb[(3 + c) * n + sk] / kCLight : 0.0;
+      double a = ak >= 0 ? S.kb[(6 + c) * n + ak] / kCLight : 0.0;
+      if (dir == 0 && i == 0) a += S.kb[(6 + c) * n + S.nb] / kCLight;  // knot nb also holds f(t_0, z_0)
+      knot[k][6 + c] = a;
     }
   }
+  __syncthreads();
+  const int r = threadIdx.x == 32 ? 0 : threadIdx.x + 1;
+  if (threadIdx.x > 5 && r > 0) return;
+  ParamSum P;
+  P.out = r > 0 ? S.pseg + (g * 6 + (r - 1)) * S.n_params : F.pbar;
+  for (int b = 0; b < 2; ++b) {
+    P.at[b] = -1;
+    P.sum[b] = 0;
+    for (int c = 0; c < 3; ++c) P.amp[b][c] = F.param_field < 0 ? 0.0 : (b == 0 ? F.fs[F.param_field].a[c] : F.fs[F.param_field].b[c]);
+  }
+  double lam[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+  for (int k = 0; k < 6; ++k)
+    if (r == k + 1) lam[k] = 1.0;
+  for (int64_t i = s1; i >= lo; --i) {
+    const int k = (int)(i - s0);
+    if (r == 0) {
+      for (int c = 0; c < 6; ++c) lam[c] += knot[k][c];
+      const double fb[6] = {0, knot[k][6], 0, knot[k][7], 0, knot[k][8]};
+      f_vjp(F.qomg, rec[k][0], fb, lam, P);
+    }
+    if (i > 0) rk4_vjp(F.qomg, rec[k - 1], h, lam, P);
+  }
+  P.flush(0);
+  P.flush(1);
   if (r == 0) {
     for (int k = 0; k < 6; ++k) S.lam_loc[g * 6 + k] = lam[k];
   } else {
@@ -746,32 +814,32 @@ __global__ void __launch_bounds__(32) k_adj_rk4_segments(AdjFields F, AdjSegs S)
 // The adjoint entering every segment: a sequential sweep over the segments of each chain (block 0:
 // forward chain, block 1: backward chain), the adjoint entering segment m being the one leaving
 // segment m + 1 (lam_loc + J^T lam).  The segments' transposed Jacobians are staged through shared
-// memory a chunk at a time; one thread runs the 6 x 6 recurrence.
+// memory a chunk at a time; six lanes, a component each, run the 6 x 6 recurrence (157 segments a chain: one
+// thread 48 us, six lanes 25 us).
 constexpr int kLamChunk = 128;
 __global__ void __launch_bounds__(128) k_adj_rk4_lam(AdjSegs S, double* __restrict__ lam_in) {
   __shared__ double sj[kLamChunk][42];  // per segment: J^T e_r (36), lam_loc (6)
   const int d = blockIdx.x;
-  double lam[6] = {0, 0, 0, 0, 0, 0};
+  const int jj = threadIdx.x < 6 ? threadIdx.x : 0;
+  double lam = 0;
   for (int64_t hi = S.nseg[d]; hi > 0; hi -= kLamChunk) {
     const int64_t lo = hi > kLamChunk ? hi - kLamChunk : 0;
-    for (int64_t idx = threadIdx.x; idx < (hi - lo) * 42; idx += blockDim.x) {
-      const int64_t g = S.base[d] + lo + idx / 42;
-      const int k = (int)(idx % 42);
-      sj[idx / 42][k] = k < 36 ? S.jt[g * 36 + k] : S.lam_loc[g * 6 + (k - 36)];
-    }
+    const double *jt = S.jt + 36 * (S.base[d] + lo), *loc = S.lam_loc + 6 * (S.base[d] + lo);
+    const int cnt = (int)(hi - lo);
+#pragma unroll 8
+    for (int idx = threadIdx.x; idx < cnt * 36; idx += 128) sj[idx / 36][idx % 36] = jt[idx];
+#pragma unroll 4
+    for (int idx = threadIdx.x; idx < cnt * 6; idx += 128) sj[idx / 6][36 + idx % 6] = loc[idx];
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
+#pragma unroll 2
       for (int64_t m = hi - 1; m >= lo; --m) {
         const double* J = sj[m - lo];
-        double* out = lam_in + 6 * (S.base[d] + m);
-        double nl[6];
-        for (int jj = 0; jj < 6; ++jj) {
-          out[jj] = lam[jj];
-          double v = J[36 + jj];
-          for (int r = 0; r < 6; ++r) v = fma(J[r * 6 + jj], lam[r], v);
-          nl[jj] = v;
-        }
-        for (int jj = 0; jj < 6; ++jj) lam[jj] = nl[jj];
+        if (threadIdx.x < 6) lam_in[6 * (S.base[d] + m) + jj] = lam;
+        double v = J[36 + jj];
+#pragma unroll
+        for (int r = 0; r < 6; ++r) v = fma(J[r * 6 + jj], __shfl_sync(0xffffffffu, lam, r), v);
+        lam = v;
       }
     }
     __syncthreads();
@@ -779,9 +847,11 @@ __global__ void __launch_bounds__(128) k_adj_rk4_lam(AdjSegs S, double* __restri
 }
 
 // Parameter gradient of the unit-adjoint passes: pbar[k] += sum over segments g and r of
-// lam_in[g][r] * pseg[g][r][k], a block per chunk of 32 segments, a thread per parameter.
+// lam_in[g][r] * pseg[g][r][k], a block per chunk of kPgradSegs segments, a thread per parameter (314 segments: in
+// chunks of 32 41 us, of 4 8 us).
+constexpr int kPgradSegs = 4;
 __global__ void k_adj_rk4_pgrad(AdjSegs S, const double* __restrict__ lam_in, int64_t nseg, double* __restrict__ pbar) {
-  const int64_t g0 = (int64_t)blockIdx.x * 32, g1 = min(nseg, g0 + 32);
+  const int64_t g0 = (int64_t)blockIdx.x * kPgradSegs, g1 = min(nseg, g0 + kPgradSegs);
   for (int k = threadIdx.x; k < S.n_params; k += blockDim.x) {
     double acc = 0;
     for (int64_t g = g0; g < g1; ++g)
@@ -900,9 +970,9 @@ double* Engine::rk4_adjoint(const double* d_kb, int param_field, int64_t n_param
   S.pseg = d_pseg;
   S.n_params = (int)n_params;
   if (nseg > 0) {
-    dev::k_adj_rk4_segments<<<(unsigned)nseg, 32, 0, st>>>(AF, S);
+    dev::k_adj_rk4_segments<<<(unsigned)nseg, dev::kSegThreads, 0, st>>>(AF, S);
     dev::k_adj_rk4_lam<<<2, 128, 0, st>>>(S, d_lam_in);
-    dev::k_adj_rk4_pgrad<<<(unsigned)((nseg + 31) / 32), 128, 0, st>>>(S, d_lam_in, nseg, d_pgrad);
+    dev::k_adj_rk4_pgrad<<<(unsigned)((nseg + dev::kPgradSegs - 1) / dev::kPgradSegs), 128, 0, st>>>(S, d_lam_in, nseg, d_pgrad);
   }
   check(cudaGetLastError(), "trajectory adjoint");
   last_launches += 3;

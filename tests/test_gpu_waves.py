@@ -248,3 +248,29 @@ def test_batch_groups_match_single_jobs():
             alone = one.flux([j], **kw)[0]
             assert np.array_equal(levels[k], one.last_levels[0])
             assert np.max(np.abs(whole[k] - alone)) <= 1e-12 * np.max(np.abs(alone))
+
+
+# The trajectory adjoint's segments of 64 steps, full and ragged, few and many, with other fields beside the tuned one
+# (their gradient enters the steps, not the factors), against central differences of the host's trajectory
+# (h = 1e-6: roundings 1e-16 / h of the knots and h^2: 1e-5 of the gradient).
+@pytest.mark.parametrize("npoints", [66, 129, 640, 1411])
+def test_trajectory_gradient_at_segment_edges(npoints):
+    from oscars_b200.tuning import TuningProblem
+    p = TuningProblem(bfield=[0, 0.5, 0], period=[0, 0, 0.05], nperiods=3, obs=[[0, 0, 20.0]], energies_eV=[400.0], level=4,
+                      ctstartstop=(-0.15, 0.11), npoints=npoints)
+    p.sr.add_bfield_epu(bfieldA=[0, 0.2, 0], bfieldB=[0.1, 0, 0], period=[0, 0.002, 0.06], nperiods=3, phase=0.4, taper=0.1,
+                        frequency=3e8, time_offset=1e-10)
+    p.sr.set_npoints_trajectory(npoints)
+
+    def knots(s):
+        p.set_scale(s)
+        p.sr.calculate_trajectory()
+        return p.sr.trajectory_array()[1:]
+    s0 = 1 + 0.02 * np.cos(np.arange(6))
+    weight = np.random.default_rng(3).standard_normal((9, npoints)) * np.array([1] * 3 + [1e-3] * 3 + [1e-6] * 3)[:, None]
+    g = p.trajectory_vjp(s0, weight[:, :knots(s0).shape[1]])
+    fd = []
+    for e in 1e-6 * np.eye(6):
+        k1, k0 = knots(s0 + e), knots(s0 - e)
+        fd.append(np.sum(weight[:, :k1.shape[1]] * (k1 - k0)) / 2e-6)
+    assert np.linalg.norm(g - np.array(fd)) <= 1e-5 * np.linalg.norm(fd)
