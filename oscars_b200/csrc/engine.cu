@@ -741,7 +741,12 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
     const int slot = speculate ? claim_stat_slot() : -1;
     const unsigned seq = report_launch(active, level_max, st, speculate ? c64 : nullptr,
                                        speculate ? stats_host_ + kStatWords * slot : nullptr, small);
-    if (speculate && !small) finish_request(slot, st);
+    if (speculate && !small) {
+      // Straight into the caller's buffers (page-locked ones, or pageable ones beyond bounce_) only after its host
+      // work, which may write them.
+      if (!tail_.bounce) overlap();
+      finish_request(slot, st);
+    }
     overlap();
     report_wait(seq, &nn, &lmax, st);
     if (nn == 0) {

@@ -95,6 +95,34 @@ def test_rectangle_formed_on_device_matches_uploaded_points(nx, ny, power):
     assert np.array_equal(pos.ravel(), xyz) and np.array_equal(got, want) and np.array_equal(levels, lv)
 
 
+# Results beyond the page-locked download buffer (64 MiB: 5.6 million entries) go straight into the caller's arrays,
+# which the rectangle call clears while the device computes; page-locked arrays take that way at any size.  Same bits.
+@pytest.mark.parametrize("nx, ny, locked", [(2400, 2400, False), (91, 91, True)])
+def test_rectangle_downloads_straight_into_the_callers_arrays(nx, ny, locked):
+    import ctypes
+    import torch
+    from oscars_b200._lib import dptr, i32ptr, lib
+    s = sr(gpu=1)
+    run_case(s, UND_SHORT_SETUP)
+    a = s._rectangle_args([nx, ny], "XY", [0.02, 0.03], None, None, [0, 0.01, 20], 0, True)
+    o = s._opts("", 112188979912321.0, None, None, 0.01, 24, 0, 0, 0, "mixed")
+    n, got = nx * ny, []
+    pts, nrm = np.empty(3 * n), np.empty(3 * n)
+    assert lib().osc_surface_rectangle(*a, dptr(pts), dptr(nrm), None) == 0
+    for rect in (True, False):
+        out, lv = torch.full((n,), -1.0, dtype=torch.float64), torch.full((n,), -1, dtype=torch.int32)
+        if locked:
+            out, lv = out.pin_memory(), lv.pin_memory()
+        out, lv, nnc = out.numpy(), lv.numpy(), ctypes.c_longlong()
+        tail = (ctypes.byref(o),) + ((None, None) if rect else ()) + (dptr(out), i32ptr(lv), ctypes.byref(nnc))
+        if rect:
+            s._ctx.call("osc_power_density_rectangle", *a, 0, *tail)
+        else:
+            s._ctx.call("osc_power_density", dptr(pts), dptr(nrm), n, 0, *tail)
+        got.append((out, lv))
+    assert got[0][0].min() > 0 and np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
 def _stl_both(path, calls):
     out = []
     for o in (sr(gpu=1), OracleSR()):
