@@ -991,7 +991,7 @@ __global__ void __launch_bounds__(256) k_batch_finalize(BatchFinalArgs A) {
 // The terms of a sample are formed once for a tile of up to 64 energies of one observer (lines.cuh), as in the
 // spectra's kernels: an (energy, pair) costs ~33 instructions in the place of 113.  Later waves go over the
 // tiles that still hold active energies, each tile's energies packed.
-__global__ void __launch_bounds__(kLnThreads, 4) k_batch_lines(BatchLineArgs A) {
+__global__ void __launch_bounds__(kLnThreads, 5) k_batch_lines(BatchLineArgs A) {
   __shared__ __align__(16) LineStage st;
   __shared__ double red[(kLnWarps - 1) * 7 * kLnTile];
   __shared__ WavePlan P;
@@ -1037,10 +1037,11 @@ __global__ void __launch_bounds__(kLnThreads, 4) k_batch_lines(BatchLineArgs A) 
     }
     // pair records of job j: absolute pair p at rec_j[kPairF4 * (p - s_off / 2)]
     const float4* rec_j = A.rec + kPairF4 * ((int64_t)j * (A.stride >> 1)) - kPairF4 * (A.s_off >> 1);
-    line_sum(st, chunk, rec_j, p0, p1, span > 0, make_pair_obs(fx, fy, fz, 0.0), n_act > 32 ? kLnPer : 1, sum);
+    line_sum(st, chunk, rec_j, p0, p1, span > 0, make_pair_obs(fx, fy, fz, 0.0), n_act > 32 ? kLnPer : 1,
+             g == P.nseg - 1, sum);
     double dm[kLnPer];
 #pragma unroll
-    for (int k = 0; k < kLnPer; ++k) dm[k] = p1 > p0 ? (double)sum.dmax[k] : -1.0;  // -1 marks an empty span
+    for (int k = 0; k < kLnPer; ++k) dm[k] = p1 > p0 ? (sum.wide[k] ? kPiD : 0.0) : -1.0;  // -1 marks an empty span
     if (tid == 0) next_unit = after;
     line_combine(sum.S, dm, red);
     if (tid < 32) {

@@ -229,7 +229,11 @@ __global__ void __launch_bounds__(kLnThreads, 4) k_fd_lines_fp64(FdWaveArgs A) {
 }
 
 // ---- mixed --------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kLnThreads, 4) k_fd_lines_mixed(FdWaveArgs A, MixedFrame F) {
+// MINB 4 and 5 CTAs an SM: the sums, bound by latency (issue slots 55 %, MUFU 57 % busy at 4), take 745 us at 5 and 802
+// at 4 for 441 observers x 256 energies at level 12, the waves that are over after a unit or two a CTA 23 us and
+// 18 at 96 and 128 registers (launch_fd_lines).
+template <int MINB>
+__global__ void __launch_bounds__(kLnThreads, MINB) k_fd_lines_mixed(FdWaveArgs A, MixedFrame F) {
   if (A.tile_entries != kLnTile) {
     if (threadIdx.x == 0) atomicOr(A.err, kErrPlan);
     return;
@@ -282,11 +286,11 @@ __global__ void __launch_bounds__(kLnThreads, 4) k_fd_lines_mixed(FdWaveArgs A, 
       if (__any_sync(0xffffffffu, e[k].live)) per = k + 1;
       if (e[k].live && warp == 0 && span == 0 && !mixed_geometry_ok(fx, fy, fz, om, F)) atomicOr(A.err, kErrBadArgs);
     }
-    line_sum(st, chunk, rec, p0, p1, span > 0, make_pair_obs(fx, fy, fz, 0.0), per, sum);
+    line_sum(st, chunk, rec, p0, p1, span > 0, make_pair_obs(fx, fy, fz, 0.0), per, A.fused && g == P.nseg - 1, sum);
     if (tid == 0) U.next = after;
     double dm[kLnPer];
 #pragma unroll
-    for (int k = 0; k < kLnPer; ++k) dm[k] = (double)sum.dmax[k];
+    for (int k = 0; k < kLnPer; ++k) dm[k] = sum.wide[k] ? kPiD : 0.0;
     line_store(A, P, tile, g, span, e, sum.S, dm, red);
     if (A.fused) fused_unit_done_grouped<kLnThreads>(A, P, tile, n_act, &s_last, kLnTile, red, P.nseg * P.spans);
     else __syncthreads();
@@ -300,14 +304,17 @@ int lines_entries_per_cta() { return dev::kLnTile; }
 
 int lines_blocks_per_sm(bool mixed) {
   int n = 0;
-  if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dev::k_fd_lines_mixed, dev::kLnThreads, 0);
+  if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dev::k_fd_lines_mixed<5>, dev::kLnThreads, 0);
   else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dev::k_fd_lines_fp64, dev::kLnThreads, 0);
   return n > 0 ? n : 1;
 }
 
 cudaError_t launch_fd_lines(const FdWaveArgs& a, const MixedFrame* F, int grid, cudaStream_t st) {
-  return F ? launch_overlapped(dev::k_fd_lines_mixed, grid, dev::kLnThreads, st, a, *F)
-           : launch_overlapped(dev::k_fd_lines_fp64, grid, dev::kLnThreads, st, a);
+  if (!F) return launch_overlapped(dev::k_fd_lines_fp64, grid, dev::kLnThreads, st, a);
+  // Up to level 10 a wave holds most of the request's entries, as a fixed-level sum does; the later ones, of the few
+  // that are left, are short.  Either takes any grid (the fewer CTAs that fit take more units each).
+  return a.level <= 10 || !a.fused ? launch_overlapped(dev::k_fd_lines_mixed<5>, grid, dev::kLnThreads, st, a, *F)
+                                   : launch_overlapped(dev::k_fd_lines_mixed<4>, grid, dev::kLnThreads, st, a, *F);
 }
 
 }  // namespace osc

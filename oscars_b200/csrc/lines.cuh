@@ -73,25 +73,60 @@ struct LineStage {
   float2 before[4];
 };
 
-// A lane's energies: frequency factors, sums and largest phase step.
+// A lane's energies: frequency factors, sums, and whether a phase step reached pi (all that the stop rule asks).
 struct LineSums {
   float2 w[kLnPer], wc[kLnPer];
-  float wt[kLnPer], wct[kLnPer], dmax[kLnPer];
+  float wt[kLnPer], wct[kLnPer];
+  bool wide[kLnPer];
   double dwt[kLnPer], dwct[kLnPer], S[kLnPer][6];
 };
 __device__ __forceinline__ void line_energy(LineSums& e, int k, double om) {
   const PairObs o = make_pair_obs(0.0, 0.0, 0.0, om);
   e.w[k] = o.w; e.wc[k] = o.wc; e.wt[k] = o.wt; e.wct[k] = o.wct; e.dwt[k] = o.dwt; e.dwct[k] = o.dwct;
-  e.dmax[k] = 0.f;
+  e.wide[k] = false;
 #pragma unroll
   for (int c = 0; c < 6; ++c) e.S[k][c] = 0;
 }
 
+// Whether a phase step of the warp's pairs [j0, j1) reaches pi, for each of a lane's energies.  A step is
+// |P_j - P_{j-1}| of P = RN(wc corr + RN(w T)), so it stays below wc |dcorr| + w |dT| plus the roundings of both P
+// (2^-24 (wc |corr| + 2 w |T|) each) and of the bound itself.  The quarter's largest |dcorr|, |dT|, |corr| and |T| serve
+// all energies, and a step is formed as such only where that bound does not clear pi (the coarse levels) and no earlier
+// step settled it: 6 of the 39 instructions an (energy, pair) took when every step was formed.
+__device__ __forceinline__ void line_steps(const LinePairs& t, float2 before, int j0, int j1, int per, LineSums& e) {
+  float dc = 0.f, dt = 0.f, c = 0.f, tt = 0.f;
+  for (int j = j0 + (threadIdx.x & 31); j < j1; j += 32) {
+    const float4 ct = t.ct[j];
+    const float2 b = j > 0 ? make_float2(t.ct[j - 1].y, t.ct[j - 1].w) : before;  // (NaN: no step into the pair)
+    dc = fmaxf(dc, fmaxf(fabsf(ct.x - b.x), fabsf(ct.y - ct.x)));
+    dt = fmaxf(dt, fmaxf(fabsf(ct.z - b.y), fabsf(ct.w - ct.z)));
+    c = fmaxf(c, fmaxf(fmaxf(fabsf(ct.x), fabsf(ct.y)), fabsf(b.x)));
+    tt = fmaxf(tt, fmaxf(fmaxf(fabsf(ct.z), fabsf(ct.w)), fabsf(b.y)));
+  }
+  auto over_warp = [](float v) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v))); };
+  dc = over_warp(dc); dt = over_warp(dt); c = over_warp(c); tt = over_warp(tt);
+#pragma unroll
+  for (int k = 0; k < kLnPer; ++k) {
+    if (k >= per || e.wide[k]) continue;
+    const float wc = fabsf(e.wc[k].x), w = fabsf(e.w[k].x);
+    if (fmaf(wc, dc, w * dt) * 1.00001f + fmaf(wc, c, 2.f * w * tt) * 2.5e-7f < 3.1415f) continue;
+    const float2 b = j0 > 0 ? make_float2(t.ct[j0 - 1].y, t.ct[j0 - 1].w) : before;
+    float last = fmaf(e.wc[k].x, b.x, __fmul_rn(e.w[k].x, b.y));
+    for (int j = j0; j < j1; ++j) {
+      const float4 ct = t.ct[j];
+      const float2 ph = fma2(e.wc[k], make_float2(ct.x, ct.y), mul2(e.w[k], make_float2(ct.z, ct.w)));
+      e.wide[k] |= (double)fmaxf(fabsf(ph.x - last), fabsf(ph.y - ph.x)) >= kPiD;
+      last = ph.y;
+    }
+  }
+}
+
 // Pairs [p0, p1) of `rec` for the tile: `joins` when pair p0 - 1 precedes them; `per` (1 or kLnPer, uniform over
-// the CTA) energies a lane are in use.  Every thread of the CTA takes part.  The folds of 16 pairs start at the
-// quarter chunks' starts, as in k_fd_wave_mixed_pair.
+// the CTA) energies a lane are in use; `steps` (uniform) when the stop rule will read their phase steps.  Every
+// thread of the CTA takes part.  The folds of 16 pairs start at the quarter chunks' starts, as in
+// k_fd_wave_mixed_pair.
 __device__ __forceinline__ void line_sum(LineStage& st, unsigned& chunk, const float4* __restrict__ rec, int64_t p0,
-                                         int64_t p1, bool joins, const PairObs& o, int per, LineSums& e) {
+                                         int64_t p1, bool joins, const PairObs& o, int per, bool steps, LineSums& e) {
   const int tid = threadIdx.x, warp = tid >> 5;
   for (int64_t lo = p0; lo < p1; lo += kLnPairs, ++chunk) {
     const int n = (int)min((int64_t)kLnPairs, p1 - lo);
@@ -110,12 +145,7 @@ __device__ __forceinline__ void line_sum(LineStage& st, unsigned& chunk, const f
     }
     __syncthreads();
     const int j0 = (warp * n) / kLnWarps, j1 = ((warp + 1) * n) / kLnWarps;
-    float last[kLnPer];
-    {
-      const float2 b = j0 > 0 ? make_float2(t.ct[max(j0, 1) - 1].y, t.ct[max(j0, 1) - 1].w) : st.before[chunk & 3u];
-#pragma unroll
-      for (int k = 0; k < kLnPer; ++k) last[k] = fmaf(e.wc[k].x, b.x, __fmul_rn(e.w[k].x, b.y));
-    }
+    if (steps) line_steps(t, st.before[chunk & 3u], j0, j1, per, e);
     auto folds = [&](auto used) {
       constexpr int PER = decltype(used)::value;
       for (int jb = j0; jb < j1; jb += kLnFold) {
@@ -125,18 +155,15 @@ __device__ __forceinline__ void line_sum(LineStage& st, unsigned& chunk, const f
         for (int k = 0; k < PER; ++k)
 #pragma unroll
           for (int c = 0; c < 6; ++c) acc[k][c] = f2(0.f);
-#pragma unroll 2
+#pragma unroll 4
         for (int j = jb; j < je; ++j) {
-          const float4 v01 = t.v01[j], v2k = t.v2k[j], ct = t.ct[j];
+          const float4 v01 = t.v01[j], v2k = t.v2k[j];
           const double2 d = t.d[j];
           const float2 s = t.s[j];
           const float2 vx = make_float2(v01.x, v01.y), vy = make_float2(v01.z, v01.w), vz = make_float2(v2k.x, v2k.y);
-          const float2 nk2 = make_float2(v2k.z, v2k.w), corr = make_float2(ct.x, ct.y), T = make_float2(ct.z, ct.w);
+          const float2 nk2 = make_float2(v2k.z, v2k.w);
 #pragma unroll
           for (int k = 0; k < PER; ++k) {
-            const float2 ph32 = fma2(e.wc[k], corr, mul2(e.w[k], T));
-            e.dmax[k] = fmaxf(e.dmax[k], fmaxf(fabsf(ph32.x - last[k]), fabsf(ph32.y - ph32.x)));
-            last[k] = ph32.y;
             const float t0 = turn_fraction(fma(e.dwct[k], d.x, fma(e.dwt[k], d.y, kTurnBase)));
             const float t1 = t0 + fmaf(e.wct[k], s.x, e.wt[k] * s.y);
             const float2 ph = mul2(make_float2(t0, t1), f2(kTwoPiF));

@@ -302,3 +302,19 @@ def test_trajectory_gradient_at_segment_edges(npoints):
         k1, k0 = knots(s0 + e), knots(s0 - e)
         fd.append(np.sum(weight[:, :k1.shape[1]] * (k1 - k0)) / 2e-6)
     assert np.linalg.norm(g - np.array(fd)) <= 1e-5 * np.linalg.norm(fd)
+
+
+# Mixed spectra whose phase steps reach pi at the coarse levels (harmonics up to the 25th at level 9 and 10): the steps
+# bounded per quarter chunk settle the stop rule as the general kernel's single ones do, so the levels are the same ones.
+@pytest.mark.parametrize("low, high, n", [(400, 12000, 130), (6000, 12000, 33), (200, 300, 64)])
+def test_mixed_spectrum_steps_settle_the_same_levels(low, high, n):
+    out = []
+    for variant in (0, -1):
+        s = sr(gpu=1)
+        s._ctx.call("osc_set_variant", 2, variant)
+        run_case(s, UND_SHORT_SETUP)
+        e, f = s.calculate_spectrum(obs=[0.002, 0.001, 20], energy_range_eV=[low, high], npoints=n, compute="mixed",
+                                    return_numpy=True)
+        out.append((f, s.last_levels.copy()))
+    assert np.array_equal(out[0][1], out[1][1])
+    assert np.max(np.abs(out[0][0] - out[1][0])) <= 1e-10 * np.max(np.abs(out[0][0]))
