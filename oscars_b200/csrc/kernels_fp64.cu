@@ -8,12 +8,13 @@
 // order of the final summation and the last-ulp behaviour of sin/cos/pow differ.
 //
 // Work decomposition ("waves"): every (observer, energy) entry that is still unconverged at level
-// L needs the 2^L samples of that level.  A wave launches one CTA per (128 entries x span of the
-// level); each thread owns one entry and walks the span's samples, which a single elected thread
-// stages into shared memory with 1-D TMA bulk copies (double buffered, mbarrier completion).
-// All threads read the same sample at the same time (shared-memory broadcast).  Per-span partial
-// sums go to global memory and a finalize kernel reduces them in span order, applies the
-// reference's stop rule and compacts the still-active entries for the next wave.
+// L needs the 2^L samples of that level.  A wave's CTAs take units (tile of entries x segment x span of
+// the level); each thread owns one entry and walks its part of the span's samples, which a single
+// elected thread stages into shared memory with 1-D TMA bulk copies (double buffered, mbarrier
+// completion).  All threads read the same sample at the same time (shared-memory broadcast).  Per-span
+// partial sums go to global memory; the CTA that finishes a tile's last unit reduces them in span order,
+// applies the reference's stop rule and compacts the still-active entries for the next wave (the
+// allocation-free entry keeps a finalize kernel).
 #include <cstdint>
 #include <cuda_runtime.h>
 #include <type_traits>
