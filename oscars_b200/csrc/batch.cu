@@ -320,49 +320,20 @@ __global__ void __launch_bounds__(32) k_batch_rk4(const DevJob* __restrict__ job
 }
 
 // The same clamped spline with each sweep split across the threads of a block (one block per job
-// and component).  Every sweep is a first-order recurrence: the factor yp_i = (sig_i - 1) /
-// (sig_i yp_{i-1} + 2) a Moebius map of yp_{i-1}, the right side u_i = (6 d_i - sig_i u_{i-1}) / p_i
-// and the back substitution ypp_k = yp_k ypp_{k+1} + u_k affine ones.  Each thread composes the maps
-// of its chunk of points, a block-wide inclusive scan of the chunk maps gives every chunk its entering
-// value, and each thread then runs its chunk with the reference's operations from that value.  The
-// maps contract (|d yp_i / d yp_{i-1}| < 1/4, |sig_i / p_i| < 1/2, |yp_k| < 1/2), so the entering
-// values' rounding does not grow along the chunk.
-constexpr int kSplThreads = 256;
-
-struct Mob { double a, b, c, d; };  // y -> (a y + b) / (c y + d)
-__device__ __forceinline__ Mob mob_then(Mob f, Mob g) {  // g(f(y)), scaled by its largest entry
-  Mob h{g.a * f.a + g.b * f.c, g.a * f.b + g.b * f.d, g.c * f.a + g.d * f.c, g.c * f.b + g.d * f.d};
-  const double m = fmax(fmax(fabs(h.a), fabs(h.b)), fmax(fabs(h.c), fabs(h.d)));
-  const double r = m > 0 ? 1.0 / m : 1.0;
-  return {h.a * r, h.b * r, h.c * r, h.d * r};
-}
-struct Aff { double a, b; };  // x -> a x + b
-__device__ __forceinline__ Aff aff_then(Aff f, Aff g) { return {g.a * f.a, g.a * f.b + g.b}; }
-
-// Inclusive block scan of the threads' maps (kSplThreads of them) in shared memory; returns the
-// composition of the maps of threads 0 .. t-1 (identity for thread 0).
-template <class M, class Then>
-__device__ __forceinline__ M block_prefix(M mine, M identity, M* sh, Then then) {
-  const int t = threadIdx.x;
-  sh[t] = mine;
-  __syncthreads();
-  for (int o = 1; o < kSplThreads; o <<= 1) {
-    M prev = identity;
-    if (t >= o) prev = sh[t - o];
-    __syncthreads();
-    if (t >= o) sh[t] = then(prev, sh[t]);
-    __syncthreads();
-  }
-  const M before = t > 0 ? sh[t - 1] : identity;
-  __syncthreads();
-  return before;
-}
+// and component).  Every sweep is a first-order recurrence that contracts: the factor yp_i = (sig_i - 1) /
+// (sig_i yp_{i-1} + 2) (|d yp_i / d yp_{i-1}| < 1/4), the right side u_i = (6 d_i - sig_i u_{i-1}) / p_i
+// (|sig_i / p_i| < 1/2) and the back substitution ypp_k = yp_k ypp_{k+1} + u_k (|yp_k| < 1/2; all three 0.07 to 0.27
+// at the trajectories' even spacing).  So a chunk's entering value is the recurrence's own after kSplWarm points from
+// any start: 2^-56 of a neighbour's value is left of it at any spacing, 1e-32 at an even one.  Each thread runs those
+// points and then its chunk with the reference's operations; chunks are at least as long as the run-up.
+// Bound by the latency of a thread's divisions: 7 jobs of about 50000 points take 0.99 ms, 1.65 ms on 256 threads that
+// first compose their chunks' maps (Moebius and affine ones, with block scans); 5 of about 12000 0.21 and 0.30 ms.
+constexpr int kSplThreads = 512;
+constexpr int kSplWarm = 56;
 
 __global__ void __launch_bounds__(kSplThreads) k_batch_spline_scan(const DevJob* __restrict__ jobs,
                                                                    double* __restrict__ arena,
                                                                    double* __restrict__ work) {
-  __shared__ Mob shm[kSplThreads];
-  __shared__ Aff sha[kSplThreads];
   const DevJob& J = jobs[blockIdx.x / 9];
   const int c = blockIdx.x % 9;
   const int t = threadIdx.x;
@@ -376,82 +347,68 @@ __global__ void __launch_bounds__(kSplThreads) k_batch_spline_scan(const DevJob*
   };
   // interior points i = 1 .. n-2 in chunks
   const int64_t m = n - 2;
-  const int64_t chunk = (m + kSplThreads - 1) / kSplThreads;
-  const int64_t i0 = 1 + t * chunk, i1 = min(n - 1, i0 + chunk);
+  const int64_t chunk = max((int64_t)kSplWarm, (m + kSplThreads - 1) / kSplThreads);
+  const int64_t i0 = min(n - 1, 1 + t * chunk), i1 = min(n - 1, i0 + chunk);
+  const int64_t from = max((int64_t)1, i0 - kSplWarm);
   // boundary values (src: the clamped first-derivative end conditions of the reference's sweep)
   const double dydx0 = __ddiv_rn(__dsub_rn(Y[1], Y[0]), __dsub_rn(X[1], X[0]));
   const double u0 = __dmul_rn(__ddiv_rn(3., __dsub_rn(X[1], X[0])),
                               __dsub_rn(__ddiv_rn(__dsub_rn(Y[1], Y[0]), __dsub_rn(X[1], X[0])), dydx0));
-  // 1. yp (stored in ypp for now): Moebius maps [[0, sig - 1], [sig, 2]]
-  Mob fm{1, 0, 0, 1};
-  for (int64_t i = i0; i < i1; ++i) {
-    const double sg = sigma(i);
-    fm = mob_then(fm, Mob{0.0, sg - 1.0, sg, 2.0});
-  }
-  const Mob pm = block_prefix<Mob>(fm, Mob{1, 0, 0, 1}, shm, mob_then);
-  double yp_prev = (pm.a * -0.5 + pm.b) / (pm.c * -0.5 + pm.d);  // yp_{i0-1}
   if (t == 0) {
-    yp_prev = -0.5;
     ypp[0] = -0.5;
     u[0] = u0;
   }
-  for (int64_t i = i0; i < i1; ++i) {
-    const double sg = sigma(i);
-    const double p = __dadd_rn(__dmul_rn(sg, yp_prev), 2.0);
-    yp_prev = __ddiv_rn(__dsub_rn(sg, 1.), p);
-    ypp[i] = yp_prev;
+  // 1. yp, stored in ypp for now (the run-up starts from any value, at the front from the exact one)
+  if (i0 < i1) {
+    double yp = -0.5;
+    for (int64_t i = from; i < i1; ++i) {
+      const double sg = sigma(i);
+      yp = __ddiv_rn(__dsub_rn(sg, 1.), __dadd_rn(__dmul_rn(sg, yp), 2.0));
+      if (i >= i0) ypp[i] = yp;
+    }
   }
   __syncthreads();
-  // 2. u: affine maps u_i = (-sig / p) u_{i-1} + (6 d_i / (x_{i+1} - x_{i-1})) / p
-  auto d_i = [&](int64_t i) {
-    return __dsub_rn(__ddiv_rn(__dsub_rn(Y[i + 1], Y[i]), __dsub_rn(X[i + 1], X[i])),
-                     __ddiv_rn(__dsub_rn(Y[i], Y[i - 1]), __dsub_rn(X[i], X[i - 1])));
-  };
-  Aff fa{1, 0};
-  for (int64_t i = i0; i < i1; ++i) {
-    const double sg = sigma(i);
-    const double p = __dadd_rn(__dmul_rn(sg, i == 1 ? -0.5 : ypp[i - 1]), 2.0);
-    fa = aff_then(fa, Aff{-sg / p, __ddiv_rn(__dmul_rn(6., d_i(i)), __dsub_rn(X[i + 1], X[i - 1])) / p});
-  }
-  const Aff pa = block_prefix<Aff>(fa, Aff{1, 0}, sha, aff_then);
-  double u_prev = t == 0 ? u0 : pa.a * u0 + pa.b;  // u_{i0-1}
-  for (int64_t i = i0; i < i1; ++i) {
-    const double sg = sigma(i);
-    const double p = __dadd_rn(__dmul_rn(sg, i == 1 ? -0.5 : ypp[i - 1]), 2.0);
-    u_prev = __ddiv_rn(__dsub_rn(__ddiv_rn(__dmul_rn(6., d_i(i)), __dsub_rn(X[i + 1], X[i - 1])), __dmul_rn(sg, u_prev)), p);
-    u[i] = u_prev;
+  // 2. u
+  if (i0 < i1) {
+    double v = from == 1 ? u0 : 0.0;
+    double slope = __ddiv_rn(__dsub_rn(Y[from], Y[from - 1]), __dsub_rn(X[from], X[from - 1]));
+    for (int64_t i = from; i < i1; ++i) {
+      const double sg = sigma(i);
+      const double p = __dadd_rn(__dmul_rn(sg, i == 1 ? -0.5 : ypp[i - 1]), 2.0);
+      const double next = __ddiv_rn(__dsub_rn(Y[i + 1], Y[i]), __dsub_rn(X[i + 1], X[i]));
+      const double d = __dsub_rn(next, slope);
+      slope = next;
+      v = __ddiv_rn(__dsub_rn(__ddiv_rn(__dmul_rn(6., d), __dsub_rn(X[i + 1], X[i - 1])), __dmul_rn(sg, v)), p);
+      if (i >= i0) u[i] = v;
+    }
   }
   __syncthreads();
-  // 3. back substitution from ypp_{n-1}: ypp_k = yp_k ypp_{k+1} + u_k, k = n-2 .. 0, in chunks of the
-  // reversed index
+  // 3. back substitution from ypp_{n-1}: ypp_k = yp_k ypp_{k+1} + u_k, k = n-2 .. 0
   const double dydxn = __ddiv_rn(__dsub_rn(Y[n - 1], Y[n - 2]), __dsub_rn(X[n - 1], X[n - 2]));
   const double un = __dmul_rn(__ddiv_rn(3., __dsub_rn(X[n - 1], X[n - 2])),
                               __dsub_rn(dydxn, __ddiv_rn(__dsub_rn(Y[n - 1], Y[n - 2]), __dsub_rn(X[n - 1], X[n - 2]))));
   const double last = __ddiv_rn(__dsub_rn(un, __dmul_rn(0.5, u[n - 2])), __dadd_rn(__dmul_rn(0.5, ypp[n - 2]), 1.));
-  const int64_t mb = n - 1;  // k = n-2 .. 0
-  const int64_t cb = (mb + kSplThreads - 1) / kSplThreads;
-  const int64_t r0 = t * cb, r1 = min(mb, r0 + cb);  // reversed positions r: k = n - 2 - r
-  Aff fb{1, 0};
-  for (int64_t r = r0; r < r1; ++r) {
-    const int64_t k = n - 2 - r;
-    fb = aff_then(fb, Aff{ypp[k], u[k]});
+  double next = last;
+  if (i0 < i1) {
+    const int64_t k0 = min(n - 2, i1 - 1 + kSplWarm);
+    if (k0 < n - 2) next = 0.0;
+    for (int64_t k = k0; k >= i1; --k) next = __dadd_rn(__dmul_rn(ypp[k], next), u[k]);
   }
-  const Aff pb = block_prefix<Aff>(fb, Aff{1, 0}, sha, aff_then);
-  double next = pb.a * last + pb.b;  // ypp_{k+1} entering the chunk
-  if (t == 0) next = last;
-  __syncthreads();  // every chunk has read its yp and u before any is overwritten
+  __syncthreads();  // every run-up has read its neighbours' yp before any is overwritten
   if (t == 0) ypp[n - 1] = last;
-  for (int64_t r = r0; r < r1; ++r) {
-    const int64_t k = n - 2 - r;
-    next = __dadd_rn(__dmul_rn(ypp[k], next), u[k]);
-    ypp[k] = next;
-  }
+  if (i0 < i1)
+    for (int64_t k = i1 - 1; k >= (t == 0 ? 0 : i0); --k) {
+      next = __dadd_rn(__dmul_rn(ypp[k], next), u[k]);
+      ypp[k] = next;
+    }
 }
 
 // Trajectory extent in the job frame: max transverse distance from the axis, max longitudinal
-// coordinate and max |tau_s| (one block of 256 threads per job).
-__global__ void k_batch_extent(DevJob* __restrict__ jobs, const double* __restrict__ arena) {
-  __shared__ double sx[256], sz[256], st[256];
+// coordinate and max |tau_s| (one block per job; 50000 points, in front of the
+// splines: 111 us, 215 us with 256 threads).
+constexpr int kExtThreads = 512;
+__global__ void __launch_bounds__(kExtThreads) k_batch_extent(DevJob* __restrict__ jobs, const double* __restrict__ arena) {
+  __shared__ double sx[kExtThreads], sz[kExtThreads], st[kExtThreads];
   DevJob& J = jobs[blockIdx.x];
   const int64_t n = (int64_t)J.nf + J.nb;
   const double* K = arena + J.knots;
@@ -1631,7 +1588,7 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
       for (int g = 0; g < n_groups; ++g) {
         const int b = begin(g), n = groups[g] - b;
         cudaStream_t ts = n_groups > 1 ? batch_stream_[g] : st;
-        dev::k_batch_extent<<<n, 256, 0, ts>>>(d_jobs + b, b_knots_.as<double>());
+        dev::k_batch_extent<<<n, dev::kExtThreads, 0, ts>>>(d_jobs + b, b_knots_.as<double>());
         dev::launch_batch_splines(d_jobs + b, n, n_max, n_total, b_knots_.as<double>(), b_work_.as<double>(), spline_kernel,
                                   ts);
         const int64_t fill_n = rec_per_job * n;  // samples 0 .. 2^(Lpre+1) - 1 of every job

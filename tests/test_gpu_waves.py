@@ -317,3 +317,21 @@ def test_mixed_spectrum_steps_settle_the_same_levels(low, high, n):
         out.append((f, s.last_levels.copy()))
     assert np.array_equal(out[0][1], out[1][1])
     assert np.max(np.abs(out[0][0] - out[1][0])) <= 1e-10 * np.max(np.abs(out[0][0]))
+
+
+# The block-parallel splines against the serial sweeps at the edges of their chunks (56 points and more, 512 threads): a
+# chunk's entering value keeps less than 2^-56 of any start, and a difference of an ulp in a factor or a right side moves
+# its neighbours by less than twice that: a few 1e-16 of the largest second derivative, 1e-14.
+@pytest.mark.parametrize("npoints", [5, 57, 58, 59, 60, 114, 115, 28674, 28675, 60001])
+def test_block_parallel_splines_match_serial_sweeps(npoints):
+    from oscars_b200.batch import BatchRunner, Job, undulator
+    job = Job(fields=[undulator([0.1, 0.5, 0], [0, 0, 0.05], 12, phase=-0.7)], energy_GeV=3.0, ctstartstop=(-4e-4 * npoints, 5e-4 * npoints),
+              npoints=npoints, obs=[[0, 0, 20]], energies_eV=[400.0])
+    got = []
+    for kernel in (1, 2):
+        r = BatchRunner(gpu=0)
+        r.ctx.call("osc_set_batch_spline_kernel", kernel)
+        got.append(r.trajectories([job])[0])
+    assert np.array_equal(got[0][:10], got[1][:10])
+    scale = np.max(np.abs(got[0][10:]), axis=1, keepdims=True)
+    assert np.all(np.abs(got[0][10:] - got[1][10:]) <= 1e-14 * scale)
