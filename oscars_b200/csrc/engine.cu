@@ -1119,6 +1119,12 @@ void Engine::radiation(RadRequest& rq) {
   omega_staged_ = obs_staged_ = nrm_staged_ = 0;
   rect_pending_ = nullptr;
   early_err_ = 0;
+  // What a request says of its results ends with it, also where a refusal leaves through collect(): the next one
+  // would take its downloads for done.
+  struct TailEnd {
+    ResultTail& tail;
+    ~TailEnd() { tail = ResultTail{}; }
+  } tail_end{tail_};
   const int64_t n_stage = (rq.power_density ? 0 : n_e) + 3 * rq.n_obs * (rq.normals ? 2 : 1);
   if (rq.obs_on_device) {
     req_obs_ = rq.obs;
@@ -1190,7 +1196,6 @@ void Engine::radiation(RadRequest& rq) {
   if (np <= 0) {
     model.ensure_trajectory();
     upload_trajectory();
-    tail_ = ResultTail{};
     if (!rq.out_on_device) {
       tail_.active = true;
       tail_.d_out = d_out;
@@ -1201,12 +1206,7 @@ void Engine::radiation(RadRequest& rq) {
       tail_.small = N <= kTailEntries;
       tail_.bounce = !tail_.small && reserve_bounce(rq.out, (size_t)N * (sizeof(double) + sizeof(int32_t)));
     }
-    try {
-      run_single(rq, N, 1.0, d_out, d_lvl, st);
-    } catch (...) {
-      tail_ = ResultTail{};
-      throw;
-    }
+    run_single(rq, N, 1.0, d_out, d_lvl, st);
     tail_.active = false;
   } else {
     // src/OSCARSSR.cc:4026-4062: new random particle, its trajectory, weight 1/N, compensated sum
@@ -1259,7 +1259,6 @@ void Engine::radiation(RadRequest& rq) {
       }
     }
     collect();
-    tail_ = ResultTail{};
   }
 }
 

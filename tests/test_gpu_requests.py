@@ -1,0 +1,39 @@
+"""Requests that follow one another on a context, and shares of a request, on the GPU."""
+import numpy as np
+import pytest
+
+from oscars_b200.sr import sr
+from cases import BEAM_GAUSS, E1_U, UND_SHORT, run_case, traj
+
+pytestmark = pytest.mark.gpu
+
+
+def _machine():
+    s = sr(gpu=1)
+    run_case(s, [UND_SHORT, BEAM_GAUSS] + traj(5001, -0.5, 0.5))
+    return s
+
+
+# A refused request leaves nothing behind: what follows is what a fresh context gives.  (Variants tuned per context
+# and FP64 sums in another order: 1e-12 of the peak.)
+@pytest.mark.parametrize("side", [2, 100])  # results through mapped memory, and downloads through page-locked memory
+@pytest.mark.parametrize("nparticles", [0, 3])
+def test_requests_after_a_refused_one(side, nparticles):
+    common = dict(max_level=6, nparticles=nparticles, return_numpy=True)
+    geo = dict(npoints=[side, side], width=[0.002, 0.002], translation=[0, 0, 20])
+    results = []
+    for refused in (False, True):
+        s = _machine()
+        for call in (lambda: s.calculate_flux_rectangle(energy_eV=E1_U, **geo, **common),
+                     lambda: s.calculate_spectrum(obs=[0, 0, 20], energy_range_eV=[400, 500], npoints=side * side, **common),
+                     lambda: s.calculate_power_density_rectangle(**geo, **common)):
+            s.set_new_particle(particle="ideal")
+            if refused:
+                with pytest.raises(ValueError, match="compute='mixed' needs observers near the beam axis"):
+                    s.calculate_flux_rectangle(energy_eV=E1_U, npoints=[side, side], width=[1e-4, 1e-4],
+                                               translation=[3, 0, 20], max_level=6, compute="mixed")
+            s.set_seed(3)
+            results.append(call() + (s.last_levels,))
+    for want, got in zip(results[:3], results[3:]):
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[2], want[2])
+        assert want[1].min() > 0 and np.max(np.abs(got[1] - want[1])) <= 1e-12 * np.max(want[1])
