@@ -1243,6 +1243,11 @@ void Engine::radiation(RadRequest& rq) {
         ++last_launches;
       }
     }
+    if (mine.empty()) {  // no particle for this process: a share of zeros, with no level, and no wave behind it
+      if (rq.meanwhile) rq.meanwhile();
+      wait_inputs(st);
+      check(cudaMemsetAsync(d_lvl, 0xff, sizeof(int32_t) * N, st), "levels");
+    }
     check(cudaMemcpyAsync(d_out, acc_.p, sizeof(double) * N, cudaMemcpyDeviceToDevice, st), "result");
   }
   if (!rq.out_on_device) {

@@ -37,3 +37,24 @@ def test_requests_after_a_refused_one(side, nparticles):
     for want, got in zip(results[:3], results[3:]):
         assert np.array_equal(got[0], want[0]) and np.array_equal(got[2], want[2])
         assert want[1].min() > 0 and np.max(np.abs(got[1] - want[1])) <= 1e-12 * np.max(want[1])
+
+
+# A process without a particle of a shared request: the positions of the whole request, zeros, no level.
+@pytest.mark.parametrize("compute", ["fp64", "mixed"])
+@pytest.mark.parametrize("form", ["rectangle", "three points", "power density"])
+def test_share_without_a_particle(compute, form):
+    s = _machine()
+    geo = dict(npoints=[91, 93], translation=[0.001, 0.002, 20], nparticles=3, max_level=4, compute=compute, return_numpy=True)
+    if form == "three points":
+        geo["x0x1x2"] = [[-0.001, -0.001, 0], [0.001, -0.001, 0], [-0.001, 0.001, 0]]
+    else:
+        geo["width"] = [0.002, 0.002]
+
+    def call(**kw):
+        s.set_seed(5)
+        if form == "power density":
+            return s.calculate_power_density_rectangle(**geo, **kw) + (s.last_levels,)
+        return s.calculate_flux_rectangle(energy_eV=E1_U, **geo, **kw) + (s.last_levels,)
+    pos, values, levels = call(shard=(3, 4))
+    whole = call()
+    assert np.array_equal(pos, whole[0]) and not values.any() and np.all(levels == -1) and whole[1].min() > 0
