@@ -20,6 +20,7 @@ from __future__ import annotations
 import ctypes
 import math
 import sys
+from array import array
 
 import numpy as np
 
@@ -437,13 +438,14 @@ class sr:
         if energy_points_eV is not None:
             if len(energy_points_eV) == 0:
                 raise ValueError("Number of points to calculate is zero.  Check input.")
-            try:
-                e = np.array(energy_points_eV, dtype=np.float64)
-                if e.ndim == 1 and not np.isnan(e).any():
-                    return e
-            except (TypeError, ValueError):
-                pass
-            return np.array([float(e) for e in energy_points_eV])  # nested, None and the like, point by point
+            if type(energy_points_eV) in (list, tuple):
+                try:
+                    return np.array(array("d", energy_points_eV))  # the elements' float(), but for texts
+                except TypeError:
+                    pass
+            elif type(energy_points_eV) is np.ndarray and energy_points_eV.ndim == 1 and energy_points_eV.dtype.kind in "biuf":
+                return np.array(energy_points_eV, dtype=np.float64)
+            return np.array([float(e) for e in energy_points_eV])
         e0 = e1 = 0.0
         if energy_range_eV is not None:
             if len(energy_range_eV) != 2:
