@@ -58,3 +58,22 @@ def test_share_without_a_particle(compute, form):
     pos, values, levels = call(shard=(3, 4))
     whole = call()
     assert np.array_equal(pos, whole[0]) and not values.any() and np.all(levels == -1) and whole[1].min() > 0
+
+
+# The deepest levels of a few entries fill the chip: at most twice the time that their share of many entries takes
+# (1.3 at one tile's 32 observers; 3.1 and 3.6 while a level went in 64 spans whatever its length).
+@pytest.mark.parametrize("compute", ["fp64", "mixed"])
+def test_deep_levels_of_few_entries_fill_the_chip(compute):
+    import time
+    s = _machine()
+
+    def seconds(n):
+        kw = dict(energy_eV=E1_U, npoints=[n, 1], width=[0.002, 0.002], translation=[0, 0, 20], precision=0.0, max_level=24,
+                  compute=compute, return_numpy=True)
+        best = np.inf
+        for _ in range(4):  # (the first fills the level cache and tunes)
+            t = time.perf_counter()
+            s.calculate_flux_rectangle(**kw)
+            best = min(best, time.perf_counter() - t)
+        return best
+    assert seconds(32) <= 2.0 * seconds(47 * 32) / 47
