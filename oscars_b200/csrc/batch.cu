@@ -1615,7 +1615,7 @@ void Engine::batch(const std::vector<FieldSpec>& fields, const std::vector<Batch
       return v;
     };
     // a new shape is tuned and run eagerly; a known shape is captured and replayed as a graph
-    const auto key = std::make_tuple(nj, N, Lfirst, Lpre);
+    const auto key = std::make_tuple(nj, N, n_entry_jobs, Lfirst, Lpre);
     const auto chunk_ev = timed_begin(st);  // with profiling on: device time of the whole chunk
     int v = forced_variant[3] >= 0 ? forced_variant[3] : current_variant_[3];
     const bool need_tune = forced_variant[3] < 0 && autotune && tuned_batch_.find(key) == tuned_batch_.end();

@@ -246,7 +246,8 @@ class Engine {
   bool adj_key_valid_ = false;
   cudaGraphExec_t graph_exec_ = nullptr;
   long long graph_launches_ = 0;
-  std::map<std::tuple<int, int64_t, int, int>, int> tuned_batch_;  // (jobs, entries, first, prefill level)
+  // (jobs, entries, those that go one by one, first, prefill level)
+  std::map<std::tuple<int, int64_t, int64_t, int, int>, int> tuned_batch_;
   int batch_resident(int variant);
   int tune_batch(int nj, int Lfirst, int64_t target, const DevJob* d_jobs, const BatchPlan& plan, unsigned* misc,
                  unsigned long long* m64, int64_t rec_stride);

@@ -77,3 +77,19 @@ def test_deep_levels_of_few_entries_fill_the_chip(compute):
             best = min(best, time.perf_counter() - t)
         return best
     assert seconds(32) <= 2.0 * seconds(47 * 32) / 47
+
+
+# A batch whose jobs all go in energy tiles leaves no choice of the other jobs' kernel behind: a later one with the
+# same numbers of jobs and entries, but few energies a job, times its variants as on a fresh context (at 900 entries
+# a job another one than a context starts with).
+def test_batch_variant_is_timed_for_jobs_of_few_energies():
+    from oscars_b200.batch import BatchRunner, Job, undulator
+
+    def jobs(m, n):
+        return [Job(fields=[undulator([0, 0.5, 0], [0, 0, 0.05], 11, phase=-np.pi / 2)], energy_GeV=3.0, ctstartstop=(-0.5, 0.5),
+                    npoints=5001, obs=[[1e-5 * k, 2e-6 * k, 20.0] for k in range(m)], energies_eV=np.linspace(300, 600, n))] * 2
+    fresh, after = BatchRunner(gpu=0), BatchRunner(gpu=0)
+    fresh.flux(jobs(100, 9))
+    after.flux(jobs(90, 10))
+    after.flux(jobs(100, 9))
+    assert after.variant() == fresh.variant()
