@@ -712,7 +712,6 @@ void Engine::run_single(const RadRequest& rq, int64_t n_items, double weight, do
     f.n_items = N; f.act = act_in; f.n_act = nact_in; f.state = state_.as<double>();
     f.act_next = act_[cur_list ^ 1].as<int>(); f.n_next = n_next;
     f.out = d_out; f.level_out = d_lvl; f.not_converged = c64; f.samples = c64 + 1; f.level_max = level_max; f.work_reset = nullptr;
-    f.dmax_spans_joined = 1;  // the flux waves carry the step into each part across groups and spans
     auto ev = timed_begin(st);
     const int g = grid_for(L);
     w.e_tiles = (w.n_e + tile - 1) / tile;
@@ -1065,14 +1064,10 @@ __global__ void __launch_bounds__(1024) k_report_counts(const unsigned* __restri
   host[0] = seq;
 }
 
-// The two device words `a` and `b` once the stream reaches this point: a one-thread kernel stores
-// them into the mapped control words (ctl_host_[1], [2]) and then the sequence number into [0],
-// which the host polls; every 4096 polls it asks whether the stream has finished, so a failed or
+// The two device words `a` and `b` once the stream reaches this point: a kernel stores them into the
+// mapped control words (ctl_host_[1], [2]) and then the sequence number into [0], which the host
+// polls (report_wait); every 4096 polls it asks whether the stream has finished, so a failed or
 // lost launch ends in the stream's error instead of a wait that does not end.
-void Engine::report_counts(const unsigned* a, const unsigned* b, unsigned* va, unsigned* vb, cudaStream_t st) {
-  report_wait(report_launch(a, b, st), va, vb, st);
-}
-
 unsigned Engine::report_launch(const unsigned* a, const unsigned* b, cudaStream_t st, const unsigned long long* c64,
                                unsigned long long* slot, bool results) {
   const unsigned seq = ++report_seq_;

@@ -184,16 +184,15 @@ class Engine {
   size_t bounce_bytes_ = 0;
   // Device counter block cnt_ (16 words): [0], [1] survivor-list counts, [4..9] three 64-bit counters
   // (not converged, samples, unit counter of the running wave), [12] highest finished level -- all
-  // zeroed by one memset of words 0..12 per request -- and [kCntErr] the sticky error word.
+  // zeroed by the request prologue (words 0..12) -- and [kCntErr] the sticky error word.
   static constexpr int kCntErr = 15;
   // pinned words the host reads back: [0] sequence word, [1] active count and [2] highest finished
-  // level between waves (report_counts), [4..7] the batch statistics (two 64-bit counters), [8] the
-  // batch error word, [9] the STL active count
+  // level between waves (report_launch), [4..7] the batch statistics (two 64-bit counters), [8] the
+  // batch error word
   unsigned* ctl_host_ = nullptr;  // mapped (cudaHostAllocMapped): also written by k_report_counts
   unsigned report_seq_ = 0;
-  void report_counts(const unsigned* a, const unsigned* b, unsigned* va, unsigned* vb, cudaStream_t st);
-  // its sequence number; with `slot`, the kernel also stores the request's statistics there (c64[0..1]
-  // and the error word)
+  // A report of the words `a` and `b`: its sequence number; with `slot`, the kernel also stores the request's
+  // statistics there (c64[0..1] and the error word), with `results` the tail's values and levels
   unsigned report_launch(const unsigned* a, const unsigned* b, cudaStream_t st, const unsigned long long* c64 = nullptr,
                          unsigned long long* slot = nullptr, bool results = false);
   void report_wait(unsigned seq, unsigned* va, unsigned* vb, cudaStream_t st);

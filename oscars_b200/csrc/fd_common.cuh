@@ -599,62 +599,10 @@ __device__ __forceinline__ int64_t fused_part_index(const WavePlan& P, int64_t t
   return ((((tile * P.nseg + g) * P.spans + sp) * kFdPartials) + k) * (int64_t)tile_entries + q;
 }
 
-// Fused finalize of one tile by all threads of the CTA that finished its last span; entry q of the
-// tile is (e * THREADS + threadIdx.x) for q < TE.  Partials are read through L2 (other CTAs wrote
-// them).  With A.dmax_spans_joined the stored maxima already include the step into each span.
-template <int EPT, int THREADS>
-__device__ void fd_tile_finalize(const FdFinalArgs& A, const WavePlan& P, int64_t tile, int64_t n_act, int TE) {
-  for (int e = 0; e < EPT; ++e) {
-    const int q = e * THREADS + (int)threadIdx.x;
-    const int64_t slot = tile * TE + q;
-    const bool live = q < TE && slot < n_act;
-    const int64_t item = live ? (A.act ? (int64_t)A.act[slot] : slot) : 0;
-    auto seg_sum = [&](int g, C3& s, double& dmax) {
-      for (int sp = 0; sp < P.spans; ++sp) {
-        const double* p = A.part + fused_part_index(P, tile, g, sp, 0, q, TE);
-        s.xr += __ldcg(p); s.xi += __ldcg(p + TE); s.yr += __ldcg(p + 2 * TE);
-        s.yi += __ldcg(p + 3 * TE); s.zr += __ldcg(p + 4 * TE); s.zi += __ldcg(p + 5 * TE);
-        const double dm = __ldcg(p + 8 * TE);
-        if (dm >= 0) {  // non-empty span (empty spans only trail the segment)
-          dmax = fmax(dmax, dm);
-          if (sp > 0 && !A.dmax_spans_joined) {
-            const double* pp = A.part + fused_part_index(P, tile, g, sp - 1, 0, q, TE);
-            dmax = fmax(dmax, fabs(__dsub_rn(__ldcg(p + 6 * TE), __ldcg(pp + 7 * TE))));
-          }
-        }
-      }
-    };
-    bool finished = false, unconverged = false, survive = false;
-    if (live) {
-      C3 S = {0, 0, 0, 0, 0, 0};
-      double last_mag = -1, dmax = 0;
-      if (A.first) {
-        double unused = 0;
-        if (P.nseg == 2) {
-          seg_sum(0, S, unused);
-          C3 t = c3_scale(S, A.dt_prev);
-          if (A.project) t = c3_project(t, A.pol);
-          last_mag = c3_mag2(t);
-        }
-        seg_sum(P.nseg - 1, S, dmax);
-      } else {
-        const int64_t N = A.n_items;
-        S = {A.state[item], A.state[N + item], A.state[2 * N + item], A.state[3 * N + item], A.state[4 * N + item],
-             A.state[5 * N + item]};
-        last_mag = A.state[6 * N + item];
-        seg_sum(0, S, dmax);
-      }
-      fd_entry_decide(A, item, S, last_mag, dmax, finished, unconverged, survive);
-    }
-    finalize_bookkeeping(finished, unconverged, survive, item, A.level, A.act_next, A.n_next, A.not_converged,
-                         A.samples, A.level_max);
-  }
-}
-
 // Fused finalize of one tile by all THREADS threads of the CTA, in G = THREADS / TE groups of TE
-// threads (entry q = threadIdx.x % TE): group g sums the spans g, g + G, ... of its entry in order, the
-// groups' sums are combined in group order through `red` ((G - 1) x 7 x TE doubles) and group 0
-// applies the stop rule.  The span maxima include the step into each span (the mixed kernels).
+// threads (entry q = threadIdx.x % TE); the partials are read through L2 (other CTAs wrote them).  Group g
+// sums the spans g, g + G, ... of its entry in order, the groups' sums are combined in group order
+// through `red` ((G - 1) x 7 x TE doubles) and group 0 applies the stop rule.  The span maxima include the step into each span.
 template <int THREADS>
 __device__ void fd_tile_finalize_grouped(const FdFinalArgs& A, const WavePlan& P, int64_t tile, int64_t n_act, int TE,
                                          double* red) {
@@ -740,7 +688,8 @@ __device__ void fd_tile_finalize_grouped(const FdFinalArgs& A, const WavePlan& P
                        A.samples, A.level_max);
 }
 
-// End of a unit of a fused wave with the grouped finalize: as fused_unit_done, for tiles of `units` units.
+// End of a unit of a fused wave: publish this CTA's partials, count the tile's finished units, and let the CTA that
+// finished the last of its `units` finalize the tile.
 template <int THREADS>
 __device__ __forceinline__ void fused_unit_done_grouped(const FdWaveArgs& A, const WavePlan& P, int64_t tile,
                                                         int64_t n_act, int* s_last, int TE, double* red, int units) {
@@ -754,25 +703,6 @@ __device__ __forceinline__ void fused_unit_done_grouped(const FdWaveArgs& A, con
   __syncthreads();
   if (*s_last) {
     fd_tile_finalize_grouped<THREADS>(A.fin, P, tile, n_act, TE, red);
-    if (threadIdx.x == 0) A.tile_done[tile] = 0;
-  }
-}
-
-// End of a unit in a fused wave: publish this CTA's partials, count the tile's finished spans, and
-// let the CTA that finished the last one finalize the tile.
-template <int EPT, int THREADS>
-__device__ __forceinline__ void fused_unit_done(const FdWaveArgs& A, const WavePlan& P, int64_t tile,
-                                                int64_t n_act, int* s_last, int TE = EPT * THREADS) {
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned done = atomicAdd(&A.tile_done[tile], 1u);
-    *s_last = done == (unsigned)(P.spans - 1);
-    if (*s_last) __threadfence();
-  }
-  __syncthreads();
-  if (*s_last) {
-    fd_tile_finalize<EPT, THREADS>(A.fin, P, tile, n_act, TE);
     if (threadIdx.x == 0) A.tile_done[tile] = 0;
   }
 }

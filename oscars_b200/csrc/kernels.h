@@ -90,7 +90,6 @@ struct FdFinalArgs {
   unsigned long long* not_converged;
   unsigned long long* samples;
   unsigned long long* work_reset;  // the wave's unit counter, zeroed for the next wave
-  int dmax_spans_joined;    // the span maxima include the step from the previous span's last sample
   unsigned* level_max;      // highest level at which an entry finished (may be NULL)
 };
 

@@ -102,10 +102,9 @@ constexpr int kFdChunk = 128;
 // per thread; group g takes the g-th of SUB equal parts of every staged chunk of the 10 level arrays.
 // Each part starts from the phase of the sample before it (the chunk's previous sample, the previous
 // chunk's last one, or the span's predecessor read from the level cache), so the phase steps of a
-// span cover exactly the consecutive pairs of the serial order and spans need no joining
-// (dmax_spans_joined); the stop rule only asks whether a step reaches pi, so a span stores pi or 0 in the
-// place of its largest step.  The groups' sums are combined in shared memory in group order.  Fused
-// waves finalize their tiles with all threads (fused_unit_done_grouped); unfused waves store
+// span cover exactly the consecutive pairs of the serial order and spans need no joining; the stop
+// rule only asks whether a step reaches pi, so a span stores pi or 0 in the place of its largest
+// step.  The groups' sums are combined in shared memory in group order.  Fused waves finalize their tiles with all threads (fused_unit_done_grouped); unfused waves store
 // entry-major partials for k_fd_finalize.
 //
 // Bound by the FP64 pipe: 95 instructions per (entry, sample) at one per two cycles and

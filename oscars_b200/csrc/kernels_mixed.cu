@@ -83,9 +83,9 @@ __global__ void k_mixed_records(const double* __restrict__ knots, int64_t n, dou
 // threads (one entry per thread); each group takes 1/SUB of every staged chunk, two samples per
 // packed step.  The largest phase step of a part starts from the sample before it (inside the
 // chunk, the previous chunk's last sample carried by group 0, or the span's predecessor read from
-// global memory), so the span maxima already include the step into each span (dmax_spans_joined).
+// global memory), so the span maxima already include the step into each span.
 // The groups' sums are reduced in shared memory in group order and one tile-major partial per entry
-// and span is stored; the CTA that finishes a tile's last span finalizes the tile (fused_unit_done).
+// and span is stored; the CTA that finishes a tile's last span finalizes the tile (fused_unit_done_grouped).
 // With A.fused == 0 the partials are only stored (the adjoint's forward sums read them).
 template <int SUB, int MINB, int CP, bool SSM>
 __global__ void __launch_bounds__(kMxThreads, MINB) k_fd_wave_mixed_pair(FdWaveArgs A, MixedFrame F) {
