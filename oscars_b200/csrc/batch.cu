@@ -202,9 +202,10 @@ __device__ __forceinline__ bool accel_d(double qomg, const double* v, const doub
 // that is the four field evaluations.  The position of a stage needs the velocity of the stage before,
 // not its acceleration, so stages 1 and 2 evaluate the field at positions both known at the start of the
 // step, and stages 3 and 4 at positions both known once those two are: the pair's lanes evaluate two
-// stages' fields side by side, exchange them and carry the same state (one thread for all four:
-// 2.05 us per undulator step with its field's constants re-read, 2.7 us with two fields; a pair with the
-// constants in registers: 0.36 and 0.49 us).  Every operation is spelled out with its rounding: a trajectory's
+// stages' fields side by side, exchange them and carry the same state.  16001 points, both directions at once (8000
+// steps each): one thread for all four stages, its field's constants re-read, 31.2 ms with one undulator and 50.7
+// with two; a pair with the constants in registers 5.0 and 7.4 ms; an EPU and half-period factors, through the general
+// evaluation, 41.2 -> 11.8 and 34.2 -> 10.1 ms.  Every operation is spelled out with its rounding: a trajectory's
 // last bits move the phases far along it, and left to the compiler the fusing differs with the code around it.
 // NF: ideal undulators held in registers (0: any fields).
 template <int NF>
@@ -320,12 +321,17 @@ __global__ void __launch_bounds__(32) k_batch_rk4(const DevJob* __restrict__ job
 }
 
 // The same clamped spline with each sweep split across the threads of a block (one block per job
-// and component).  Every sweep is a first-order recurrence that contracts: the factor yp_i = (sig_i - 1) /
-// (sig_i yp_{i-1} + 2) (|d yp_i / d yp_{i-1}| < 1/4), the right side u_i = (6 d_i - sig_i u_{i-1}) / p_i
-// (|sig_i / p_i| < 1/2) and the back substitution ypp_k = yp_k ypp_{k+1} + u_k (|yp_k| < 1/2; all three 0.07 to 0.27
-// at the trajectories' even spacing).  So a chunk's entering value is the recurrence's own after kSplWarm points from
-// any start: 2^-56 of a neighbour's value is left of it at any spacing, 1e-32 at an even one.  Each thread runs those
-// points and then its chunk with the reference's operations; chunks are at least as long as the run-up.
+// and component).  Every sweep is a first-order recurrence that contracts.  With a_i = -yp_i, 0 <= a_i <= 1/2 and
+// p_i = 2 - sig_i a_{i-1}:
+//   the factor a_i = (1 - sig_i) / p_i, |d a_i / d a_{i-1}| = sig_i (1 - sig_i) / p_i^2 <= 1/12;
+//   the right side u_i = (6 d_i - sig_i u_{i-1}) / p_i.  One factor f_i = sig_i / p_i may reach 2/3, but 1 - a_i =
+//     (1 + sig_i (1 - a_{i-1})) / p_i gives f_i / (1 - a_i) = y / (1 + y) / (1 - a_{i-1}) with y = sig_i (1 - a_{i-1})
+//     <= 1, so n neighbouring ones multiply to at most 2^-n (1 - a_n) / (1 - a_0) <= 2^(1-n);
+//   the back substitution ypp_k = u_k - a_k ypp_{k+1}, a_k <= 1/2.
+// (All three are 0.07 to 0.27 at the trajectories' even spacing.)  So a chunk's entering value is the recurrence's own
+// after kSplWarm points from any start: at most 2^-55 of the start's error is left at any spacing, 1e-32 at an even
+// one.  Each thread runs those points and then its chunk with the reference's operations; chunks are at least as long
+// as the run-up.
 // Bound by the latency of a thread's divisions: 7 jobs of about 50000 points take 0.99 ms, 1.65 ms on 256 threads that
 // first compose their chunks' maps (Moebius and affine ones, with block scans); 5 of about 12000 0.21 and 0.30 ms.
 constexpr int kSplThreads = 512;
@@ -1173,7 +1179,7 @@ static cudaError_t launch_batch_wave(const BatchWaveArgs& a, int grid, int varia
 // Host orchestration
 // ---------------------------------------------------------------------------------------------
 namespace {
-// trajectories per warp of k_batch_rk4: as few as keep one warp per sub-partition (592 on B200)
+// trajectories per warp of k_batch_rk4: as few as keep one warp per sub-partition (4 x 148 SMs on B200)
 int rk4_per_warp(int nj) { return std::min(16, std::max(1, (2 * nj + 591) / 592)); }
 int rk4_blocks(int nj) { return (2 * nj + rk4_per_warp(nj) - 1) / rk4_per_warp(nj); }
 constexpr int kBatchPrefill = 13;        // levels enqueued without the host (records kept resident)

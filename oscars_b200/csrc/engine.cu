@@ -1182,8 +1182,10 @@ void Engine::radiation(RadRequest& rq) {
   // Mixed multi-particle flux / spectrum requests with at least beam_batch_min particles (this
   // process's share) run as one batch with device RK4 trajectories; smaller ones, and those with RKAS
   // trajectories, take the host integrator on worker threads like the FP64 path: the device RK4 is a
-  // serial chain per particle (~4 us per step, ~60 ms for 16001 points whatever the batch size), which
-  // only pays once the batch is large.
+  // serial chain per particle, the same for one as for many.  Two undulators, 16001 points, 31 x 31
+  // observers, 16 host cores, batch and host route: 8.3 and 2.6 ms with 1 particle, 9.1 and 7.3 with 16, 11
+  // and 21 with 64, 62 and 359 with 1024.  (They cross between 16 and 64 particles, at 60001 points and
+  // with an EPU too; the threshold is from the time when the chain of these two undulators took 51 ms.)
   const int shard_n = rq.opts.shard_count > 1 ? rq.opts.shard_count : 1;
   const int shard_r = shard_n > 1 ? rq.opts.shard_rank % shard_n : 0;
   const int np_local = np > shard_r ? (np - shard_r + shard_n - 1) / shard_n : 0;

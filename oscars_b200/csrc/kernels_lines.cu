@@ -229,9 +229,9 @@ __global__ void __launch_bounds__(kLnThreads, 4) k_fd_lines_fp64(FdWaveArgs A) {
 }
 
 // ---- mixed --------------------------------------------------------------------------------------
-// MINB 4 and 5 CTAs an SM: the sums, bound by latency (issue slots 55 %, MUFU 57 % busy at 4), take 745 us at 5 and 802
-// at 4 for 441 observers x 256 energies at level 12, the waves that are over after a unit or two a CTA 23 us and
-// 18 at 96 and 128 registers (launch_fd_lines).
+// MINB 4 and 5 CTAs an SM, 128 and 96 registers a thread (launch_fd_lines): long sums are bound by latency and gain from
+// the fifth CTA (441 observers x 256 energies at level 12: 802 us at 4, 748 at 5, MUFU 71 % and issue slots 57 %
+// busy), waves that are over after a unit or two a CTA lose by the fewer registers.
 template <int MINB>
 __global__ void __launch_bounds__(kLnThreads, MINB) k_fd_lines_mixed(FdWaveArgs A, MixedFrame F) {
   if (A.tile_entries != kLnTile) {
@@ -311,8 +311,13 @@ int lines_blocks_per_sm(bool mixed) {
 
 cudaError_t launch_fd_lines(const FdWaveArgs& a, const MixedFrame* F, int grid, cudaStream_t st) {
   if (!F) return launch_overlapped(dev::k_fd_lines_fp64, grid, dev::kLnThreads, st, a);
-  // Up to level 10 a wave holds most of the request's entries, as a fixed-level sum does; the later ones, of the few
-  // that are left, are short.  Either takes any grid (the fewer CTAs that fit take more units each).
+  // The host does not know how many entries a later wave still has; what the level tells is that entries stop from
+  // level 9 on, so that the waves up to 10, and fixed-level sums, hold most of a request's tiles, and later ones
+  // fewer.  Kernels of a spectrum of 41 periods over four harmonics, by 4, by 5 and by this rule: 5001 energies 122, 127
+  // and 117 us, 20000 205, 205 and 202; of 200 periods up to the ninth harmonic, whose entries stop at level 13 to 15,
+  // 218, 228 and 213 us and 449, 443 and 444.  Below about 5000 energies every wave is short and 4 alone
+  // would be 1 to 3 us faster (61 energies: 61, 67 and 62).  Either takes any grid (the fewer CTAs that fit
+  // take more units each).
   return a.level <= 10 || !a.fused ? launch_overlapped(dev::k_fd_lines_mixed<5>, grid, dev::kLnThreads, st, a, *F)
                                    : launch_overlapped(dev::k_fd_lines_mixed<4>, grid, dev::kLnThreads, st, a, *F);
 }

@@ -20,7 +20,7 @@ void Engine::power_density_stl(const double* tri, const double* centers, int64_t
   cudaStream_t st = stream;
   pending_.clear();
   last_samples = last_launches = last_not_converged = 0;
-  // one CTA per facet walks a whole level, so the levels stop at 26 here
+  // the levels stop at the deepest one that the reference keeps in memory (26; its samples take 10.7 GB)
   int ext_from = kMaxLevelMemory;
   const int lstop = request_levels(o, kMaxLevelMemory, &ext_from);
   if (n <= 0) return;
