@@ -332,8 +332,10 @@ __global__ void __launch_bounds__(32) k_batch_rk4(const DevJob* __restrict__ job
 // after kSplWarm points from any start: at most 2^-55 of the start's error is left at any spacing, 1e-32 at an even
 // one.  Each thread runs those points and then its chunk with the reference's operations; chunks are at least as long
 // as the run-up.
-// Bound by the latency of a thread's divisions: 7 jobs of about 50000 points take 0.99 ms, 1.65 ms on 256 threads that
-// first compose their chunks' maps (Moebius and affine ones, with block scans); 5 of about 12000 0.21 and 0.30 ms.
+// Bound by the latency of a thread's divisions.  On 256 threads that first compose their chunks' maps (Moebius and affine
+// ones, with block scans) the few long trajectories of a group took longer: 7 jobs of 50001 points 1.77 ms, 1.16 this
+// way; 16 of 20001 0.88 and 0.62; 7 of 12001 0.35 and 0.22.  Short ones and many jobs, which fill the chip, took
+// less: 7 of 4001 0.09 and 0.15 ms; 64 of 50001 5.1 and 5.5; 256 of 20001 7.2 and 9.0, of 12001 4.3 and 5.5.
 constexpr int kSplThreads = 512;
 constexpr int kSplWarm = 56;
 
@@ -528,13 +530,16 @@ __global__ void k_batch_spline(const DevJob* __restrict__ jobs, int njobs, doubl
 }
 
 // Clamped splines of a chunk's trajectories: the serial sweeps (one thread per job and component)
-// take the latency of the longest trajectory's recurrences (~1.6 us per point for both sweeps on
-// B200), the block-parallel ones the chunk's total work (~1.3 ns per point, all 9 components).  mode
-// 0 takes whichever the chunk's shape makes shorter, 1 the serial and 2 the block-parallel kernel.
+// take the latency of the longest trajectory's recurrences (1.3 us per point for both sweeps on B200), the
+// block-parallel ones the chunk's total work (all 9 components 1.3 ns per point while a trajectory fills few of a
+// block's threads, 1.8 from 12000 points on).  Serial and parallel: 800 jobs of 4001 points 5.2 and 4.1 ms, 1300 of
+// them 5.3 and 6.5; 600 of 12001 15.5 and 13.5, 1000 of them 15.6 and 22.8.  mode 0 takes whichever the
+// chunk's shape makes shorter, 1 the serial and 2 the block-parallel kernel.
 // n_max, n_total: of the whole chunk, also where only some of its jobs are solved here.
 void launch_batch_splines(const DevJob* d_jobs, int nj, int64_t n_max, int64_t n_total, double* knots, double* work,
                           int mode, cudaStream_t st) {
-  const double serial_ms = 1.6e-3 * (double)n_max, parallel_ms = 1.3e-6 * (double)n_total;
+  const double serial_ms = 1.3e-3 * (double)n_max;
+  const double parallel_ms = (n_max < 8000 ? 1.3e-6 : 1.8e-6) * (double)n_total;
   if (mode == 2 || (mode == 0 && parallel_ms < serial_ms))
     k_batch_spline_scan<<<9 * nj, kSplThreads, 0, st>>>(d_jobs, knots, work);
   else

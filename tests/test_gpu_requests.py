@@ -114,3 +114,19 @@ def test_last_trajectory_of_a_beam(method):
         s.calculate_trajectory()
         want = s.trajectory_array()
         assert np.isfinite(want).all() and np.array_equal(got, want)
+
+
+# The batch's splines by the rule on its shape, on both sides of its two lines (1000 times the longest trajectory's
+# points, 722 times from 8000 points on), are one of the two kernels' splines bit for bit, the one that the rule
+# states.
+@pytest.mark.parametrize("jobs, npoints, kernel", [(990, 1001, 2), (1010, 1001, 1), (715, 8001, 2), (730, 8001, 1), (3, 8001, 2)])
+def test_spline_kernel_by_the_chunks_shape(jobs, npoints, kernel):
+    from oscars_b200.batch import BatchRunner, Job, undulator
+    job = Job(fields=[undulator([0.1, 0.5, 0], [0, 0, 0.05], 12, phase=-0.7)], energy_GeV=3.0, ctstartstop=(-0.4, 0.5),
+              npoints=npoints, obs=[[0, 0, 20]], energies_eV=[400.0])
+    got = []
+    for mode in (0, 1, 2):
+        r = BatchRunner(gpu=0)
+        r.ctx.call("osc_set_batch_spline_kernel", mode)
+        got.append(r.trajectories([job] * jobs)[-1])
+    assert not np.array_equal(got[1], got[2]) and np.array_equal(got[0], got[kernel])
