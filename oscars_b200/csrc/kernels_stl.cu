@@ -9,7 +9,7 @@
 // (stl_clear: the barycentric coordinates of the ray's crossing are ratios of functions linear in the
 // sample's position, so their ranges over the samples' bounding box are exact up to rounding); testing
 // every pair for every sample was all of the time before (514 facets: 2.7 ms of launches, of which
-// ~0.1 ms remain).  The threads then take the samples in chunks of kStlThreads (sample order = thread
+// 0.07 ms remain).  The threads then take the samples in chunks of kStlThreads (sample order = thread
 // order inside a chunk), test each against the facets left, and find each visible sample's predecessor
 // among the visible ones (warp ballot, then the previous warps' last visible samples, then the previous
 // chunks') for the beta differences.  Sums are reduced in a fixed order; the stop rule
